@@ -404,16 +404,17 @@ int v2d_solver_phase_times(v2d_solver *s, double *out6, int reset);
  * `reps` applications of the current LU factors (the preconditioner solve of
  * one GMRES iteration), each preceded by a write of flush_bytes to evict L2;
  * *factor_bytes receives the bytes of factor entries one application reads
- * (per front the pivot-block inverses and the blocks G = L21 L11^-1 and
- * H = U11^-1 U12, which hold as many entries as L21 and U12). */
+ * (per front the pivot-block inverse A11^-1 and the blocks G = A21 A11^-1 and
+ * H = A11^-1 A12, which hold as many entries as A11, A21 and A12). */
 int v2d_solver_time_lu_apply(v2d_solver *s, int reps, long long flush_bytes, double *ms_avg,
                              long long *factor_bytes);
 
 /* Measurement aid (no reference counterpart): sizes of the handle's LU
  * preconditioner -- out6 = fronts, tree levels, factor entries (sum f^2),
- * flops of one factorization (per front: the partial LU
- * 2 sum_{k<S} (f-k-1)^2, the pivot-block inverses 2 S^3 / 3, and
- * G = L21 L11^-1, H = U11^-1 U12 2 (f-S) S^2), factor entries one solve reads
+ * flops of one factorization as LU factors brought into the solve's form
+ * would take them (per front: the partial LU 2 sum_{k<S} (f-k-1)^2, the
+ * triangular inverses 2 S^3 / 3, and G, H 2 (f-S) S^2; the block
+ * Gauss-Jordan elimination used performs 2 S f^2), factor entries one solve reads
  * (sum S (2f - S)), work items of the dataflow solve. */
 int v2d_solver_lu_stats(v2d_solver *s, double *out6);
 
@@ -460,9 +461,8 @@ int v2d_solver_time_lu_launches(v2d_solver *s, int reps, long long flush_bytes, 
 /* Measurement aid (no reference counterpart): the device time of each kernel
  * of one LU factorization of the last assembled Jacobian, launched directly,
  * averaged over `reps` (codes kind * 1000 + level; kinds 0 row scaling,
- * 1 scatter, 2 extend-add, 3 first panel, 4 L21 + row swaps + U12, 6 Schur
- * update + next panel, 7 pivot-block inversion, 8 inverse copy, 9 products
- * G = L21 L11^-1 and H = U11^-1 U12, 10 their copy). */
+ * 1 scatter, 2 extend-add, 3 pivot-block inverse, 4 row block of a step,
+ * 6 update of the front, 11 rounding to FP32). */
 int v2d_solver_time_lu_factor(v2d_solver *s, int reps, double *ms, int *codes, int cap, int *n);
 
 /* Measurement aid (no reference counterpart): average ms of `reps` launches

@@ -89,15 +89,13 @@ struct MfPlan {
     long long apply_entries = 0;   // factor entries one solve reads: sum S (2f - S)
     std::vector<int> S, f, voff, uoff, child0, child1, parent;
     std::vector<long long> foff;
-    std::vector<long long> toff;   // offset of the front's S x S block in the level's scratch
-    long long tmax = 0;            // largest sum of S^2 over the fronts of one level
-    std::vector<long long> goff;   // offset of the front's G and H in the level's scratch
-    long long gmax = 0;            // largest sum of 2 m S over the fronts of one level
-    std::vector<int> lvl_off, lvl_maxS, lvl_maxf, lvl_maxm, lvl_maxm_child;
-    std::vector<long long> lvl_fbeg, lvl_fend, lvl_abeg, lvl_aend;
+    std::vector<int> lvl_off, lvl_maxS, lvl_maxf;
+    std::vector<long long> lvl_abeg, lvl_aend;   // assembly entries of each level (forest plans)
     int *d_S = nullptr, *d_f = nullptr, *d_voff = nullptr, *d_uoff = nullptr;
     int *d_child0 = nullptr, *d_child1 = nullptr, *d_parent = nullptr;
-    long long *d_foff = nullptr, *d_toff = nullptr, *d_goff = nullptr;
+    long long *d_foff = nullptr;
+    // per front variable: its position in child 0's / child 1's contribution block (-1: none)
+    int *d_inv0 = nullptr, *d_inv1 = nullptr;
     int *d_vars = nullptr, *d_cbmap = nullptr, *d_asm_csr = nullptr, *d_asm_row = nullptr;
     long long *d_asm_pos = nullptr;
     // work items of the solve (12 ints each: kind, front, rows [beg, end),
@@ -119,10 +117,11 @@ struct MfPlan {
     std::vector<long long> h_asm_pos;
 };
 
-// Flops of one front's factorization into the solve's form (S pivots of f
+// Flops of bringing one front into the solve's form by LU (S pivots of f
 // variables, m = f - S): the partial LU, 2 sum_{k<S} (f - k - 1)^2; the two
-// inverses of the pivot block, 2 S^3 / 3; G = L21 L11^-1 and H = U11^-1 U12,
-// 2 m S^2 (multiply and add each counted).
+// triangular inverses of the pivot block, 2 S^3 / 3; G and H, 2 m S^2
+// (multiply and add each counted).  The least count of the routes considered;
+// the block Gauss-Jordan elimination used performs 2 S f^2.
 inline double front_flops(int S, int f)
 {
     auto sq = [](double n) { return n * (n + 1.0) * (2.0 * n + 1.0) / 6.0; };   // sum_{j<=n} j^2
@@ -144,15 +143,11 @@ struct MfFactor {
                                 // are rounded to FP32 for the solve (F32)
     void *F = nullptr, *upd = nullptr, *z = nullptr;
     void *F32 = nullptr;        // fact64: FP32 copy of F that the solve reads
-    void *tmp = nullptr;        // triangular inverses of one level before they replace L11 / U11
-    void *gh = nullptr;         // G = L21 L11^-1 and H = U11^-1 U12 of one level before they
-                                // replace L21 / U12
-    void *inv_g = nullptr;      // inversion work space in global memory for separators too
-                                // wide for shared memory (per CTA: S x (CW + 33))
+    void *cols = nullptr;       // one elimination step's pivot columns of a level's fronts
     void *wb = nullptr;         // transposed solve: per-front adjoint right-hand sides (vtotal)
     void *tw = nullptr;         // solve: gathered fronts' t, w and struct x (vtotal)
     double *rs = nullptr;       // row scaling 1 / max |a_r.|
-    int *ipiv = nullptr, *perm = nullptr, *flag = nullptr;
+    int *flag = nullptr;
     MfBarrier *bar = nullptr;
     int *sctr = nullptr;        // dataflow solve: 3 counters per front + the work ticket
     int flow_grid = 0;          // most CTAs of the dataflow solve resident at once
@@ -162,7 +157,6 @@ struct MfFactor {
                                 // (forward before, backward after the upper levels)
     int low_grid = 0;           // CTAs of those launches
     size_t low_smem = 0;        // and their shared memory
-    int low_wcap = 0;           // their largest front
     int flow = 1;               // 1: the solve is one dataflow launch; 0: one launch per level
                                 // and sweep
     cudaGraphExec_t graph = nullptr;
@@ -175,7 +169,7 @@ struct MfFactor {
 struct MfDev {
     const int *S, *f, *voff, *uoff, *child0, *child1, *parent;
     const long long *foff;
-    const int *vars, *cbmap, *perm;
+    const int *vars, *cbmap;
     int maxS, maxf;
     void *tw;   // gathered fronts: t and w (forward), -x on the struct variables (backward)
 };
@@ -211,7 +205,7 @@ int mf_factor(const MfPlan *P, MfFactor *M, const int *rowptr, const double *val
 int mf_apply(const MfPlan *P, const MfFactor *M, const void *b, void *x, const int *stop_a,
              const int *stop_b, cudaStream_t s, long long *n_launches);
 // lambda = A^-T g with the factors (the transposed solve: a bottom-up sweep
-// with U11^-T / H^T, then a top-down sweep with L11^-T / G^T).
+// with A11^-T / H^T, then a top-down sweep with G^T).
 int mf_apply_transpose(const MfPlan *P, MfFactor *M, const void *g, void *lambda, cudaStream_t s,
                        long long *launches = nullptr);
 int mf_flag(const MfFactor *M, int *flag, cudaStream_t s);
@@ -233,8 +227,8 @@ int mf_time_apply_launches(const MfPlan *P, const MfFactor *M, int reps, size_t 
                            cudaStream_t s, double *ms, int *codes, int cap, int *n);
 // Per-kernel device time of one factorization launched directly (not from
 // its graph), average of reps; codes kind * 1000 + level (kinds 0 rowscale,
-// 1 scatter, 2 extend_add, 3 panel, 4 L21 + row swaps + U12, 6 gemm,
-// 7 trinv, 8 trcopy, 9 G/H products, 10 G/H copy).  The factors are recomputed from the same values.
+// 1 scatter, 2 extend_add, 3 pivot-block inverse, 4 row block, 6 update,
+// 11 rounding to FP32).  The factors are recomputed from the same values.
 int mf_time_factor_launches(const MfPlan *P, MfFactor *M, const int *rowptr, const double *val,
                             int reps, cudaStream_t s, double *ms, int *codes, int cap, int *n);
 

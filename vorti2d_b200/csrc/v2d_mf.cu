@@ -27,24 +27,17 @@
 //    over the symmetrised node graph of the CSR pattern; each CSR entry goes
 //    to the front of whichever of its two nodes is eliminated first.
 //
-// Numeric phase (device, per Newton iteration), per level bottom-up:
-//  row-scaled CSR values scattered into the zeroed fronts, children's
-//  contribution blocks added (one child slot per launch: deterministic, no
-//  atomics), then a blocked right-looking partial LU of each front, four
-//  batched launches per 32-column panel: the diagonal block (one CTA per
-//  front, pivoting among the block's rows), L21 for the rows below (row
-//  chunks), row swaps + TRSM for the U12 block row (column chunks), GEMM
-//  update of the trailing block (which leaves the Schur complement for the
-//  parent).
+// Numeric phase (device, per Newton iteration): the row-scaled CSR values are
+// scattered into the zeroed fronts; then, per level bottom-up, the children's
+// contribution blocks are added and the fronts are eliminated by blocked
+// Gauss-Jordan steps (v2d_factor.cuh), which leave A11^-1, G = A21 A11^-1
+// (negated) and H = A11^-1 A12 in place and the Schur complement for the
+// parent.
 //
-// After each level's factorization the S x S pivot block of every front is
-// replaced by the explicit inverses of its triangular factors (L11^-1 below
-// the diagonal, U11^-1 on and above it).
-//
-// Solve (device): forward per level bottom-up (gather, permute, z = L11^-1 w,
-// contribution vector for the parent), backward top-down (U12 x_struct,
-// x = U11^-1 y, scatter).  Every step is a row-parallel product split over
-// CTAs of 8 rows, so the large top fronts spread over many SMs.
+// Solve (device): forward per level bottom-up (gather t, contribution vector
+// w - G t for the parent), backward top-down (x = A11^-1 t - H x_struct,
+// scatter).  Every step is a row-parallel product split over CTAs, so the
+// large top fronts spread over many SMs.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -57,6 +50,7 @@
 #include <utility>
 #include <vector>
 
+#include "v2d_factor.cuh"
 #include "v2d_internal.cuh"
 
 namespace v2d {
@@ -205,7 +199,7 @@ void mf_plan_destroy(MfPlan *p)
 {
     if (!p) return;
     void *ptrs[] = {p->d_S, p->d_f, p->d_voff, p->d_uoff, p->d_child0, p->d_child1, p->d_parent,
-                    p->d_foff, p->d_toff, p->d_goff, p->d_vars, p->d_cbmap, p->d_asm_csr,
+                    p->d_foff, p->d_vars, p->d_cbmap, p->d_inv0, p->d_inv1, p->d_asm_csr,
                     p->d_asm_row, p->d_asm_pos, p->d_items};
     for (void *q : ptrs)
         if (q) cudaFree(q);
@@ -540,10 +534,8 @@ int mf_plan_build(int imax, int jmax, int n, const int *h_rowptr, const int *h_c
     P->child0.assign(nf, -1); P->child1.assign(nf, -1); P->parent.assign(nf, -1);
     P->foff.resize(nf);
     P->lvl_off.assign(nlevel + 1, 0);
-    P->lvl_fbeg.assign(nlevel, 0); P->lvl_fend.assign(nlevel, 0);
     P->lvl_abeg.assign(nlevel, 0); P->lvl_aend.assign(nlevel, 0);
-    P->lvl_maxS.assign(nlevel, 0); P->lvl_maxf.assign(nlevel, 0); P->lvl_maxm.assign(nlevel, 0);
-    P->lvl_maxm_child.assign(nlevel, 0);
+    P->lvl_maxS.assign(nlevel, 0); P->lvl_maxf.assign(nlevel, 0);
     std::vector<int> vars, cbmap;
     long long ftot = 0;
     int vtot = 0, utot = 0;
@@ -559,7 +551,6 @@ int mf_plan_build(int imax, int jmax, int n, const int *h_rowptr, const int *h_c
         P->lvl_off[L + 1]++;
         P->lvl_maxS[L] = std::max(P->lvl_maxS[L], S);
         P->lvl_maxf[L] = std::max(P->lvl_maxf[L], f);
-        P->lvl_maxm[L] = std::max(P->lvl_maxm[L], f - S);
         if (tb.t[q].parent >= 0) P->parent[id] = newid[tb.t[q].parent];
         if (tb.t[q].kid[0] >= 0) P->child0[id] = newid[tb.t[q].kid[0]];
         if (tb.t[q].kid[1] >= 0) P->child1[id] = newid[tb.t[q].kid[1]];
@@ -570,32 +561,6 @@ int mf_plan_build(int imax, int jmax, int n, const int *h_rowptr, const int *h_c
         P->maxf = std::max(P->maxf, f);
     }
     for (int L = 0; L < nlevel; ++L) P->lvl_off[L + 1] += P->lvl_off[L];
-    P->toff.assign(nf, 0);
-    for (int L = 0; L < nlevel; ++L) {
-        long long t = 0;
-        for (int id = P->lvl_off[L]; id < P->lvl_off[L + 1]; ++id) {
-            P->toff[id] = t;
-            t += (long long)P->S[id] * P->S[id];
-        }
-        P->tmax = std::max(P->tmax, t);
-    }
-    P->goff.assign(nf, 0);
-    for (int L = 0; L < nlevel; ++L) {
-        long long t = 0;
-        for (int id = P->lvl_off[L]; id < P->lvl_off[L + 1]; ++id) {
-            P->goff[id] = t;
-            t += 2LL * P->S[id] * (P->f[id] - P->S[id]);
-        }
-        P->gmax = std::max(P->gmax, t);
-    }
-    for (int L = 0; L < nlevel; ++L) {
-        const int a = P->lvl_off[L], b = P->lvl_off[L + 1];
-        P->lvl_fbeg[L] = P->foff[a];
-        P->lvl_fend[L] = P->foff[b - 1] + (long long)P->f[b - 1] * P->f[b - 1];
-        for (int id = a; id < b; ++id)
-            for (int c : {P->child0[id], P->child1[id]})
-                if (c >= 0) P->lvl_maxm_child[L] = std::max(P->lvl_maxm_child[L], P->f[c] - P->S[c]);
-    }
     // contribution-block maps: struct var of child -> local index in parent
     cbmap.assign(utot, -1);
     std::vector<int> loc(n, -1);
@@ -702,6 +667,22 @@ int mf_plan_build(int imax, int jmax, int n, const int *h_rowptr, const int *h_c
     return V2D_OK;
 }
 
+// The inverse contribution maps (k_extend_add), from the uploaded arrays.
+static int invert_cbmap(MfPlan *P)
+{
+    const size_t bytes = std::max<size_t>(1, P->vtotal) * sizeof(int);
+    for (int **d : {&P->d_inv0, &P->d_inv1}) {
+        V2D_CUDA_TRY(cudaMalloc((void **)d, bytes));
+        V2D_CUDA_TRY(cudaMemset(*d, 0xff, bytes));
+    }
+    k_invert_cbmap<<<std::min(P->nfront, 32 * kSMs), 128>>>(
+        P->nfront, P->d_S, P->d_f, P->d_voff, P->d_uoff, P->d_parent, P->d_child0, P->d_cbmap,
+        P->d_inv0, P->d_inv1);
+    V2D_CUDA_TRY(cudaGetLastError());
+    V2D_CUDA_TRY(cudaStreamSynchronize(0));
+    return V2D_OK;
+}
+
 // Device copies of a host plan's arrays; the host copies of the large index
 // arrays are released.  On failure the plan is destroyed.
 static int mf_plan_upload(MfPlan *P)
@@ -715,14 +696,13 @@ static int mf_plan_upload(MfPlan *P)
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_child1, P->child1);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_parent, P->parent);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_foff, P->foff);
-    if (st_up == V2D_OK) st_up = upload_vec(&P->d_toff, P->toff);
-    if (st_up == V2D_OK) st_up = upload_vec(&P->d_goff, P->goff);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_vars, P->h_vars);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_cbmap, P->h_cbmap);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_asm_csr, P->h_asm_csr);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_asm_row, P->h_asm_row);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_asm_pos, P->h_asm_pos);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_items, P->h_items);
+    if (st_up == V2D_OK) st_up = invert_cbmap(P);
     if (st_up != V2D_OK) {
         mf_plan_destroy(P);
         return st_up;
@@ -842,31 +822,13 @@ int mf_plan_forest(const std::vector<MfPlan *> &parts, const std::vector<int> &r
         P->apply_entries += (long long)Q->S[q] * (2LL * Q->f[q] - Q->S[q]);
     }
     P->ftotal = ftot; P->vtotal = vtot; P->utotal = utot;
-    P->lvl_maxS.assign(nl, 0); P->lvl_maxf.assign(nl, 0); P->lvl_maxm.assign(nl, 0);
-    P->lvl_maxm_child.assign(nl, 0);
-    P->lvl_fbeg.assign(nl, 0); P->lvl_fend.assign(nl, 0);
+    P->lvl_maxS.assign(nl, 0); P->lvl_maxf.assign(nl, 0);
     P->lvl_abeg.assign(nl, 0); P->lvl_aend.assign(nl, 0);
-    P->toff.assign(nf, 0);
-    P->goff.assign(nf, 0);
     for (int L = 0; L < nl; ++L) {
         const int a = P->lvl_off[L], b = P->lvl_off[L + 1];
-        long long t = 0, g = 0;
         for (int id = a; id < b; ++id) {
             P->lvl_maxS[L] = std::max(P->lvl_maxS[L], P->S[id]);
             P->lvl_maxf[L] = std::max(P->lvl_maxf[L], P->f[id]);
-            P->lvl_maxm[L] = std::max(P->lvl_maxm[L], P->f[id] - P->S[id]);
-            for (int c : {P->child0[id], P->child1[id]})
-                if (c >= 0) P->lvl_maxm_child[L] = std::max(P->lvl_maxm_child[L], P->f[c] - P->S[c]);
-            P->toff[id] = t;
-            t += (long long)P->S[id] * P->S[id];
-            P->goff[id] = g;
-            g += 2LL * P->S[id] * (P->f[id] - P->S[id]);
-        }
-        P->tmax = std::max(P->tmax, t);
-        P->gmax = std::max(P->gmax, g);
-        if (b > a) {
-            P->lvl_fbeg[L] = P->foff[a];
-            P->lvl_fend[L] = P->foff[b - 1] + (long long)P->f[b - 1] * P->f[b - 1];
         }
     }
     // front variables (shifted rows) and contribution maps (front-local)
@@ -1007,1073 +969,19 @@ namespace v2d {
 // ================================================================ numeric
 namespace {
 
-constexpr int kMfThreads = 256;
-constexpr int kGemmTile = 64;
-constexpr int kTileStages = 2;   // operand slices in flight in the tile engine
-// levels whose largest front has at least kDelayFront variables update the
-// trailing block once per kDelayPanels panels (k_gemm)
-constexpr int kDelayFront = 1024;
-constexpr int kDelayPanels = 8;
-
-template <class T> struct PanelWidth;
-template <> struct PanelWidth<float> { static constexpr int v = 32; };
-template <> struct PanelWidth<double> { static constexpr int v = 32; };
-
-// rs[r] = 1 / max_c |a_rc| (1 for an empty row).
-__global__ void k_rowscale(int n, const int *__restrict__ rowptr, const double *__restrict__ val,
-                           double *rs)
-{
-    V2D_GRID_STRIDE(r, n)
-    {
-        double m = 0.0;
-        for (int p = rowptr[r]; p < rowptr[r + 1]; ++p) m = fmax(m, fabs(val[p]));
-        rs[r] = m > 0.0 ? 1.0 / m : 1.0;
-    }
-}
-
-template <class T>
-__global__ void k_scatter(long long a0, long long a1, const int *__restrict__ csr,
-                          const int *__restrict__ row, const long long *__restrict__ pos,
-                          const double *__restrict__ val, const double *__restrict__ rs, T *F)
-{
-    for (long long e = a0 + (long long)blockIdx.x * blockDim.x + threadIdx.x; e < a1;
-         e += (long long)gridDim.x * blockDim.x)
-        F[pos[e]] += (T)(val[csr[e]] * rs[row[e]]);
-}
-
-// Add child `slot`'s contribution block into each front of the level.
-template <class T>
-__global__ void k_extend_add(int q0, int slot, const int *__restrict__ S, const int *__restrict__ f,
-                             const long long *__restrict__ foff, const int *__restrict__ uoff,
-                             const int *__restrict__ child0, const int *__restrict__ child1,
-                             const int *__restrict__ cbmap, T *F)
-{
-    const int P = q0 + blockIdx.y;
-    const int c = slot == 0 ? child0[P] : child1[P];
-    if (c < 0) return;
-    const int Sc = S[c], fc = f[c], m = fc - Sc, fp = f[P];
-    const T *src = F + foff[c];
-    T *dst = F + foff[P];
-    const int *map = cbmap + uoff[c];
-    const long long tot = (long long)m * m;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < tot;
-         e += (long long)gridDim.x * blockDim.x) {
-        const int a = (int)(e / m), b = (int)(e - (long long)a * m);
-        dst[(long long)map[a] * fp + map[b]] += src[(long long)(Sc + a) * fc + Sc + b];
-    }
-}
-
-// Panel factorization of columns [k, k+w) of every front of the level with
-// S > k.  One warp factors the w x w diagonal block in shared memory with
-// partial pivoting restricted to the block's rows and records both the swap
-// sequence (ipiv) and the block's part of the row permutation; the row scaling applied at
-// assembly keeps the pivots meaningful and the FP64 Krylov iteration around
-// the factors absorbs the weaker pivoting.  The rows below the block (fully
-// summed and contribution rows alike) get their L entries from l21_rows.
-// k_panel factors a level's first panel; every later panel is factored by
-// the trailing update of the panel before it (k_gemm).
-template <class T>
-__device__ __forceinline__ void panel_factor(T *A, int f, int S, int k, int vo, int *ipiv,
-                                             int *perm, int *flag,
-                                             T (*U)[PanelWidth<T>::v + 1], int *pv)
-{
-    constexpr int NB = PanelWidth<T>::v;
-    const int w = min(NB, S - k);
-    const int tid = threadIdx.x, lane = tid & 31;
-    for (int e = tid; e < NB * NB; e += blockDim.x) {
-        const int r = e / NB, c = e - r * NB;
-        U[r][c] = (r < w && c < w) ? A[(long long)(k + r) * f + k + c] : T(0);
-    }
-    __syncthreads();
-    if (tid < 32) {
-        // one warp; lane = row for the pivot search and the elimination,
-        // lane = column for the row swap
-        int bad = 0;
-        if (lane < NB) pv[lane] = lane;
-        __syncwarp();
-        for (int c = 0; c < w; ++c) {
-            T v = (lane >= c && lane < w) ? (T)fabs(U[lane][c]) : T(-1);
-            int idx = lane;
-            for (int o = 16; o > 0; o >>= 1) {
-                const T ov = __shfl_xor_sync(0xffffffffu, v, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-                if (ov > v || (ov == v && oi < idx)) {
-                    v = ov;
-                    idx = oi;
-                }
-            }
-            int p = idx;
-            if (!(v > T(0)) || p < c || p >= w) {
-                p = c;
-                bad = 1;
-            }
-            if (lane == 0) {
-                ipiv[vo + k + c] = k + p;
-                const int t = pv[c];
-                pv[c] = pv[p];
-                pv[p] = t;
-            }
-            if (p != c && lane < NB) {
-                const T t = U[c][lane];
-                U[c][lane] = U[p][lane];
-                U[p][lane] = t;
-            }
-            __syncwarp();
-            const T d = U[c][c];
-            const T inv = d != T(0) ? T(1) / d : T(0);
-            if (lane > c && lane < w) {
-                const T l = U[lane][c] * inv;
-                U[lane][c] = l;
-                // eight entries per batch: their loads issue together (a store
-                // to this lane's row may not be reordered with the next
-                // entry's loads, so one entry at a time is a chain of
-                // shared-memory round trips)
-                int j = c + 1;
-                for (; j + 7 < w; j += 8) {
-                    T a[8], bv[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        a[u] = U[lane][j + u];
-                        bv[u] = U[c][j + u];
-                    }
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) U[lane][j + u] = a[u] - l * bv[u];
-                }
-                for (; j < w; ++j) U[lane][j] -= l * U[c][j];
-            }
-            __syncwarp();
-        }
-        if (bad && lane == 0) atomicOr(flag, 1);
-        // row i of the factored front came from local row perm[i]; the swaps
-        // stay inside the panel's rows, so the panel fixes its own entries
-        if (lane < w) perm[vo + k + lane] = k + pv[lane];
-    }
-    __syncthreads();
-    for (int e = tid; e < w * w; e += blockDim.x) {
-        const int r = e / w, c = e - r * w;
-        A[(long long)(k + r) * f + k + c] = U[r][c];
-    }
-}
-
-template <class T>
-__global__ void __launch_bounds__(kMfThreads) k_panel(int q0, int k, const int *__restrict__ S_,
-                                                      const int *__restrict__ f_,
-                                                      const long long *__restrict__ foff,
-                                                      const int *__restrict__ voff, T *F,
-                                                      int *ipiv, int *perm, int *flag)
-{
-    constexpr int NB = PanelWidth<T>::v;
-    __shared__ T U[NB][NB + 1];
-    __shared__ int pv[NB];
-    const int q = q0 + blockIdx.x;
-    const int S = S_[q], f = f_[q];
-    if (S <= k) return;
-    panel_factor<T>(F + foff[q], f, S, k, voff[q], ipiv, perm, flag, U, pv);
-}
-
-// L entries of the panel for the rows below its diagonal block: x U = a with
-// U the upper triangle of the factored block (no pivoting outside the block).
-// Grid: (chunks of kL21Rows rows, fronts); one thread per row.
-constexpr int kL21Rows = 64;
-
-// L21 entries of row r: x U = a, U the upper triangle of the factored w x w
-// diagonal block (in shared memory).
-template <class T>
-__device__ __forceinline__ void l21_row(T *A, int f, int k, int w, int r,
-                                        const T (*U)[PanelWidth<T>::v + 1])
-{
-    constexpr int NB = PanelWidth<T>::v;
-    T x[NB];
-    T *row = A + (long long)r * f + k;
-#pragma unroll
-    for (int c = 0; c < NB; ++c) x[c] = c < w ? row[c] : T(0);
-    // by rows of U: each finished entry updates the entries after it, so the
-    // dependent chain is NB steps long, not NB^2 / 2 products
-#pragma unroll
-    for (int c = 0; c < NB; ++c) {
-        const T d = U[c][c];
-        const T xc = (c < w && d != T(0)) ? x[c] / d : T(0);
-        x[c] = xc;
-#pragma unroll
-        for (int j = c + 1; j < NB; ++j) x[j] -= xc * U[c][j];
-    }
-#pragma unroll
-    for (int c = 0; c < NB; ++c)
-        if (c < w) row[c] = x[c];
-}
-
-template <class T>
-__device__ __forceinline__ void l21_rows(T *A, int f, int S, int k, int chunk,
-                                         T (*U)[PanelWidth<T>::v + 1])
-{
-    constexpr int NB = PanelWidth<T>::v;
-    const int w = min(NB, S - k);
-    const int rbeg = k + w + chunk * kL21Rows;
-    if (rbeg >= f) return;
-    for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-        const int r = e / NB, c = e - r * NB;
-        U[r][c] = (r < w && c < w) ? A[(long long)(k + r) * f + k + c] : T(0);
-    }
-    __syncthreads();
-    const int r = rbeg + threadIdx.x;
-    if (r >= f) return;
-    l21_row<T>(A, f, k, w, r, U);
-}
-
-// The panel's row swaps (confined to its w rows) applied to every column
-// outside the panel, then U12 = L11^-1 A12 for the panel's block row.  One
-// thread per column: the w entries are gathered through the block
-// permutation into registers, solved and written back.
-// Column col outside the panel: the panel's row swaps (new row t = old row
-// src[t]) applied to its w entries, then U12 = L11^-1 A12 for col >= k + w.
-template <class T>
-__device__ __forceinline__ void swap_trsm_col(T *A, int f, int k, int w, int col,
-                                              const T (*Ld)[PanelWidth<T>::v + 1],
-                                              const int *src)
-{
-    constexpr int NB = PanelWidth<T>::v;
-    T x[NB];
-#pragma unroll
-    for (int t = 0; t < NB; ++t) x[t] = t < w ? A[(long long)(k + src[t]) * f + col] : T(0);
-    if (col >= k + w) {
-#pragma unroll
-        for (int u = 0; u < NB - 1; ++u) {   // by columns of L: an NB-step chain
-            const T xu = x[u];
-#pragma unroll
-            for (int t = u + 1; t < NB; ++t) x[t] -= Ld[t][u] * xu;
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < NB; ++t)
-        if (t < w) A[(long long)(k + t) * f + col] = x[t];
-}
-
-template <class T>
-__device__ __forceinline__ void swap_trsm_cols(T *A, int f, int S, int k, int vo, int chunk,
-                                               const int *__restrict__ ipiv,
-                                               T (*Ld)[PanelWidth<T>::v + 1], int *src)
-{
-    constexpr int NB = PanelWidth<T>::v;
-    const int w = min(NB, S - k);
-    for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-        const int r = e / NB, c = e - r * NB;
-        Ld[r][c] = (r < w && c < w) ? A[(long long)(k + r) * f + k + c] : T(0);
-    }
-    // the panel's pivot rows, loaded by the first NB threads at once (thread 0
-    // loading them one after another would wait out NB dependent load
-    // latencies), then new row t of the block = old row src[t]
-    if (threadIdx.x < NB) src[NB + threadIdx.x] = threadIdx.x < w ? ipiv[vo + k + threadIdx.x] - k : 0;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int t = 0; t < NB; ++t) src[t] = t;
-        for (int t = 0; t < w; ++t) {
-            const int p = src[NB + t];
-            const int u = src[t];
-            src[t] = src[p];
-            src[p] = u;
-        }
-    }
-    __syncthreads();
-    const int col = chunk * blockDim.x + threadIdx.x;
-    if (col >= f || (col >= k && col < k + w)) return;
-    swap_trsm_col<T>(A, f, k, w, col, Ld, src);
-}
-
-// Both panel steps that only read the factored diagonal block, in one launch:
-// blocks [0, nl) compute L21 for kL21Rows rows each, blocks [nl, gridDim.x)
-// apply the row swaps and U12 for kL21Rows columns each.  The two write
-// disjoint parts of the front (rows below the block in its columns; the
-// block's rows outside its columns) and read neither's output.
-template <class T>
-__global__ void __launch_bounds__(kL21Rows) k_l21_trsm(int q0, int k, int nl,
-                                                       const int *__restrict__ S_,
-                                                       const int *__restrict__ f_,
-                                                       const long long *__restrict__ foff,
-                                                       const int *__restrict__ voff, T *F,
-                                                       const int *__restrict__ ipiv)
-{
-    constexpr int NB = PanelWidth<T>::v;
-    __shared__ T D[NB][NB + 1];
-    __shared__ int src[2 * NB];
-    const int q = q0 + blockIdx.y;
-    const int S = S_[q], f = f_[q];
-    if (S <= k) return;
-    T *A = F + foff[q];
-    if ((int)blockIdx.x < nl)
-        l21_rows<T>(A, f, S, k, blockIdx.x, D);
-    else
-        swap_trsm_cols<T>(A, f, S, k, voff[q], blockIdx.x - nl, ipiv, D, src);
-}
-
-// Accumulator of one 64 x 64 output tile of a CTA of 256 threads, fed NB-wide
-// slices of its two operands through shared memory (Smem: a(rr, t) at
-// refA, b(t, cc) at refB; staged by tile_mac, t fastest for A and cc fastest
-// for B, then mac).
-//   float:  CUDA cores, each thread 4 x 4 outputs (rows ty + 16 a, columns
-//           tx + 16 b).
-//   double: FP64 tensor cores, mma.sync m8n8k4 (the one FP64 tensor-core
-//           instruction on sm_100a: tcgen05 has no FP64 kind).  Warp w owns
-//           rows 32 (w / 4) .. + 32 and columns 16 (w % 4) .. + 16, i.e. 4 x 2
-//           8x8 blocks; per k step of 4 a lane holds A[8 mi + g][t], the B
-//           element [t][8 ni + g] and the outputs [8 mi + g][8 ni + 2 t + j]
-//           (g = lane / 4, t = lane % 4).  Row strides of 36 and 72 doubles
-//           spread a warp's 32 fragment reads evenly over the shared-memory
-//           banks (two wavefronts, the minimum for 256 bytes).
-template <class T> struct TileAcc;
-
-template <> struct TileAcc<float> {
-    static constexpr int NB = PanelWidth<float>::v, TL = kGemmTile;
-    struct Smem {
-        float A[NB][TL + 1];
-        float B[NB][TL];
-    };
-    float acc[4][4];
-    __device__ __forceinline__ static float &refA(Smem &s, int rr, int t) { return s.A[t][rr]; }
-    __device__ __forceinline__ static float &refB(Smem &s, int t, int cc) { return s.B[t][cc]; }
-    __device__ __forceinline__ void zero()
-    {
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
-    }
-    __device__ __forceinline__ void mac(const Smem &s)
-    {
-        const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-#pragma unroll 4
-        for (int t = 0; t < NB; ++t) {
-            float av[4], bv[4];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) av[a] = s.A[t][ty + 16 * a];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) bv[b] = s.B[t][tx + 16 * b];
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 4; ++b) acc[a][b] += av[a] * bv[b];
-        }
-    }
-    // fn(rr, cc, value) for every output of the thread
-    template <class Fn> __device__ __forceinline__ void each(Fn fn) const
-    {
-        const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) fn(ty + 16 * a, tx + 16 * b, acc[a][b]);
-    }
-};
-
-__device__ __forceinline__ void dmma_8x8x4(double &c0, double &c1, double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                 : "+d"(c0), "+d"(c1)
-                 : "d"(a), "d"(b));
-}
-
-template <> struct TileAcc<double> {
-    static constexpr int NB = PanelWidth<double>::v, TL = kGemmTile;
-    struct Smem {
-        double A[TL][NB + 4];
-        double B[NB][TL + 8];
-    };
-    double acc[4][2][2];
-    __device__ __forceinline__ static double &refA(Smem &s, int rr, int t) { return s.A[rr][t]; }
-    __device__ __forceinline__ static double &refB(Smem &s, int t, int cc) { return s.B[t][cc]; }
-    __device__ __forceinline__ void zero()
-    {
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-    }
-    __device__ __forceinline__ void mac(const Smem &s)
-    {
-        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-        const int wr = (w >> 2) * 32, wc = (w & 3) * 16;
-#pragma unroll
-        for (int k = 0; k < NB; k += 4) {
-            double a[4], b[2];
-#pragma unroll
-            for (int mi = 0; mi < 4; ++mi) a[mi] = s.A[wr + 8 * mi + g][k + t];
-#pragma unroll
-            for (int ni = 0; ni < 2; ++ni) b[ni] = s.B[k + t][wc + 8 * ni + g];
-#pragma unroll
-            for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 2; ++ni)
-                    dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], a[mi], b[ni]);
-        }
-    }
-    template <class Fn> __device__ __forceinline__ void each(Fn fn) const
-    {
-        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-        const int wr = (w >> 2) * 32, wc = (w & 3) * 16;
-#pragma unroll
-        for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-                    fn(wr + 8 * mi + g, wc + 8 * ni + 2 * t + j, acc[mi][ni][j]);
-    }
-};
-
-// Asynchronous global -> shared copy of one element (cp.async, L1-allocating
-// form: 4- and 8-byte copies need no 16-byte alignment, so any row stride
-// works); ok == false writes zero and reads nothing.
-template <class T>
-__device__ __forceinline__ void cp_async_elem(T *dst, const T *src, bool ok)
-{
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src),
-                 "n"((int)sizeof(T)), "r"(ok ? (int)sizeof(T) : 0));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N> __device__ __forceinline__ void cp_async_wait()
-{
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-// acc += sum over k in [ka, kb) of a(rr, k) b(k, cc), in NB-wide slices
-// through kTileStages shared buffers (sm[0 .. kTileStages)): the copies of
-// the next kTileStages - 1 slices are in flight while the tensor cores (or
-// CUDA cores) work on slice s.  Two buffers leave room for three CTAs per SM
-// in FP64, which hide the copies' latency better than a third buffer.  srcA(rr, k)
-// and srcB(k, cc) give the element's address or nullptr (zero); oneA(rr, k)
-// and oneB(k, cc) mark entries that are 1 instead (a unit diagonal), written
-// after the slice's copies have landed.  base: any valid address (the source
-// of zero-filled copies, never read).
-struct NoOnes {
-    __device__ __forceinline__ bool operator()(int, int) const { return false; }
-};
-
-template <class T, class SA, class SB, class OB, class OA = NoOnes>
-__device__ __forceinline__ void tile_mac(TileAcc<T> &acc, typename TileAcc<T>::Smem *sm, int ka,
-                                         int kb, const T *base, SA srcA, SB srcB, OB oneB,
-                                         OA oneA = OA())
-{
-    constexpr int NB = PanelWidth<T>::v;
-    constexpr int TL = kGemmTile;
-    const int tid = threadIdx.x;
-    const int ns = (kb - ka + NB - 1) / NB;
-    auto stage = [&](int sl) {
-        const int k = ka + sl * NB;
-        typename TileAcc<T>::Smem &b = sm[sl % kTileStages];
-        for (int e = tid; e < TL * NB; e += blockDim.x) {
-            const int rr = e / NB, t = e - rr * NB;
-            const T *p = k + t < kb ? srcA(rr, k + t) : nullptr;
-            cp_async_elem(&TileAcc<T>::refA(b, rr, t), p ? p : base, p != nullptr);
-        }
-        for (int e = tid; e < NB * TL; e += blockDim.x) {
-            const int t = e / TL, cc = e - t * TL;
-            const T *p = k + t < kb ? srcB(k + t, cc) : nullptr;
-            cp_async_elem(&TileAcc<T>::refB(b, t, cc), p ? p : base, p != nullptr);
-        }
-        cp_async_commit();
-    };
-    auto ones = [&](int sl) {
-        const int k = ka + sl * NB;
-        typename TileAcc<T>::Smem &b = sm[sl % kTileStages];
-        for (int e = tid; e < NB * TL; e += blockDim.x) {
-            const int t = e / TL, cc = e - t * TL;
-            if (k + t < kb && oneB(k + t, cc)) TileAcc<T>::refB(b, t, cc) = T(1);
-        }
-        for (int e = tid; e < TL * NB; e += blockDim.x) {
-            const int rr = e / NB, t = e - rr * NB;
-            if (k + t < kb && oneA(rr, k + t)) TileAcc<T>::refA(b, rr, t) = T(1);
-        }
-    };
-    static_assert(kTileStages == 2 || kTileStages == 3, "two or three stages");
-    for (int p = 0; p < kTileStages - 1 && p < ns; ++p) stage(p);
-    for (int sl = 0; sl < ns; ++sl) {
-        // slice sl has landed once at most the later slices already issued pend
-        if (kTileStages == 3 && sl + 1 < ns) cp_async_wait<kTileStages - 2>();
-        else cp_async_wait<0>();
-        ones(sl);
-        __syncthreads();
-        // the buffer of slice sl + kTileStages - 1 held slice sl - 1, which
-        // every thread finished before the barrier above
-        if (sl + kTileStages - 1 < ns) stage(sl + kTileStages - 1);
-        acc.mac(sm[sl % kTileStages]);
-    }
-    __syncthreads();   // the buffers may be reused after the last slice
-}
-
-// One 64 x 64 tile of a trailing update: A[r][c] -= sum_{t in [ka, kb)}
-// A[r][t] A[t][c] for rows [r0, min(r0 + 64, r1)) and columns
-// [c0, min(c0 + 64, c1)).
-template <class T>
-__device__ __forceinline__ void gemm_tile_range(T *A, int f, int r0, int r1, int c0, int c1,
-                                                int ka, int kb, typename TileAcc<T>::Smem *sm)
-{
-    TileAcc<T> acc;
-    acc.zero();
-    tile_mac<T>(
-        acc, sm, ka, kb, A,
-        [&](int rr, int k) -> const T * {
-            const int r = r0 + rr;
-            return r < r1 ? A + (long long)r * f + k : nullptr;
-        },
-        [&](int k, int cc) -> const T * {
-            const int c = c0 + cc;
-            return c < c1 ? A + (long long)k * f + c : nullptr;
-        },
-        [](int, int) { return false; });
-    acc.each([&](int rr, int cc, T v) {
-        const int r = r0 + rr, c = c0 + cc;
-        if (r < r1 && c < c1) A[(long long)r * f + c] -= v;
-    });
-}
-
-// dynamic shared memory of the tile engine's kernels: the operand buffers
-template <class T> constexpr size_t tile_smem_bytes()
-{
-    return kTileStages * sizeof(typename TileAcc<T>::Smem);
-}
-
-// Trailing updates after panel [k, k + w), with delayed updates in
-// super-panels of W columns (a multiple of NB; W = NB is the plain
-// right-looking scheme).  Within the super-panel [k0, E), E = min(k0 + W, S),
-// the panel's rank-w update goes only to the super-panel's remaining columns
-// [kn, E) (all rows below, kn = k + w), and the next panel's rows [kn,
-// kn + w') of the columns beyond it get the delayed contributions of the
-// super-panel's panels so far (rank kn - k0), so that the next panel's swaps
-// and U12 see updated rows; after the super-panel's last panel, one rank-W
-// update covers rows and columns [E, f).  A big trailing block is then read
-// and written once per W columns instead of once per panel.  Tiles are
-// numbered per front for whichever case applies to it; the tile holding the
-// next panel's diagonal block (the first one) factors that panel after its
-// update (panel_factor), which saves the next step's panel launch.
-template <class T>
-__global__ void __launch_bounds__(256) k_gemm(int q0, int k, int W, const int *__restrict__ S_,
-                                              const int *__restrict__ f_,
-                                              const long long *__restrict__ foff,
-                                              const int *__restrict__ voff, T *F, int *ipiv,
-                                              int *perm, int *flag)
-{
-    constexpr int NB = PanelWidth<T>::v;
-    constexpr int TL = kGemmTile;
-    extern __shared__ __align__(16) unsigned char tile_raw[];
-    typename TileAcc<T>::Smem *sm = reinterpret_cast<typename TileAcc<T>::Smem *>(tile_raw);
-    // the next panel's block and pivots reuse the operand buffers once the
-    // tile is done
-    T(*U)[NB + 1] = reinterpret_cast<T(*)[NB + 1]>(tile_raw);
-    int *pv = reinterpret_cast<int *>(tile_raw + sizeof(T) * NB * (NB + 1));
-    const int q = q0 + blockIdx.y;
-    const int S = S_[q], f = f_[q];
-    if (S <= k) return;
-    const int w = min(NB, S - k), kn = k + w;
-    const int k0 = (k / W) * W, E = min(k0 + W, S);
-    T *A = F + foff[q];
-    int t = blockIdx.x;
-    bool first = false;
-    if (kn < E) {
-        const int nr = (f - kn + TL - 1) / TL, nc = (E - kn + TL - 1) / TL;
-        if (t < nr * nc) {
-            gemm_tile_range<T>(A, f, kn + (t / nc) * TL, f, kn + (t % nc) * TL, E, k, kn, sm);
-            first = t == 0;
-        } else {
-            t -= nr * nc;
-            const int wn = min(NB, S - kn), nf = (f - E + TL - 1) / TL;
-            if (t >= nf) return;
-            gemm_tile_range<T>(A, f, kn, kn + wn, E + t * TL, f, k0, kn, sm);
-        }
-    } else {
-        const int rem = f - E;
-        if (rem <= 0) return;
-        const int nt = (rem + TL - 1) / TL;
-        if (t >= nt * nt) return;
-        gemm_tile_range<T>(A, f, E + (t / nt) * TL, f, E + (t % nt) * TL, f, k0, E, sm);
-        first = t == 0;
-    }
-    if (first && kn < S) {
-        __syncthreads();   // the tile's updated entries are visible to the block
-        panel_factor<T>(A, f, S, kn, voff[q], ipiv, perm, flag, U, pv);
-    }
-}
-
-// Explicit inverses of the factored S x S block of every front of a level:
-// strictly lower part <- L11^-1 (unit diagonal implied), upper part incl. the
-// diagonal <- U11^-1, written to the level's scratch and copied back by
-// k_trcopy.  One CTA per (front, column block of CW columns); the column
-// block of each inverse is solved against the identity right-looking: the CTA
-// keeps the S x CW block in shared memory, solves one 32-row diagonal block
-// (one thread per column), then updates every remaining row with a rank-32
-// product (all threads).  With the inverses the solve applies each front by
-// row-parallel products instead of a chain of dependent triangular blocks.
-constexpr int kTrinvThreads = 512;
-// levels with more column blocks than SMs launch k_trinv with this many
-// threads: at about 100 (FP32) / 128 (FP64) registers a 512-thread CTA fills
-// an SM's register file alone, 128-thread CTAs fit four or five per SM, and
-// on those levels resident CTAs matter more than the row updates' thread
-// count
-constexpr int kTrinvThreadsMany = 128;
-constexpr int kTrinvManyCtas = 148;
-template <class T> struct InvWidth;
-template <> struct InvWidth<float> { static constexpr int v = 32; };
-template <> struct InvWidth<double> { static constexpr int v = 16; };
-
-// Columns [c0, c0 + CW) of L11^-1 (unit lower) and U11^-1 of one front's
-// factored pivot block, into X (S x S, row-major); Xs (S x CW) and Lp (S x 33)
-// in shared memory, Dg a 32 x 33 shared tile.
-template <class T>
-__device__ __forceinline__ void trinv_colblock(const T *A, int S, int f, T *X, int c0, T *Xs,
-                                               T *Lp, T (*Dg)[33])
-{
-    constexpr int CW = InvWidth<T>::v;
-    const int cw = min(CW, S - c0);
-    const int tid = threadIdx.x;
-    // ---------------- L11^-1 (unit lower): rows [c0, S)
-    for (int e = tid; e < S * CW; e += blockDim.x) {
-        const int r = e / CW, cc = e - r * CW;
-        Xs[e] = (r == c0 + cc) ? T(1) : T(0);
-    }
-    __syncthreads();
-    for (int r0 = (c0 / 32) * 32; r0 < S; r0 += 32) {
-        const int bh = min(32, S - r0);
-        // the diagonal block and the L panel below it do not depend on each
-        // other: load both in one phase
-        const int rows = S - r0 - bh;
-        for (int e = tid; e < 1024; e += blockDim.x) {
-            const int rr = e >> 5, cc = e & 31;
-            Dg[rr][cc] = (rr < bh && cc < bh) ? A[(long long)(r0 + rr) * f + r0 + cc] : T(0);
-        }
-        for (int e = tid; e < rows * 32; e += blockDim.x) {    // stage L[r0+bh.., r0..r0+32)
-            const int rr = e >> 5, t = e & 31;
-            Lp[rr * 33 + t] = t < bh ? A[(long long)(r0 + bh + rr) * f + r0 + t] : T(0);
-        }
-        __syncthreads();
-        if (tid < CW) {   // diagonal block, one thread per column, column in registers
-            T xr[32];
-#pragma unroll
-            for (int r = 0; r < 32; ++r) xr[r] = r < bh ? Xs[(r0 + r) * CW + tid] : T(0);
-#pragma unroll
-            for (int t = 0; t < 31; ++t) {   // by columns: a 31-step chain
-                const T xt = xr[t];
-#pragma unroll
-                for (int r = t + 1; r < 32; ++r) xr[r] -= Dg[r][t] * xt;
-            }
-#pragma unroll
-            for (int r = 1; r < 32; ++r)
-                if (r < bh) Xs[(r0 + r) * CW + tid] = xr[r];
-        }
-        __syncthreads();
-        for (int e = tid; e < rows * CW; e += blockDim.x) {   // rank-bh update below
-            const int rr = e / CW, cc = e % CW;
-            const T *lr = Lp + rr * 33;
-            T v0 = T(0), v1 = T(0);
-            int t = 0;
-            for (; t + 1 < bh; t += 2) {   // rows r0 .. r0+bh-1 of Xs only
-                v0 += lr[t] * Xs[(r0 + t) * CW + cc];
-                v1 += lr[t + 1] * Xs[(r0 + t + 1) * CW + cc];
-            }
-            if (t < bh) v0 += lr[t] * Xs[(r0 + t) * CW + cc];
-            Xs[(r0 + bh + rr) * CW + cc] -= v0 + v1;
-        }
-        __syncthreads();
-    }
-    for (int e = tid; e < S * CW; e += blockDim.x) {
-        const int r = e / CW, cc = e - r * CW;
-        if (cc < cw && r > c0 + cc) X[(long long)r * S + c0 + cc] = Xs[e];
-    }
-    __syncthreads();
-    // ---------------- U11^-1 (upper): rows [0, c0 + cw)
-    const int rtop = c0 + cw;
-    for (int e = tid; e < rtop * CW; e += blockDim.x) {
-        const int r = e / CW, cc = e - r * CW;
-        Xs[e] = (r == c0 + cc) ? T(1) : T(0);
-    }
-    __syncthreads();
-    for (int r0 = ((rtop - 1) / 32) * 32; r0 >= 0; r0 -= 32) {
-        const int r1 = min(r0 + 32, rtop);
-        const int bh = r1 - r0;
-        for (int e = tid; e < 1024; e += blockDim.x) {
-            const int rr = e >> 5, cc = e & 31;
-            Dg[rr][cc] = (rr < bh && cc < bh) ? A[(long long)(r0 + rr) * f + r0 + cc] : T(0);
-        }
-        for (int e = tid; e < r0 * 32; e += blockDim.x) {      // stage U[0..r0, r0..r0+32)
-            const int rr = e >> 5, t = e & 31;
-            Lp[rr * 33 + t] = t < bh ? A[(long long)rr * f + r0 + t] : T(0);
-        }
-        __syncthreads();
-        if (tid < CW) {   // column in registers
-            T xr[32];
-#pragma unroll
-            for (int r = 0; r < 32; ++r) xr[r] = r < bh ? Xs[(r0 + r) * CW + tid] : T(0);
-#pragma unroll
-            for (int t = 31; t >= 0; --t) {   // by columns, from the bottom row up
-                if (t < bh) {
-                    const T d = Dg[t][t];
-                    const T xt = d != T(0) ? xr[t] / d : T(0);
-                    xr[t] = xt;
-#pragma unroll
-                    for (int r = 0; r < t; ++r) xr[r] -= Dg[r][t] * xt;
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < 32; ++r)
-                if (r < bh) Xs[(r0 + r) * CW + tid] = xr[r];
-        }
-        __syncthreads();
-        for (int e = tid; e < r0 * CW; e += blockDim.x) {   // rank update above
-            const int r = e / CW, cc = e % CW;
-            const T *ur = Lp + r * 33;
-            T v0 = T(0), v1 = T(0);
-            int t = 0;
-            for (; t + 1 < bh; t += 2) {   // rows r0 .. r0+bh-1 of Xs only
-                v0 += ur[t] * Xs[(r0 + t) * CW + cc];
-                v1 += ur[t + 1] * Xs[(r0 + t + 1) * CW + cc];
-            }
-            if (t < bh) v0 += ur[t] * Xs[(r0 + t) * CW + cc];
-            Xs[r * CW + cc] -= v0 + v1;
-        }
-        __syncthreads();
-    }
-    for (int e = tid; e < rtop * CW; e += blockDim.x) {
-        const int r = e / CW, cc = e - r * CW;
-        if (cc < cw && r <= c0 + cc) X[(long long)r * S + c0 + cc] = Xs[e];
-    }
-}
-
-template <class T>
-__global__ void __launch_bounds__(kTrinvThreads) k_trinv(int q0, const int *__restrict__ S_,
-                                                         const long long *__restrict__ foff,
-                                                         const int *__restrict__ f_,
-                                                         const long long *__restrict__ toff,
-                                                         const T *__restrict__ F, T *tmp)
-{
-    constexpr int CW = InvWidth<T>::v;
-    extern __shared__ unsigned char smem_raw[];
-    T *Xs = reinterpret_cast<T *>(smem_raw);    // S x CW
-    T *Lp = Xs + (size_t)S_[q0 + blockIdx.y] * CW;   // S x 33: the 32 columns of the current step
-    __shared__ T Dg[32][33];                     // current 32 x 32 diagonal block
-    const int q = q0 + blockIdx.y;
-    const int S = S_[q], f = f_[q];
-    const int c0 = blockIdx.x * CW;
-    if (c0 >= S) return;
-    trinv_colblock<T>(F + foff[q], S, f, tmp + toff[q], c0, Xs, Lp, Dg);
-}
-
-// The same inversion for separators whose column block does not fit in
-// shared memory: the S x CW block and the S x 33 panel live in a global work
-// space, one slice of S x (CW + 33) per CTA (sstride elements apart).
-constexpr size_t kInvSmemMax = 200 * 1024;
-// grids with one y index per front take at most this many fronts per launch
-// (the grid's y dimension is limited to 65535)
-constexpr int kMaxFrontsY = 65535;
-constexpr int kTrinvThreadsG = 256;
-
-template <class T>
-__global__ void __launch_bounds__(kTrinvThreadsG) k_trinv_g(int q0, const int *__restrict__ S_,
-                                                           const long long *__restrict__ foff,
-                                                           const int *__restrict__ f_,
-                                                           const long long *__restrict__ toff,
-                                                           const T *__restrict__ F, T *tmp,
-                                                           T *work, long long sstride)
-{
-    constexpr int CW = InvWidth<T>::v;
-    __shared__ T Dg[32][33];
-    const int q = q0 + blockIdx.y;
-    const int S = S_[q], f = f_[q];
-    const int c0 = blockIdx.x * CW;
-    if (c0 >= S) return;
-    T *Xs = work + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * sstride;
-    T *Lp = Xs + (size_t)S * CW;
-    trinv_colblock<T>(F + foff[q], S, f, tmp + toff[q], c0, Xs, Lp, Dg);
-}
-
-// Explicit inverses of separators too wide for the shared-memory column
-// blocks (FP64), by 64 x 64 blocks on the tile engine.  With X = L11^-1 and
-// Y = U11^-1 in blocks of 64 (nb blocks), X L11 = I and U11 Y = I give, for
-// s = nb-2 down to 0,
-//   X_is = -sum_{k=s+1..i} X_ik (L_ks X_ss)     (i > s, block column s)
-//   Y_sj = -sum_{k=s+1..j} (Y_ss U_sk) Y_kj     (j > s, block row s)
-// from blocks of later steps and the diagonal blocks' inverses X_kk (unit
-// diagonal, stored strictly below it) and Y_kk.  k_trinv_diag inverts every
-// diagonal block; each step is two launches of k_trinv_step: phase 0 forms
-// W_k = L_ks X_ss and V_sk = Y_ss U_sk in place of L_ks and U_sk (read by
-// this step only; the whole pivot block is replaced by k_trcopy afterwards),
-// phase 1 the products.  Results go to the level's scratch like k_trinv's.
-constexpr int kInvBlk = 64;   // the tile engine's tile
-// separators from this width on are inverted by blocks (fewer dependent
-// steps per CTA than the column-block solves; measured on 362-wide ones)
-constexpr int kBlockedInvMinS = 256;
-constexpr int kTrinvDiagThreads = 128;
-
-template <class T> constexpr size_t trinv_diag_smem() { return 3 * kInvBlk * (kInvBlk + 1) * sizeof(T); }
-
-template <class T>
-__global__ void __launch_bounds__(kTrinvDiagThreads) k_trinv_diag(int q0, const int *__restrict__ S_,
-                                                                  const int *__restrict__ f_,
-                                                                  const long long *__restrict__ foff,
-                                                                  const long long *__restrict__ toff,
-                                                                  const T *__restrict__ F, T *tmp)
-{
-    constexpr int B = kInvBlk;
-    extern __shared__ __align__(16) unsigned char diag_raw[];
-    T (*Ab)[B + 1] = reinterpret_cast<T (*)[B + 1]>(diag_raw);
-    T (*Xs)[B + 1] = Ab + B;
-    T (*Ys)[B + 1] = Xs + B;
-    const int q = q0 + blockIdx.y;
-    const int S = S_[q], f = f_[q], s0 = blockIdx.x * B;
-    if (s0 >= S) return;
-    const int bs = min(B, S - s0), tid = threadIdx.x;
-    const T *A = F + foff[q] + (long long)s0 * f + s0;
-    for (int e = tid; e < B * B; e += blockDim.x) {
-        const int r = e / B, c = e - r * B;
-        Ab[r][c] = (r < bs && c < bs) ? A[(long long)r * f + c] : T(0);
-    }
-    __syncthreads();
-    // One column of an inverse per thread, held in registers and solved by
-    // columns of the block (each finished entry updates all rows after it):
-    // the dependent chain is B steps long instead of B^2 / 2 dependent
-    // products through shared memory.  The padding beyond bs is zero and
-    // leaves the solution's zeros in place.
-    const int c = tid & (B - 1);
-    if (c < bs) {
-        T x[B];
-#pragma unroll
-        for (int r = 0; r < B; ++r) x[r] = r == c ? T(1) : T(0);
-        if (tid < B) {   // column c of L^-1 (unit lower): L x = e_c
-#pragma unroll
-            for (int t = 0; t < B - 1; ++t) {
-                const T xt = x[t];
-#pragma unroll
-                for (int r = t + 1; r < B; ++r) x[r] -= Ab[r][t] * xt;
-            }
-#pragma unroll
-            for (int r = 0; r < B; ++r) Xs[r][c] = x[r];
-        } else {         // column c of U^-1: U x = e_c from the bottom row up
-#pragma unroll
-            for (int t = B - 1; t >= 0; --t) {
-                const T d = Ab[t][t];
-                const T xt = d != T(0) ? x[t] / d : T(0);
-                x[t] = xt;
-#pragma unroll
-                for (int r = 0; r < t; ++r) x[r] -= Ab[r][t] * xt;
-            }
-#pragma unroll
-            for (int r = 0; r < B; ++r) Ys[r][c] = x[r];
-        }
-    }
-    __syncthreads();
-    T *X = tmp + toff[q] + (long long)s0 * S + s0;
-    for (int e = tid; e < bs * bs; e += blockDim.x) {
-        const int r = e / bs, cc = e - r * bs;
-        X[(long long)r * S + cc] = r > cc ? Xs[r][cc] : Ys[r][cc];
-    }
-}
-
-// One step s of the blocked inversion (see k_trinv_diag); grid: (2 half,
-// fronts), tiles [0, half) the blocks k = s + 1 + t of L's block column s,
-// [half, 2 half) those of U's block row s.
-template <class T>
-__global__ void __launch_bounds__(256) k_trinv_step(int q0, int s, int phase, int half,
-                                                    const int *__restrict__ S_,
-                                                    const int *__restrict__ f_,
-                                                    const long long *__restrict__ foff,
-                                                    const long long *__restrict__ toff, T *F,
-                                                    T *tmp)
-{
-    constexpr int B = kInvBlk;
-    extern __shared__ __align__(16) unsigned char tile_raw[];
-    typename TileAcc<T>::Smem *sm = reinterpret_cast<typename TileAcc<T>::Smem *>(tile_raw);
-    const int q = q0 + blockIdx.y;
-    const int S = S_[q], f = f_[q], nb = (S + B - 1) / B;
-    int t = blockIdx.x;
-    const bool up = t >= half;
-    if (up) t -= half;
-    const int k = s + 1 + t;
-    if (k >= nb) return;
-    T *A = F + foff[q];
-    T *X = tmp + toff[q];
-    const int s0 = s * B, k0 = k * B, se = s0 + B, ke = min(k0 + B, S);
-    TileAcc<T> acc;
-    acc.zero();
-    if (phase == 0 && !up) {          // W_k = L_ks X_ss (in place of L_ks)
-        tile_mac<T>(
-            acc, sm, s0, se, A,
-            [&](int rr, int j) -> const T * {
-                const int r = k0 + rr;
-                return r < ke ? A + (long long)r * f + j : nullptr;
-            },
-            [&](int j, int cc) -> const T * {
-                return j > s0 + cc ? X + (long long)j * S + s0 + cc : nullptr;
-            },
-            [&](int j, int cc) { return j == s0 + cc; });
-        acc.each([&](int rr, int cc, T v) {
-            if (k0 + rr < ke) A[(long long)(k0 + rr) * f + s0 + cc] = v;
-        });
-    } else if (phase == 0) {          // V_sk = Y_ss U_sk (in place of U_sk)
-        tile_mac<T>(
-            acc, sm, s0, se, A,
-            [&](int rr, int j) -> const T * {
-                return j >= s0 + rr ? X + (long long)(s0 + rr) * S + j : nullptr;
-            },
-            [&](int j, int cc) -> const T * {
-                const int c = k0 + cc;
-                return c < ke ? A + (long long)j * f + c : nullptr;
-            },
-            NoOnes());
-        acc.each([&](int rr, int cc, T v) {
-            if (k0 + cc < ke) A[(long long)(s0 + rr) * f + k0 + cc] = v;
-        });
-    } else if (!up) {                 // X_ks = -sum_{m=s+1..k} X_km W_m
-        tile_mac<T>(
-            acc, sm, se, ke, A,
-            [&](int rr, int j) -> const T * {
-                const int r = k0 + rr;
-                if (r >= ke || (j >= k0 && j >= r)) return nullptr;   // X_kk: strictly lower
-                return X + (long long)r * S + j;
-            },
-            [&](int j, int cc) -> const T * { return A + (long long)j * f + s0 + cc; },
-            NoOnes(), [&](int rr, int j) { return k0 + rr == j; });
-        acc.each([&](int rr, int cc, T v) {
-            if (k0 + rr < ke) X[(long long)(k0 + rr) * S + s0 + cc] = -v;
-        });
-    } else {                          // Y_sk = -sum_{m=s+1..k} V_sm Y_mk
-        tile_mac<T>(
-            acc, sm, se, ke, A,
-            [&](int rr, int j) -> const T * { return A + (long long)(s0 + rr) * f + j; },
-            [&](int j, int cc) -> const T * {
-                const int c = k0 + cc;
-                if (c >= ke || (j >= k0 && j > c)) return nullptr;    // Y_kk: upper
-                return X + (long long)j * S + c;
-            },
-            NoOnes());
-        acc.each([&](int rr, int cc, T v) {
-            if (k0 + cc < ke) X[(long long)(s0 + rr) * S + k0 + cc] = -v;
-        });
-    }
-}
-
-// Inverted S x S blocks of the level's fronts: scratch -> factor storage.
-template <class T>
-__global__ void k_trcopy(int q0, const int *__restrict__ S_, const int *__restrict__ f_,
-                         const long long *__restrict__ foff, const long long *__restrict__ toff,
-                         const T *__restrict__ tmp, T *F)
-{
-    const int q = q0 + blockIdx.y;
-    const int S = S_[q], f = f_[q];
-    const T *src = tmp + toff[q];
-    T *dst = F + foff[q];
-    const long long tot = (long long)S * S;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < tot;
-         e += (long long)gridDim.x * blockDim.x) {
-        const int r = (int)(e / S), c = (int)(e - (long long)r * S);
-        dst[(long long)r * f + c] = src[e];
-    }
-}
-
-// FP64 factors rounded to FP32 (the solve of the mixed form with FP64
-// factorization).
-__global__ void k_round_f32(const double *__restrict__ a, float *__restrict__ b, long long n)
-{
-    V2D_GRID_STRIDE(i, n) { b[i] = (float)a[i]; }
-}
-
-// G = L21 L11^-1 (rows [S, f) x columns [0, S)) and H = U11^-1 U12 (rows
-// [0, S) x columns [S, f)) of every front of a level, from the inverted pivot
-// block, into the level's scratch (G row-major m x S, then H S x m; copied over
-// L21 and U12 by k_ghcopy: each tile of G reads L21 entries that other tiles
-// overwrite).  One CTA per 64 x 64 output tile (TileAcc: CUDA cores in FP32,
-// FP64 tensor cores in FP64); the triangular factor bounds the inner range (G: k >= c0,
-// with L11^-1's unit diagonal; H: k >= r0).  Grid: (tiles of G then of H for
-// the level's largest front, fronts).
-template <class T>
-__global__ void __launch_bounds__(256) k_gh(int q0, const int *__restrict__ S_,
-                                            const int *__restrict__ f_,
-                                            const long long *__restrict__ foff,
-                                            const long long *__restrict__ goff, const T *F, T *gh)
-{
-    constexpr int TL = kGemmTile;
-    extern __shared__ __align__(16) unsigned char tile_raw[];
-    typename TileAcc<T>::Smem *sm = reinterpret_cast<typename TileAcc<T>::Smem *>(tile_raw);
-    const int q = q0 + blockIdx.y;
-    const int S = S_[q], f = f_[q], m = f - S;
-    if (m <= 0) return;
-    const int ts = (S + TL - 1) / TL, tm = (m + TL - 1) / TL;
-    int t = blockIdx.x;
-    const bool isG = t < tm * ts;
-    if (!isG) t -= tm * ts;
-    if (t >= tm * ts) return;
-    const T *A = F + foff[q];
-    T *out = gh + goff[q];
-    int r0, c0, kb;
-    if (isG) {
-        r0 = S + (t / ts) * TL;
-        c0 = (t % ts) * TL;
-        kb = c0;
-    } else {
-        r0 = (t / tm) * TL;
-        c0 = S + (t % tm) * TL;
-        kb = r0;
-    }
-    TileAcc<T> acc;
-    acc.zero();
-    // G: L21 rows times L11^-1 (strictly lower part stored, unit diagonal);
-    // H: U11^-1 (upper part with the diagonal) times U12
-    tile_mac<T>(
-        acc, sm, kb, S, A,
-        [&](int rr, int kk) -> const T * {
-            const int r = r0 + rr;
-            return (isG ? r < f : (r < S && kk >= r)) ? A + (long long)r * f + kk : nullptr;
-        },
-        [&](int kk, int cc) -> const T * {
-            const int c = c0 + cc;
-            return (isG ? (c < S && kk > c) : c < f) ? A + (long long)kk * f + c : nullptr;
-        },
-        [&](int kk, int cc) { return isG && kk == c0 + cc; });
-    acc.each([&](int rr, int cc, T v) {
-        const int r = r0 + rr, col = c0 + cc;
-        if (isG) {
-            if (r < f && col < S) out[(long long)(r - S) * S + col] = v;
-        } else if (r < S && col < f) {
-            out[(long long)m * S + (long long)r * m + (col - S)] = v;
-        }
-    });
-}
-
-// G and H of the level's fronts: scratch -> factor storage.
-template <class T>
-__global__ void k_ghcopy(int q0, const int *__restrict__ S_, const int *__restrict__ f_,
-                         const long long *__restrict__ foff, const long long *__restrict__ goff,
-                         const T *__restrict__ gh, T *F)
-{
-    const int q = q0 + blockIdx.y;
-    const int S = S_[q], f = f_[q], m = f - S;
-    const T *src = gh + goff[q];
-    T *dst = F + foff[q];
-    const long long ng = (long long)m * S, tot = 2 * ng;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < tot;
-         e += (long long)gridDim.x * blockDim.x) {
-        long long r, c;
-        if (e < ng) {
-            r = S + e / S;
-            c = e % S;
-        } else {
-            r = (e - ng) / m;
-            c = S + (e - ng) % m;
-        }
-        dst[r * f + c] = src[e];
-    }
-}
-
 // ------------------------------------------------------------------ solve
-// After the factorization each front's storage holds, row-major f x f:
-//   [0,S) x [0,S)   L11^-1 strictly below the diagonal (unit diagonal implied)
-//                   and U11^-1 on and above it,
-//   [S,f) x [0,S)   G = L21 L11^-1,
-//   [0,S) x [S,f)   H = U11^-1 U12,
+// After the factorization each front's storage holds, row-major f x f,
+//   [0,S) x [0,S)   A11^-1,
+//   [S,f) x [0,S)   -G, G = A21 A11^-1,
+//   [0,S) x [S,f)   H = A11^-1 A12,
 // so every row of the solve is one contiguous dot product with a vector
-// gathered once per work item:
-//   forward,  r <  S:  z_r = t_r + F[r, 0:r] . t[0:r]      t = P w_FS (permuted)
-//             r >= S:  u_r = w_r - F[r, 0:S] . t[0:S]      contribution to the parent
-//   backward, r <  S:  x_r = F[r, r:f] . v[r:f]            v = (z, -x_struct)
+// gathered once per work item (t = the right-hand side on the pivots):
+//   forward,  r <  S:  z_r = t_r (kept for the backward sweep)
+//             r >= S:  u_r = w_r + F[r, 0:S] . t[0:S]      contribution to the parent
+//   backward, r <  S:  x_r = F[r, 0:f] . v[0:f]            v = (t, -x_struct)
 // A front's forward rows need only its children's contributions and its
 // backward rows only its own z and its ancestors' x: one dependent step per
-// level and sweep.  G and H hold as many entries as L21 and U12, so a solve
+// level and sweep.  G and H hold as many entries as A21 and A12, so a solve
 // still reads sum S (2f - S) factor entries.
 
 __device__ __forceinline__ bool stopped(const int *a, const int *b)
@@ -2180,9 +1088,9 @@ __device__ __forceinline__ void row_range(bool fwd, int r, int S, int f, int &lo
 {
     if (fwd) {
         lo = 0;
-        hi = r < S ? r : S;
+        hi = r < S ? 0 : S;
     } else {
-        lo = r;
+        lo = 0;
         hi = f;
     }
 }
@@ -2197,11 +1105,12 @@ struct SolveItemCtx {
     int kind;    // 0 forward rows, 1 backward rows, 2 forward gather, 3 backward gather
     bool gath;   // rows of a front whose gather item ran (its vectors are in tw)
     int q, S, f, vo, rbeg, rend;
+    int r0;      // first row with a product (forward: the first contribution row)
     const T *A;
-    // staged gather (forward: vars/perm/child maps; backward: struct vars)
+    // staged gather (forward: vars and child maps; backward: struct vars)
     bool staged;
     int ch[2], m[2], uof[2];
-    int pi[kGatherRegs], mp[2][kGatherRegs], xi[kGatherRegs];
+    int mp[2][kGatherRegs], xi[kGatherRegs];
     T rsb[kGatherRegs];
     // this warp's single row, if the item has at most one row per warp
     bool onerow;
@@ -2224,8 +1133,9 @@ struct SolveItemCtx {
         A = F + D.foff[q];
         const int tid = threadIdx.x, nt = blockDim.x, wid = tid >> 5, nw = nt >> 5;
         const int *vars = D.vars + vo;
-        onerow = kind < 2 && rend - rbeg <= nw;
-        const int r = rbeg + wid;
+        r0 = fwd ? max(rbeg, S) : rbeg;
+        onerow = kind < 2 && rend - r0 <= nw;
+        const int r = r0 + wid;
         if (onerow && r < rend) {
             int lo, hi;
             row_range(fwd, r, S, f, lo, hi);
@@ -2252,7 +1162,6 @@ struct SolveItemCtx {
                 for (int k = 0; k < kGatherRegs; ++k) {
                     const int p = tid + k * nt;
                     vi[k] = p < S ? vars[p] : -1;
-                    pi[k] = p < S ? D.perm[vo + p] : 0;
 #pragma unroll
                     for (int sl = 0; sl < 2; ++sl) mp[sl][k] = p < m[sl] ? D.cbmap[uof[sl] + p] : 0;
                 }
@@ -2273,10 +1182,9 @@ struct SolveItemCtx {
     }
 
     // Forward gather: w (f entries: scaled b on the fully summed rows plus
-    // the children's contributions), t = P w_FS, in shared memory.
+    // the children's contributions) in shared memory; t is its first S.
     __device__ __forceinline__ void gather_w(const MfDev &D, const T *b,
-                                             const double *__restrict__ rs, const T *upd, T *w,
-                                             T *t)
+                                             const double *__restrict__ rs, const T *upd, T *w)
     {
         const int tid = threadIdx.x, nt = blockDim.x;
         if (staged) {
@@ -2301,9 +1209,6 @@ struct SolveItemCtx {
                     if (tid + k * nt < m[sl]) w[mp[sl][k]] += uv[sl][k];
                 __syncthreads();
             }
-#pragma unroll
-            for (int k = 0; k < kGatherRegs; ++k)
-                if (tid + k * nt < S) t[tid + k * nt] = w[pi[k]];
         } else {
             // wide fronts: the same in batches of kGatherRegs entries per
             // thread, each batch's index loads issued before its gathers
@@ -2342,17 +1247,7 @@ struct SolveItemCtx {
                 }
                 __syncthreads();
             }
-            for (int i0 = tid; i0 < S; i0 += kGatherRegs * nt) {
-                int pk[kGatherRegs];
-#pragma unroll
-                for (int k = 0; k < kGatherRegs; ++k)
-                    pk[k] = i0 + k * nt < S ? D.perm[vo + i0 + k * nt] : -1;
-#pragma unroll
-                for (int k = 0; k < kGatherRegs; ++k)
-                    if (pk[k] >= 0) t[i0 + k * nt] = w[pk[k]];
-            }
         }
-        __syncthreads();
     }
 
     // -x on the struct variables [S, f) into dst[0, f - S), in batches of
@@ -2383,39 +1278,33 @@ struct SolveItemCtx {
     }
 
     // Forward rows: t from the gather item (gathered fronts) or gathered
-    // here; then z_r = t_r + F[r, 0:r] t on pivot rows and u_r = w_r -
-    // F[r, 0:S] t on contribution rows.
+    // here; then z_r = t_r on pivot rows and u_r = w_r - G[r, 0:S] t on
+    // contribution rows.
     __device__ __forceinline__ void run_fwd(const MfDev &D, const T *b,
-                                            const double *__restrict__ rs, T *zbuf, T *upd, T *w,
-                                            T *t)
+                                            const double *__restrict__ rs, T *zbuf, T *upd, T *w)
     {
         T *uo = upd + D.uoff[q] - S;   // row r >= S -> uo[r]
+        const T *tw = (const T *)D.tw + vo;
         if (gath) {
-            const T *tw = (const T *)D.tw + vo;
-            for (int i = threadIdx.x; i < S; i += blockDim.x) t[i] = __ldcg(tw + i);
+            for (int i = threadIdx.x; i < S; i += blockDim.x) w[i] = __ldcg(tw + i);
             __syncthreads();
-            rows(t, [&](int r, T v) {
-                if (r < S) zbuf[vo + r] = t[r] + v;
-                else uo[r] = __ldcg(tw + r) - v;
-            });
-            return;
+        } else {
+            gather_w(D, b, rs, upd, w);
         }
-        gather_w(D, b, rs, upd, w, t);
-        rows(t, [&](int r, T v) {
-            if (r < S) zbuf[vo + r] = t[r] + v;
-            else uo[r] = w[r] - v;
-        });
+        for (int r = rbeg + (int)threadIdx.x; r < min(rend, S); r += blockDim.x) zbuf[vo + r] = w[r];
+        if (gath) rows(w, [&](int r, T v) { uo[r] = __ldcg(tw + r) + v; });
+        else rows(w, [&](int r, T v) { uo[r] = w[r] + v; });
     }
 
     // Forward gather item: t on the pivot positions and w on the
     // contribution rows into tw, once for all of the front's row items.
     __device__ __forceinline__ void run_gather_fwd(const MfDev &D, const T *b,
                                                    const double *__restrict__ rs, const T *upd,
-                                                   T *w, T *t)
+                                                   T *w)
     {
-        gather_w(D, b, rs, upd, w, t);
+        gather_w(D, b, rs, upd, w);
         T *tw = (T *)D.tw + vo;
-        for (int i = threadIdx.x; i < f; i += blockDim.x) tw[i] = i < S ? t[i] : w[i];
+        for (int i = threadIdx.x; i < f; i += blockDim.x) tw[i] = w[i];
     }
 
     // Backward gather item: -x on the front's struct variables into tw.
@@ -2424,7 +1313,7 @@ struct SolveItemCtx {
         gather_struct_x(D, x, (T *)D.tw + vo + S);
     }
 
-    // Backward: v = (z, -x on the front's struct variables); then the rows.
+    // Backward: v = (t, -x on the front's struct variables); then the rows.
     __device__ __forceinline__ void run_bwd(const MfDev &D, const T *zbuf, T *x, T *v)
     {
         const int tid = threadIdx.x, nt = blockDim.x, mm = f - S;
@@ -2452,8 +1341,8 @@ struct SolveItemCtx {
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
         // one row per thread: short FP32 rows only (a warp's loads touch 32
         // rows at once, which pays only while the rows stay in L1)
-        if (fwd && f <= kThreadRowMaxF && 2 * (rend - rbeg) >= (int)blockDim.x) {
-            for (int r = rbeg + (int)threadIdx.x; r < rend; r += blockDim.x) {
+        if (fwd && f <= kThreadRowMaxF && 2 * (rend - r0) >= (int)blockDim.x) {
+            for (int r = r0 + (int)threadIdx.x; r < rend; r += blockDim.x) {
                 int lo, hi;
                 row_range(fwd, r, S, f, lo, hi);
                 const T *row = A + (long long)r * f;
@@ -2471,8 +1360,8 @@ struct SolveItemCtx {
             }
             return;
         }
-        if (rend - rbeg <= nw) {
-            const int r = rbeg + wid;
+        if (rend - r0 <= nw) {
+            const int r = r0 + wid;
             if (r < rend) {
                 int lo, hi;
                 row_range(fwd, r, S, f, lo, hi);
@@ -2493,7 +1382,7 @@ struct SolveItemCtx {
         constexpr int G = R >= 32 ? 8 : 4;   // rows per warp in flight (register budget)
         // column chunks per row in flight: 2 in the small-register forms
         constexpr int KC = (R < RowRegs<T>::v || G >= 8) ? 2 : 4;
-        for (int r = rbeg + wid; r < rend; r += G * nw) {
+        for (int r = r0 + wid; r < rend; r += G * nw) {
             const T *p[G];
             int bb[G], ee[G], rr[G];
 #pragma unroll
@@ -2529,13 +1418,13 @@ struct SolveItemDev {
 template <class T, int R>
 __device__ __forceinline__ void run_item(SolveItemCtx<T, R> &c, const MfDev &D, const T *b,
                                          const double *__restrict__ rs, T *zbuf, T *upd, T *x,
-                                         T *smem, int wcap)
+                                         T *smem)
 {
-    // shared memory: w (wcap entries, the largest front of the launch), then t
+    // shared memory: w (forward) or v (backward), up to the launch's largest front
     switch (c.kind) {
-    case 0: c.run_fwd(D, b, rs, zbuf, upd, smem, smem + wcap); break;
+    case 0: c.run_fwd(D, b, rs, zbuf, upd, smem); break;
     case 1: c.run_bwd(D, zbuf, x, smem); break;
-    case 2: c.run_gather_fwd(D, b, rs, upd, smem, smem + wcap); break;
+    case 2: c.run_gather_fwd(D, b, rs, upd, smem); break;
     default: c.run_gather_bwd(D, x); break;
     }
 }
@@ -2553,7 +1442,7 @@ __global__ void __launch_bounds__(kSolveThreads, 2) k_solve_level(
     const SolveItemDev it = items[i0 + blockIdx.x];
     SolveItemCtx<T> c;
     c.pre(D, F, b, rs, it.x.x, it.z.w, it.x.y, it.x.z, it.x.w);
-    run_item(c, D, b, rs, zbuf, upd, x, smem, D.maxf);
+    run_item(c, D, b, rs, zbuf, upd, x, smem);
 }
 
 // The split form's lower-level launches: CTA size and resident CTAs per SM.
@@ -2617,12 +1506,12 @@ __device__ __forceinline__ bool wait_count(const int *ctr, int target, volatile 
 // forward items, the upper levels, the lower levels' backward items as three
 // launches in stream order -- an item then only waits for items of its own
 // launch or of an earlier, finished one.  The lower launches use NT = 128
-// threads and shared memory for their own largest front (wcap), so more of
+// threads and shared memory for their own largest front, so more of
 // their many small items are in flight per SM.
 template <class T, int R, int MINB, int NT = kSolveThreads>
 __global__ void __launch_bounds__(NT, MINB) k_solve_flow(
     const MfDev D, const T *F, const T *b, const double *__restrict__ rs, T *zbuf, T *upd, T *x,
-    const SolveItemDev *__restrict__ items, int item0, int item1, int wcap, int *ctr, int nctr,
+    const SolveItemDev *__restrict__ items, int item0, int item1, int *ctr, int nctr,
     int slot, MfBarrier *bar, const int *stop_a, const int *stop_b, unsigned long long *trace)
 {
     if (stopped(stop_a, stop_b)) return;   // the flags are the same for every CTA
@@ -2655,7 +1544,7 @@ __global__ void __launch_bounds__(NT, MINB) k_solve_flow(
         __syncthreads();
         if (!ok_s) return;
         if (trace && threadIdx.x == 0) trace[3 * i + 1] = globaltimer_ns();
-        run_item(c, D, b, rs, zbuf, upd, x, smem, wcap);
+        run_item(c, D, b, rs, zbuf, upd, x, smem);
         // the barrier orders every thread's writes before thread 0's release
         // additions (cumulative at GPU scope), which the waiters' acquire
         // loads pair with
@@ -2672,12 +1561,11 @@ __global__ void __launch_bounds__(NT, MINB) k_solve_flow(
 // The transposed solve is the adjoint of the solve's steps taken in reverse
 // order.  Bottom-up (adjoint of the backward sweep): the front gathers g on
 // its fully summed variables plus its children's contributions (the same
-// contribution-block maps as the forward sweep), forms ybar = U11^-T acc_FS
+// contribution-block maps as the forward sweep), forms ybar = A11^-T acc_FS
 // (kept in zbuf) and passes acc_CB - H^T acc_FS up.  Top-down (adjoint of the
 // forward sweep): the front takes its parent's adjoint right-hand side
-// upd_bar on its contribution rows, t = L11^-T ybar - G^T upd_bar (unit
-// diagonal), scatters t through the row permutation and writes
-// lambda = rs .* w_bar on its fully summed variables.  One CTA per front; the
+// upd_bar on its contribution rows, t = ybar - G^T upd_bar, and writes
+// lambda = rs .* t on its fully summed variables.  One CTA per front; the
 // transposed products read the factor rows column-wise (one thread per
 // column, coalesced across the warp).
 template <class T>
@@ -2704,9 +1592,9 @@ __global__ void __launch_bounds__(kSolveThreads) k_tup_front(int q0, const MfDev
         }
         __syncthreads();
     }
-    for (int j = tid; j < S; j += blockDim.x) {     // ybar = Uinv^T acc_FS
+    for (int j = tid; j < S; j += blockDim.x) {     // ybar = A11^-T acc_FS
         T v = T(0);
-        for (int i = 0; i <= j; ++i) v += A[(long long)i * f + j] * acc[i];
+        for (int i = 0; i < S; ++i) v += A[(long long)i * f + j] * acc[i];
         yb[j] = v;
     }
     __syncthreads();
@@ -2726,7 +1614,6 @@ __global__ void __launch_bounds__(kSolveThreads) k_tdown_front(int q0, const MfD
 {
     extern __shared__ unsigned char smem_raw[];
     T *wbar = reinterpret_cast<T *>(smem_raw);  // f
-    T *v = wbar + D.maxf;                         // f: (ybar, -upd_bar)
     const int q = q0 + blockIdx.x;
     const int S = D.S[q], f = D.f[q], vo = D.voff[q], m = f - S;
     const T *A = F + D.foff[q];
@@ -2736,16 +1623,13 @@ __global__ void __launch_bounds__(kSolveThreads) k_tdown_front(int q0, const MfD
     for (int k = tid; k < m; k += blockDim.x) {     // upd_bar from the parent
         const T u = pa >= 0 ? wb[D.voff[pa] + D.cbmap[D.uoff[q] + k]] : T(0);
         wbar[S + k] = u;
-        v[S + k] = -u;
     }
-    for (int j = tid; j < S; j += blockDim.x) v[j] = zbuf[vo + j];
     __syncthreads();
-    const int *perm = D.perm + vo;
-    // t = Linv^T ybar - G^T upd_bar: column i of rows (i, f); w_bar[perm[i]] = t
+    // t = ybar - G^T upd_bar: column i of the stored -G
     for (int i = tid; i < S; i += blockDim.x) {
-        T t = v[i];
-        for (int j = i + 1; j < f; ++j) t += A[(long long)j * f + i] * v[j];
-        wbar[perm[i]] = t;
+        T t = zbuf[vo + i];
+        for (int j = S; j < f; ++j) t += A[(long long)j * f + i] * wbar[j];
+        wbar[i] = t;
     }
     __syncthreads();
     for (int p = tid; p < f; p += blockDim.x) wb[vo + p] = wbar[p];
@@ -2796,14 +1680,17 @@ int mf_factor_create(const MfPlan *P, int fp32, int fact64, MfFactor **out)
     if (M->fact64) grab(&M->F32, (size_t)P->ftotal * sizeof(float));
     grab(&M->upd, (size_t)P->utotal * es);
     grab(&M->z, (size_t)P->vtotal * es);
-    grab(&M->tmp, (size_t)P->tmax * esf);
-    grab(&M->gh, (size_t)P->gmax * esf);
+    long long cols = 0;   // front variables of the largest level
+    for (int L = 0; L < P->nlevel; ++L) {
+        long long v = 0;
+        for (int q = P->lvl_off[L]; q < P->lvl_off[L + 1]; ++q) v += P->f[q];
+        cols = std::max(cols, v);
+    }
+    grab(&M->cols, (size_t)cols * kPiv * esf);
     grab((void **)&M->sctr, (size_t)(P->nctr + kFlowSlots) * sizeof(int));
     grab(&M->wb, (size_t)P->vtotal * es);
     grab(&M->tw, (size_t)P->vtotal * es);
     grab((void **)&M->rs, (size_t)P->n * sizeof(double));
-    grab((void **)&M->ipiv, (size_t)P->vtotal * sizeof(int));
-    grab((void **)&M->perm, (size_t)P->vtotal * sizeof(int));
     grab((void **)&M->flag, sizeof(int));
     grab((void **)&M->bar, sizeof(MfBarrier));
     if (e == cudaSuccess) e = cudaMemset(M->bar, 0, sizeof(MfBarrier));
@@ -2813,42 +1700,21 @@ int mf_factor_create(const MfPlan *P, int fp32, int fact64, MfFactor **out)
         mf_factor_destroy(M);
         return V2D_ENOMEM;
     }
-    // dynamic shared memory of the solve and inversion kernels (set once,
+    // dynamic shared memory of the solve and factorization kernels (set once,
     // outside any stream capture)
-    const size_t solve = (size_t)(P->maxf + P->maxS) * es;
-    const int cw = esf == sizeof(float) ? InvWidth<float>::v : InvWidth<double>::v;
-    // shared-memory inversion where its column block fits, the global work
-    // space elsewhere (sized for the largest such level)
-    size_t inv = 0, inv_g = 0;
-    for (int L = 0; L < P->nlevel; ++L) {
-        const size_t sl = (size_t)P->lvl_maxS[L] * (cw + 33);
-        if (sl * esf <= kInvSmemMax) {
-            inv = std::max(inv, sl * esf);
-        } else if (esf == sizeof(float)) {   // FP64 inverts these by blocks in place
-            const size_t nbc = (P->lvl_maxS[L] + cw - 1) / cw;
-            inv_g = std::max(inv_g, nbc * (size_t)(P->lvl_off[L + 1] - P->lvl_off[L]) * sl);
-        }
-    }
-    if (solve > 227 * 1024) {
+    const size_t solve = (size_t)P->maxf * es;
+    if (solve + P->maxS * es > 227 * 1024) {
         set_error("mf_factor: front of %d unknowns (separator %d) exceeds shared memory",
                   P->maxf, P->maxS);
         mf_factor_destroy(M);
         return V2D_EARG;
     }
-    if (inv_g > 0) {
-        cudaError_t ge = cudaMalloc(&M->inv_g, inv_g * esf);
-        if (ge != cudaSuccess) {
-            set_error("mf_factor: inversion work space of %.1f MB: %s", inv_g * esf / 1e6,
-                      cudaGetErrorString(ge));
-            mf_factor_destroy(M);
-            return V2D_ENOMEM;
-        }
-    }
     auto attr = [&](const void *fn, size_t bytes) {
         if (e == cudaSuccess) e = raise_dyn_smem(fn, bytes);
     };
-    const size_t tsolve = (size_t)2 * P->maxf * es;   // transposed solve: two f vectors
-    if (tsolve > 227 * 1024) {
+    // transposed solve: an f and an S vector (limit kept at two f vectors)
+    const size_t tsolve = (size_t)(P->maxf + P->maxS) * es;
+    if (2 * P->maxf * es > 227 * 1024) {
         set_error("mf_factor: front of %d unknowns exceeds shared memory (transposed solve)",
                   P->maxf);
         mf_factor_destroy(M);
@@ -2867,8 +1733,13 @@ int mf_factor_create(const MfPlan *P, int fp32, int fact64, MfFactor **out)
         attr((const void *)k_tup_front<double>, tsolve);
         attr((const void *)k_tdown_front<double>, tsolve);
     }
-    if (esf == sizeof(float)) attr((const void *)k_trinv<float>, inv);
-    else attr((const void *)k_trinv<double>, inv);
+    if (esf == sizeof(float)) {
+        attr((const void *)k_row_block<float>, tile_smem_bytes<float>());
+        attr((const void *)k_update<float>, tile_smem_bytes<float>());
+    } else {
+        attr((const void *)k_row_block<double>, tile_smem_bytes<double>());
+        attr((const void *)k_update<double>, tile_smem_bytes<double>());
+    }
     if (e != cudaSuccess) {
         set_error("mf_factor: %s", cudaGetErrorString(e));
         mf_factor_destroy(M);
@@ -2910,8 +1781,8 @@ void mf_factor_destroy(MfFactor *M)
 {
     if (!M) return;
     if (M->graph) cudaGraphExecDestroy(M->graph);
-    void *ptrs[] = {M->F,    M->F32,  M->upd,  M->z,    M->tmp,   M->gh,    M->wb,  M->tw,
-                    M->rs,   M->ipiv, M->perm, M->flag, M->bar,  M->inv_g, M->sctr};
+    void *ptrs[] = {M->F,  M->F32, M->upd,  M->z,   M->cols, M->wb,
+                    M->tw, M->rs,  M->flag, M->bar, M->sctr};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     delete M;
@@ -2922,7 +1793,7 @@ MfDev mf_dev(const MfPlan *P, const MfFactor *M)
     MfDev D;
     D.S = P->d_S; D.f = P->d_f; D.voff = P->d_voff; D.uoff = P->d_uoff;
     D.child0 = P->d_child0; D.child1 = P->d_child1; D.parent = P->d_parent; D.foff = P->d_foff;
-    D.vars = P->d_vars; D.cbmap = P->d_cbmap; D.perm = M->perm;
+    D.vars = P->d_vars; D.cbmap = P->d_cbmap;
     D.maxS = P->maxS; D.maxf = P->maxf;
     D.tw = M->tw;
     return D;
@@ -2933,18 +1804,12 @@ static int factor_launches(const MfPlan *P, MfFactor *M, const int *rowptr, cons
                            cudaStream_t s, cudaEvent_t *ev = nullptr, int *codes = nullptr,
                            int cap = 0, int *nev_out = nullptr)
 {
-    constexpr int NB = PanelWidth<T>::v;
-    T *F = (T *)M->F;
+    T *F = (T *)M->F, *C = (T *)M->cols;
     long long launches = 0;
-    const size_t tile_smem = tile_smem_bytes<T>();
-    V2D_CUDA_TRY(raise_dyn_smem((const void *)k_gemm<T>, tile_smem));
-    V2D_CUDA_TRY(raise_dyn_smem((const void *)k_gh<T>, tile_smem));
-    V2D_CUDA_TRY(raise_dyn_smem((const void *)k_trinv_step<T>, tile_smem));
-    V2D_CUDA_TRY(raise_dyn_smem((const void *)k_trinv_diag<T>, trinv_diag_smem<T>()));
+    const size_t smem = tile_smem_bytes<T>();
     // with ev: an event is recorded after each kernel (kind * 1000 + level;
-    // kinds 0 rowscale, 1 scatter, 2 extend_add, 3 first panel, 4 L21 + row
-    // swaps + U12, 6 trailing update + next panel, 7 trinv, 8 trcopy, 9 G/H
-    // products, 10 G/H copy)
+    // kinds 0 rowscale, 1 scatter, 2 extend_add, 3 pivot-block inverse, 4 row
+    // block, 6 update)
     int nev = 0;
     auto mark = [&](int code) -> int {
         const cudaError_t le = cudaGetLastError();
@@ -2966,125 +1831,41 @@ static int factor_launches(const MfPlan *P, MfFactor *M, const int *rowptr, cons
     k_rowscale<<<grid_for(P->n, 256), 256, 0, s>>>(P->n, rowptr, val, M->rs);
     V2D_TRY(mark(0));
     ++launches;
+    V2D_CUDA_TRY(cudaMemsetAsync(F, 0, (size_t)P->ftotal * sizeof(T), s));
+    k_scatter<T><<<grid_for(P->nasm, 256), 256, 0, s>>>(P->nasm, P->d_asm_csr, P->d_asm_row,
+                                                      P->d_asm_pos, val, M->rs, F);
+    V2D_TRY(mark(1000));
+    ++launches;
     for (int L = 0; L < P->nlevel; ++L) {
         const int q0 = P->lvl_off[L], nq = P->lvl_off[L + 1] - q0;
-        V2D_CUDA_TRY(cudaMemsetAsync(F + P->lvl_fbeg[L], 0,
-                                     (size_t)(P->lvl_fend[L] - P->lvl_fbeg[L]) * sizeof(T), s));
-        const long long na = P->lvl_aend[L] - P->lvl_abeg[L];
-        if (na > 0) {
-            k_scatter<T><<<grid_for(na, 256), 256, 0, s>>>(P->lvl_abeg[L], P->lvl_aend[L],
-                                                         P->d_asm_csr, P->d_asm_row,
-                                                         P->d_asm_pos, val, M->rs, F);
-            V2D_TRY(mark(1000 + L));
-            ++launches;
-        }
+        const int maxf = P->lvl_maxf[L], nt = (maxf + kTile - 1) / kTile;
         if (L > 0) {
-            const long long mm = (long long)P->lvl_maxm_child[L] * P->lvl_maxm_child[L];
-            const int gx = (int)std::max(1LL, std::min<long long>((mm + 255) / 256, 64));
-            for (int slot = 0; slot < 2; ++slot) {
-                for (int qb = 0; qb < nq; qb += kMaxFrontsY) {
-                    k_extend_add<T><<<dim3(gx, std::min(nq - qb, kMaxFrontsY)), 256, 0, s>>>(
-                        q0 + qb, slot, P->d_S, P->d_f, P->d_foff, P->d_uoff, P->d_child0,
-                        P->d_child1, P->d_cbmap, F);
-                    ++launches;
-                }
-                V2D_TRY(mark(2000 + L));
-            }
-        }
-        const int maxf = P->lvl_maxf[L];
-        // delayed trailing updates on levels with large fronts
-        const int W = maxf >= kDelayFront ? kDelayPanels * NB : NB;
-        for (int k = 0; k < P->lvl_maxS[L]; k += NB) {
-            if (k == 0) {   // later panels are factored by the previous trailing update
-                k_panel<T><<<nq, kMfThreads, 0, s>>>(q0, k, P->d_S, P->d_f, P->d_foff, P->d_voff,
-                                                     F, M->ipiv, M->perm, M->flag);
-                V2D_TRY(mark(3000 + L));
+            const int gx = (maxf + kExtendWarps - 1) / kExtendWarps;
+            for (int qb = 0; qb < nq; qb += kMaxFrontsY) {
+                k_extend_add<T><<<dim3(gx, std::min(nq - qb, kMaxFrontsY)), 32 * kExtendWarps, 0,
+                                  s>>>(q0 + qb, P->d_S, P->d_f, P->d_foff, P->d_voff, P->d_child0,
+                                       P->d_child1, P->d_inv0, P->d_inv1, F);
                 ++launches;
             }
-            const int below = std::max(1, maxf - k - 1);
-            const int nl = (below + kL21Rows - 1) / kL21Rows;
-            const int ncol = (maxf + kL21Rows - 1) / kL21Rows;
+            V2D_TRY(mark(2000 + L));
+        }
+        for (int k = 0; k < P->lvl_maxS[L]; k += kPiv) {
+            k_pivot_inverse<T><<<nq, kInvThreads, 0, s>>>(q0, k, P->d_S, P->d_f, P->d_foff, F,
+                                                        M->flag);
+            V2D_TRY(mark(3000 + L));
+            ++launches;
             for (int qb = 0; qb < nq; qb += kMaxFrontsY) {
-                k_l21_trsm<T><<<dim3(nl + ncol, std::min(nq - qb, kMaxFrontsY)), kL21Rows, 0,
-                                s>>>(q0 + qb, k, nl, P->d_S, P->d_f, P->d_foff, P->d_voff, F,
-                                     M->ipiv);
-                if (qb > 0) ++launches;
+                k_row_block<T><<<dim3(2 * nt, std::min(nq - qb, kMaxFrontsY)), 256, smem, s>>>(
+                    q0 + qb, k, nt, P->voff[q0], P->d_S, P->d_f, P->d_foff, P->d_voff, F, C);
+                ++launches;
             }
             V2D_TRY(mark(4000 + L));
-            const int rem = std::max(1, maxf - k - 1);
-            const int nt = (rem + kGemmTile - 1) / kGemmTile;
-            // tiles of the larger of the two cases (narrow + row block, or
-            // the super-panel's full update)
-            const int ntile = nt * nt + nt;
             for (int qb = 0; qb < nq; qb += kMaxFrontsY) {
-                k_gemm<T><<<dim3(ntile, std::min(nq - qb, kMaxFrontsY)), 256, tile_smem, s>>>(
-                    q0 + qb, k, W, P->d_S, P->d_f, P->d_foff, P->d_voff, F, M->ipiv, M->perm,
-                    M->flag);
-                if (qb > 0) ++launches;
+                k_update<T><<<dim3(nt * nt, std::min(nq - qb, kMaxFrontsY)), 256, smem, s>>>(
+                    q0 + qb, k, nt, P->voff[q0], P->d_S, P->d_f, P->d_foff, P->d_voff, F, C);
+                ++launches;
             }
             V2D_TRY(mark(6000 + L));
-            launches += 2;
-        }
-        const int nbc = (P->lvl_maxS[L] + InvWidth<T>::v - 1) / InvWidth<T>::v;
-        const size_t inv_bytes = (size_t)P->lvl_maxS[L] * (InvWidth<T>::v + 33) * sizeof(T);
-        for (int qb = 0; qb < nq; qb += kMaxFrontsY) {
-            const int nb = std::min(nq - qb, kMaxFrontsY);
-            const bool blocked = P->lvl_maxS[L] >= kBlockedInvMinS &&
-                                 (std::is_same<T, double>::value || inv_bytes <= kInvSmemMax);
-            if (inv_bytes <= kInvSmemMax && !blocked) {
-                const int nth = nbc * nb > kTrinvManyCtas ? kTrinvThreadsMany : kTrinvThreads;
-                k_trinv<T><<<dim3(nbc, nb), nth, inv_bytes, s>>>(
-                    q0 + qb, P->d_S, P->d_foff, P->d_f, P->d_toff, F, (T *)M->tmp);
-            } else if (blocked) {
-                // wide separators: blocked inversion on the tile engine (the
-                // FP64 tensor cores; CUDA cores in FP32)
-                const int nbk = (P->lvl_maxS[L] + kInvBlk - 1) / kInvBlk;
-                k_trinv_diag<T><<<dim3(nbk, nb), kTrinvDiagThreads, trinv_diag_smem<T>(), s>>>(
-                    q0 + qb, P->d_S, P->d_f, P->d_foff, P->d_toff, F, (T *)M->tmp);
-                for (int st = nbk - 2; st >= 0; --st)
-                    for (int phase = 0; phase < 2; ++phase) {
-                        const int half = nbk - st - 1;
-                        k_trinv_step<T><<<dim3(2 * half, nb), 256, tile_smem, s>>>(
-                            q0 + qb, st, phase, half, P->d_S, P->d_f, P->d_foff, P->d_toff, F,
-                            (T *)M->tmp);
-                        ++launches;
-                    }
-            } else {
-                k_trinv_g<T><<<dim3(nbc, nb), kTrinvThreadsG, 0, s>>>(
-                    q0 + qb, P->d_S, P->d_foff, P->d_f, P->d_toff, F, (T *)M->tmp,
-                    (T *)M->inv_g, (long long)P->lvl_maxS[L] * (InvWidth<T>::v + 33));
-            }
-            if (qb > 0) ++launches;
-        }
-        V2D_TRY(mark(7000 + L));
-        const long long ss = (long long)P->lvl_maxS[L] * P->lvl_maxS[L];
-        const int gcp = (int)std::max(1LL, std::min<long long>((ss + 255) / 256, 256));
-        for (int qb = 0; qb < nq; qb += kMaxFrontsY) {
-            k_trcopy<T><<<dim3(gcp, std::min(nq - qb, kMaxFrontsY)), 256, 0, s>>>(
-                q0 + qb, P->d_S, P->d_f, P->d_foff, P->d_toff, (const T *)M->tmp, F);
-            if (qb > 0) ++launches;
-        }
-        V2D_TRY(mark(8000 + L));
-        launches += 2;
-        // G = L21 L11^-1, H = U11^-1 U12 (the solve's row products)
-        if (P->lvl_maxm[L] > 0) {
-            const int ts = (P->lvl_maxS[L] + kGemmTile - 1) / kGemmTile;
-            const int tm = (P->lvl_maxm[L] + kGemmTile - 1) / kGemmTile;
-            const long long sm = 2LL * P->lvl_maxS[L] * P->lvl_maxm[L];
-            const int gcg = (int)std::max(1LL, std::min<long long>((sm + 255) / 256, 256));
-            for (int qb = 0; qb < nq; qb += kMaxFrontsY) {
-                k_gh<T><<<dim3(2 * ts * tm, std::min(nq - qb, kMaxFrontsY)), 256, tile_smem, s>>>(
-                    q0 + qb, P->d_S, P->d_f, P->d_foff, P->d_goff, F, (T *)M->gh);
-                if (qb > 0) ++launches;
-            }
-            V2D_TRY(mark(9000 + L));
-            for (int qb = 0; qb < nq; qb += kMaxFrontsY) {
-                k_ghcopy<T><<<dim3(gcg, std::min(nq - qb, kMaxFrontsY)), 256, 0, s>>>(
-                    q0 + qb, P->d_S, P->d_f, P->d_foff, P->d_goff, (const T *)M->gh, F);
-                if (qb > 0) ++launches;
-            }
-            V2D_TRY(mark(10000 + L));
-            launches += 2;
         }
     }
     if (M->fact64) {   // FP64 factors rounded to FP32 for the solve
@@ -3169,7 +1950,7 @@ static int apply_launches(const MfPlan *P, const MfFactor *M, const T *b, T *x, 
     const T *F = (const T *)(M->fact64 ? M->F32 : M->F);
     T *z = (T *)M->z, *upd = (T *)M->upd;
     const SolveItemDev *items = (const SolveItemDev *)P->d_items;
-    const size_t smf = (size_t)(P->maxf + P->maxS) * sizeof(T);
+    const size_t smf = (size_t)P->maxf * sizeof(T);
     long long launches = 0;
     if (M->flow) {
         V2D_CUDA_TRY(cudaMemsetAsync(M->sctr, 0, (size_t)(P->nctr + kFlowSlots) * sizeof(int), s));
@@ -3178,18 +1959,18 @@ static int apply_launches(const MfPlan *P, const MfFactor *M, const T *b, T *x, 
             if (M->flow_form == 1 && M->flow_grid1 > 0)
                 k_solve_flow<T, RowRegs3<T>::v, 3><<<std::min(n, M->flow_grid1), kSolveThreads, smf,
                                                      s>>>(D, F, b, M->rs, z, upd, x, items, i0, i1,
-                                                          P->maxf, M->sctr, P->nctr, slot, M->bar,
+                                                          M->sctr, P->nctr, slot, M->bar,
                                                           stop_a, stop_b, trace);
             else
                 k_solve_flow<T, RowRegs<T>::v, 2><<<std::min(n, M->flow_grid), kSolveThreads, smf,
                                                     s>>>(D, F, b, M->rs, z, upd, x, items, i0, i1,
-                                                         P->maxf, M->sctr, P->nctr, slot, M->bar,
+                                                         M->sctr, P->nctr, slot, M->bar,
                                                          stop_a, stop_b, trace);
         };
         auto lower = [&](int i0, int i1, int slot) {
             k_solve_flow<T, RowRegs<T>::v, kLowMinBlocks, kLowThreads>
                 <<<std::max(1, std::min(i1 - i0, M->low_grid)), kLowThreads, M->low_smem, s>>>(
-                    D, F, b, M->rs, z, upd, x, items, i0, i1, M->low_wcap, M->sctr, P->nctr, slot,
+                    D, F, b, M->rs, z, upd, x, items, i0, i1, M->sctr, P->nctr, slot,
                     M->bar, stop_a, stop_b, trace);
         };
         const int Ls = M->split;
@@ -3298,13 +2079,10 @@ int mf_set_split(const MfPlan *P, MfFactor *M, int split)
         M->split = 0;
         return V2D_OK;
     }
-    int wcap = 0, smax = 0;
-    for (int L = 0; L < split; ++L) {
-        wcap = std::max(wcap, P->lvl_maxf[L]);
-        smax = std::max(smax, P->lvl_maxS[L]);
-    }
+    int wcap = 0;
+    for (int L = 0; L < split; ++L) wcap = std::max(wcap, P->lvl_maxf[L]);
     const size_t es = M->fp32 ? sizeof(float) : sizeof(double);
-    const size_t bytes = (size_t)(wcap + smax) * es;
+    const size_t bytes = (size_t)wcap * es;
     const void *fn = M->fp32
                          ? (const void *)k_solve_flow<float, RowRegs<float>::v, kLowMinBlocks,
                                                       kLowThreads>
@@ -3316,7 +2094,6 @@ int mf_set_split(const MfPlan *P, MfFactor *M, int split)
     V2D_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     V2D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLowThreads, bytes));
     V2D_ARG_CHECK(per_sm > 0, "lu split: no CTA of the lower-level launch fits on an SM");
-    M->low_wcap = wcap;
     M->low_smem = bytes;
     M->low_grid = nsm * per_sm;
     M->split = split;

@@ -4,7 +4,7 @@
 // Each front (S pivots of f variables, row-major f x f) is eliminated by
 // blocked Gauss-Jordan steps of kPiv pivots.  A step on the pivots K = [k, e)
 // of a front A does, in place,
-//   X = A_KK^-1                          k_pivot_inverse (X replaces A_KK)
+//   X = A_KK^-1                          k_assemble, k_update (X replaces A_KK)
 //   R = X A_KJ for all columns J != K    k_row_block     (R replaces A_KJ)
 //   A_IJ -= A_IK R, A_IK = -A_IK X       k_update, every row I outside K
 // and leaves, after the last step, exactly what a solve multiplies with:
@@ -29,6 +29,8 @@
 // more).
 #pragma once
 
+#include <algorithm>
+
 #include "v2d_internal.cuh"
 
 namespace v2d {
@@ -37,10 +39,6 @@ namespace {
 constexpr int kPiv = 64;      // pivots per elimination step
 constexpr int kTile = 64;     // output tile of the step's products
 constexpr int kSlice = 32;    // inner columns per operand slice
-// grids with one y index per front take at most this many fronts per launch
-// (the grid's y dimension is limited to 65535)
-constexpr int kMaxFrontsY = 65535;
-
 // rs[r] = 1 / max_c |a_rc| (1 for an empty row).
 __global__ void k_rowscale(int n, const int *__restrict__ rowptr, const double *__restrict__ val,
                            double *rs)
@@ -81,48 +79,85 @@ __global__ void k_invert_cbmap(int nf, const int *__restrict__ S, const int *__r
     }
 }
 
-// Adds both children's contribution blocks to every front of a level: one
-// warp per front row, each entry pulled from the children through the
-// inverse maps (a fixed order of addition, no atomics, one pass over the
-// front for both children).
-constexpr int kExtendWarps = 8;
+// A front of the level being assembled and its children's contribution
+// blocks (null where it has no such child), with the inverse maps of its
+// variables.
+template <class T> struct Assembly {
+    T *A;
+    const T *src[2];
+    const int *map[2];
+    int f, w, fc[2];   // w: pivots of the first elimination step
+};
+
+struct AssemblyMaps {
+    const int *S, *f, *voff, *child0, *child1, *inv0, *inv1;
+    const long long *foff;
+};
 
 template <class T>
-__global__ void __launch_bounds__(32 * kExtendWarps) k_extend_add(
-    int q0, const int *__restrict__ S, const int *__restrict__ f,
-    const long long *__restrict__ foff, const int *__restrict__ voff,
-    const int *__restrict__ child0, const int *__restrict__ child1,
-    const int *__restrict__ inv0, const int *__restrict__ inv1, T *F)
+__device__ __forceinline__ Assembly<T> assembly_of(const AssemblyMaps &m, int q, T *F)
 {
-    const int q = q0 + blockIdx.y, fq = f[q], vo = voff[q];
-    const int c0 = child0[q], c1 = child1[q];
-    const int *m0 = inv0 + vo, *m1 = inv1 + vo;
-    const int lane = threadIdx.x & 31;
-    const T *A0 = nullptr, *A1 = nullptr;
-    int f0 = 0, f1 = 0;
-    if (c0 >= 0) {
-        f0 = f[c0];
-        A0 = F + foff[c0] + (long long)S[c0] * f0 + S[c0];
-    }
-    if (c1 >= 0) {
-        f1 = f[c1];
-        A1 = F + foff[c1] + (long long)S[c1] * f1 + S[c1];
-    }
-    T *A = F + foff[q];
-    for (int a = blockIdx.x * kExtendWarps + (threadIdx.x >> 5); a < fq;
-         a += gridDim.x * kExtendWarps) {
-        const int r0 = c0 >= 0 ? m0[a] : -1, r1 = c1 >= 0 ? m1[a] : -1;
-        if (r0 < 0 && r1 < 0) continue;
-        const T *s0 = A0 + (long long)r0 * f0, *s1 = A1 + (long long)r1 * f1;
-        T *d = A + (long long)a * fq;
-        for (int b = lane; b < fq; b += 32) {
-            const int j0 = r0 >= 0 ? m0[b] : -1, j1 = r1 >= 0 ? m1[b] : -1;
-            if (j0 < 0 && j1 < 0) continue;
-            T v = d[b];
-            if (j0 >= 0) v += s0[j0];
-            if (j1 >= 0) v += s1[j1];
-            d[b] = v;
+    Assembly<T> a;
+    const int c[2] = {m.child0[q], m.child1[q]}, vo = m.voff[q];
+    a.A = F + m.foff[q];
+    a.f = m.f[q];
+    a.w = min(kPiv, m.S[q]);
+    a.map[0] = m.inv0 + vo;
+    a.map[1] = m.inv1 + vo;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        a.src[u] = nullptr;
+        a.fc[u] = 0;
+        if (c[u] >= 0) {
+            a.fc[u] = m.f[c[u]];
+            const int sc = m.S[c[u]];
+            a.src[u] = F + m.foff[c[u]] + (long long)sc * a.fc[u] + sc;
         }
+    }
+    return a;
+}
+
+// One warp's share of the extend-add: kExtRows rows x kExtCols columns of a
+// front, each entry pulled from the children through the inverse maps (a
+// fixed order of addition, no atomics, one pass for both children).  A lane
+// keeps its columns' positions for all rows, and a row's loads are all in
+// flight together; the first step's pivot block is left out (k_assemble adds
+// it where it inverts it).
+constexpr int kExtRows = 4, kExtCols = 256, kExtWarps = 8;
+
+template <class T>
+__device__ __forceinline__ void extend_rows(const Assembly<T> &a, int r0, int c0)
+{
+    constexpr int U = kExtCols / 32;
+    const int lane = threadIdx.x & 31;
+    int j[2][U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int c = c0 + lane + 32 * u;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) j[h][u] = a.src[h] && c < a.f ? a.map[h][c] : -1;
+    }
+#pragma unroll 2
+    for (int r = r0; r < min(r0 + kExtRows, a.f); ++r) {
+        int i[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) i[h] = a.src[h] ? a.map[h][r] : -1;
+        if (i[0] < 0 && i[1] < 0) continue;
+        const T *s0 = a.src[0] + (long long)i[0] * a.fc[0], *s1 = a.src[1] + (long long)i[1] * a.fc[1];
+        T *d = a.A + (long long)r * a.f + c0 + lane;
+        T v[U], x0[U], x1[U];
+        bool on[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool p0 = i[0] >= 0 && j[0][u] >= 0, p1 = i[1] >= 0 && j[1][u] >= 0;
+            on[u] = (p0 || p1) && !(r < a.w && c0 + lane + 32 * u < a.w);
+            v[u] = on[u] ? d[32 * u] : T(0);
+            x0[u] = p0 ? s0[j[0][u]] : T(0);
+            x1[u] = p1 ? s1[j[1][u]] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (on[u]) d[32 * u] = v[u] + x0[u] + x1[u];
     }
 }
 
@@ -153,17 +188,34 @@ __device__ __forceinline__ void dmma_8x8x4(double &c0, double &c1, double a, dou
                  : "d"(a), "d"(b));
 }
 
-// X = A_KK^-1 of one step's pivot block of every front (one CTA each), in
-// place, in FP64.  The block sits in shared memory as 2 x 2 blocks of 32 and
-// is inverted by block Gauss-Jordan: the 32 x 32 diagonal blocks one after
-// the other in the registers of the CTA's four warps (invert32), the products
-// between the blocks on the FP64 tensor cores.  The chain of pivot columns
+// X = A_KK^-1 of one step's pivot block, in FP64, by four warps: for a level's
+// first step by the CTA that adds the children's entries to that block
+// (k_assemble), for every later step by the CTA that has just updated it in
+// the step before (k_update): no launch and no round trip through memory in
+// the chain of steps, and hidden behind the other CTAs on levels with many.
+// The block sits in shared memory as 2 x 2 blocks of 32 and is inverted by
+// block Gauss-Jordan: the 32 x 32 diagonal blocks one after the other in
+// registers (invert32), the products between the blocks on the FP64 tensor
+// cores.  The chain of pivot columns
 // bounds it, not its 2 kPiv^3 flops: the code is kept short and rolled, since
 // straight-line code that runs once waits for its own instructions.
 constexpr int kInvThreads = 128;
 constexpr int kHalf = kPiv / 2;
 constexpr int kLdX = kPiv + 2;   // two wavefronts per fragment read, rows 16-byte aligned
 constexpr int kPanel = 4;        // columns per panel of invert32, one per warp
+
+// Shared memory of one pivot block's inversion.
+struct PivotSmem {
+    double M[kPiv * kLdX];
+    double col[2][kPanel][kHalf];
+    int piv[kHalf];
+};
+
+// Barrier of the inversion's four warps (the first of the CTA).
+__device__ __forceinline__ void pivot_sync()
+{
+    asm volatile("bar.sync 1, %0;" ::"n"(kInvThreads) : "memory");
+}
 
 // 1 / x to a few units in the last place: the hardware's approximation and
 // two Newton steps (x = 0 and denormals: not finite; the caller looks at x).
@@ -203,7 +255,7 @@ __device__ __forceinline__ bool invert32(double *M, double (*col)[kPanel][kHalf]
 #pragma unroll 1
     for (int P = 0; P < R; ++P) {
         col[P & 1][w][lane] = a[0];
-        __syncthreads();
+        pivot_sync();
         double pan[kPanel];
 #pragma unroll
         for (int t = 0; t < kPanel; ++t) pan[t] = col[P & 1][t][lane];
@@ -240,44 +292,26 @@ __device__ __forceinline__ bool invert32(double *M, double (*col)[kPanel][kHalf]
         for (int i = 1; i < R; ++i) a[i - 1] = a[i];
         a[R - 1] = w == 0 ? pan[0] : w == 1 ? pan[1] : w == 2 ? pan[2] : pan[3];
     }
-    __syncthreads();
+    pivot_sync();
 #pragma unroll
     for (int i = 0; i < R; ++i) M[step * kLdX + piv[kPanel * i + w]] = a[i] * scale;
     return bad;
 }
 
-template <class T>
-__global__ void __launch_bounds__(kInvThreads) k_pivot_inverse(int q0, int k,
-                                                               const int *__restrict__ S_,
-                                                               const int *__restrict__ f_,
-                                                               const long long *__restrict__ foff,
-                                                               T *F, int *flag)
+// The w x w block at sm.M (padded to 64 x 64 by the identity) inverted in
+// place by the CTA's first four warps; sm.M must be visible to them.
+__device__ __forceinline__ void invert_block(PivotSmem &sm, int w, int *flag)
 {
-    __shared__ __align__(16) double M[kPiv * kLdX];
-    __shared__ double col[2][kPanel][kHalf];
-    __shared__ int piv[kHalf];
-    const int q = q0 + blockIdx.x;
-    const int S = S_[q], f = f_[q];
-    if (S <= k) return;
-    const int w = min(kPiv, S - k), tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, t = lane & 3;
-    T *A = F + foff[q] + (long long)k * f + k;
-    // padded by the identity
-    const int c0 = tid & (kPiv - 1);
-#pragma unroll 16
-    for (int r = tid / kPiv; r < kPiv; r += kInvThreads / kPiv)
-        M[r * kLdX + c0] = (r < w && c0 < w) ? (double)A[(long long)r * f + c0]
-                                             : (r == c0 ? 1.0 : 0.0);
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     bool bad = false;
     const int nh = w > kHalf ? 2 : 1;
 #pragma unroll 1
     for (int h = 0; h < nh; ++h) {
         // the step's block X, its row O, its column C and the rest Y
-        double *X = M + h * (kHalf * kLdX + kHalf), *Y = M + (1 - h) * (kHalf * kLdX + kHalf);
-        double *O = M + (h ? kHalf * kLdX : kHalf), *C = M + (h ? kHalf : kHalf * kLdX);
-        __syncthreads();
-        bad |= invert32(X, col, piv);
-        __syncthreads();
+        double *X = sm.M + h * (kHalf * kLdX + kHalf), *Y = sm.M + (1 - h) * (kHalf * kLdX + kHalf);
+        double *O = sm.M + (h ? kHalf * kLdX : kHalf), *C = sm.M + (h ? kHalf : kHalf * kLdX);
+        bad |= invert32(X, sm.col, sm.piv);
+        pivot_sync();
         if (nh == 1) break;
 #pragma unroll 1
         for (int i = 0; i < 3; ++i) {   // O = X O, Y -= C O, C = -C X; a warp's 8 rows
@@ -291,7 +325,7 @@ __global__ void __launch_bounds__(kInvThreads) k_pivot_inverse(int q0, int k,
                 for (int n = 0; n < 4; ++n)
                     dmma_8x8x4(acc[n][0], acc[n][1], a, B[(k4 + t) * kLdX + 8 * n + g]);
             }
-            __syncthreads();
+            pivot_sync();
 #pragma unroll
             for (int n = 0; n < 4; ++n) {
                 double *d = D + (8 * wid + g) * kLdX + 8 * n + 2 * t;
@@ -299,13 +333,65 @@ __global__ void __launch_bounds__(kInvThreads) k_pivot_inverse(int q0, int k,
                 for (int u = 0; u < 2; ++u)
                     d[u] = i == 0 ? acc[n][u] : (i == 1 ? d[u] : 0.0) - acc[n][u];
             }
-            __syncthreads();
+            pivot_sync();
         }
     }
     if (bad && tid == 0) atomicOr(flag, 1);
-#pragma unroll 16
-    for (int r = tid / kPiv; r < kPiv; r += kInvThreads / kPiv)
-        if (r < w && c0 < w) A[(long long)r * f + c0] = (T)M[r * kLdX + c0];
+}
+
+// sm.M's w x w block to the front (leading dimension f), four warps.
+template <class T>
+__device__ __forceinline__ void store_block(const PivotSmem &sm, int w, T *A, int f)
+{
+    const int c = threadIdx.x & (kPiv - 1);
+#pragma unroll 8
+    for (int r = threadIdx.x / kPiv; r < kPiv; r += kInvThreads / kPiv)
+        if (r < w && c < w) A[(long long)r * f + c] = (T)sm.M[r * kLdX + c];
+}
+
+// A level's fronts get their children's contribution blocks, and the first
+// step's pivot blocks are inverted: the first of a front's `per` CTAs adds the
+// children's entries of that block, inverts it and stores X; the others (none
+// on a level without children) add the rest, 32 rows x 256 columns each.  A
+// front's CTAs are neighbours in the grid, here and in the step's kernels:
+// with the first CTAs of all fronts in front the large levels lose their L2
+// locality (8.8 against 7.1 ms on all levels of 1025 x 1025).
+template <class T>
+__global__ void __launch_bounds__(32 * kExtWarps) k_assemble(int q0, int per, int nc,
+                                                             const AssemblyMaps m, T *F, int *flag)
+{
+    __shared__ __align__(16) PivotSmem sm;
+    const int q = q0 + blockIdx.x / per, t = blockIdx.x % per;
+    const Assembly<T> a = assembly_of(m, q, F);
+    if (t > 0) {
+        const int r0 = ((t - 1) / nc) * (kExtRows * kExtWarps) + (threadIdx.x >> 5) * kExtRows;
+        const int c0 = ((t - 1) % nc) * kExtCols;
+        if (r0 < a.f && c0 < a.f) extend_rows(a, r0, c0);
+        return;
+    }
+    constexpr int R = kPiv * kPiv / (32 * kExtWarps), step = 32 * kExtWarps / kPiv;
+    const int c = threadIdx.x & (kPiv - 1), r0 = threadIdx.x / kPiv;
+    T v[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int r = r0 + i * step;
+        v[i] = (r < a.w && c < a.w) ? a.A[(long long)r * a.f + c] : (r == c ? T(1) : T(0));
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int j = a.src[h] && c < a.w ? a.map[h][c] : -1;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = r0 + i * step, k = j >= 0 && r < a.w ? a.map[h][r] : -1;
+            if (k >= 0) v[i] += a.src[h][(long long)k * a.fc[h] + j];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) sm.M[(r0 + i * step) * kLdX + c] = (double)v[i];
+    __syncthreads();
+    if (threadIdx.x >= kInvThreads) return;
+    invert_block(sm, a.w, flag);
+    store_block(sm, a.w, a.A, a.f);
 }
 
 // Accumulator of one 64 x 64 output tile of a CTA of 256 threads, fed
@@ -330,22 +416,26 @@ template <> struct Tile<double> {
         double B[kSlice][kLdB];
     };
     double acc[4][2][2];
-    __device__ __forceinline__ void mac(const Smem &s)
+    // nr x nc: the tile's valid rows and columns (8 x 8 blocks beyond are skipped)
+    __device__ __forceinline__ void mac(const Smem &s, int nr, int nc)
     {
         const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
         const int wr = (w >> 2) * 32, wc = (w & 3) * 16;
+        if (wc >= nc) return;
+        nr -= wr;
 #pragma unroll
         for (int k = 0; k < kSlice; k += 4) {
-            double a[4], b[2];
-#pragma unroll
-            for (int mi = 0; mi < 4; ++mi) a[mi] = s.A[wr + 8 * mi + g][k + t];
+            double b[2];
 #pragma unroll
             for (int ni = 0; ni < 2; ++ni) b[ni] = s.B[k + t][wc + 8 * ni + g];
 #pragma unroll
             for (int mi = 0; mi < 4; ++mi)
+                if (8 * mi < nr) {
+                    const double a = s.A[wr + 8 * mi + g][k + t];
 #pragma unroll
-                for (int ni = 0; ni < 2; ++ni)
-                    dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], a[mi], b[ni]);
+                    for (int ni = 0; ni < 2; ++ni)
+                        dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], a, b[ni]);
+                }
         }
     }
     // fn(row, first column, the kVec accumulators)
@@ -368,7 +458,7 @@ template <> struct Tile<float> {
         float B[kSlice][kLdB];
     };
     float acc[4][2][2];
-    __device__ __forceinline__ void mac(const Smem &s)
+    __device__ __forceinline__ void mac(const Smem &s, int, int)
     {
         const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
 #pragma unroll 2
@@ -444,20 +534,25 @@ __device__ __forceinline__ void tile_product(Tile<T> &t, typename Tile<T>::Smem 
         stage_slice<T>(sm[1], a, lda, nr, b, ldb, nc, kSlice, ke);
         cp_async_wait<1>();
         __syncthreads();
-        t.mac(sm[0]);
+        t.mac(sm[0], nr, nc);
         cp_async_wait<0>();
         __syncthreads();
-        t.mac(sm[1]);
+        t.mac(sm[1], nr, nc);
     } else {
         cp_async_wait<0>();
         __syncthreads();
-        t.mac(sm[0]);
+        t.mac(sm[0], nr, nc);
     }
 }
 
-template <class T> constexpr size_t tile_smem_bytes() { return 2 * sizeof(typename Tile<T>::Smem); }
+// Dynamic shared memory of k_row_block and k_update: two operand slices, or
+// the next pivot block's inversion in their place.
+template <class T> constexpr size_t tile_smem_bytes()
+{
+    return std::max(2 * sizeof(typename Tile<T>::Smem), sizeof(PivotSmem));
+}
 
-// R = X A_KJ of a step, in place, 64 columns per CTA (blocks [0, nt)); blocks
+// R = X A_KJ of a step, in place, 64 columns per CTA (a front's blocks [0, nt)); blocks
 // [nt, 2 nt) copy 64 rows of the pivot columns A_IK to the step's scratch C
 // (front rows x kPiv, zero beyond the step's pivots; v0 = the level's first
 // voff), where k_update reads them while it overwrites A_IK.
@@ -470,13 +565,13 @@ __global__ void __launch_bounds__(256) k_row_block(int q0, int k, int nt, int v0
 {
     using P2 = typename Pair<T>::type;
     extern __shared__ __align__(16) unsigned char tile_raw[];
-    const int q = q0 + blockIdx.y;
+    const int q = q0 + blockIdx.x / (2 * nt), tile = blockIdx.x % (2 * nt);
     const int S = S_[q], f = f_[q];
     if (S <= k) return;
     const int w = min(kPiv, S - k), e = k + w;
     T *A = F + foff[q];
-    if ((int)blockIdx.x >= nt) {
-        const int r0 = ((int)blockIdx.x - nt) * kTile;
+    if (tile >= nt) {
+        const int r0 = (tile - nt) * kTile;
         const int nr = min(kTile, f - r0);
         T *Cq = C + (long long)(voff[q] - v0) * kPiv;
         for (int i = threadIdx.x; i < nr * (kPiv / 2); i += 256) {
@@ -488,7 +583,7 @@ __global__ void __launch_bounds__(256) k_row_block(int q0, int k, int nt, int v0
         }
         return;
     }
-    const int c0 = blockIdx.x * kTile;
+    const int c0 = tile * kTile;
     if (c0 >= f || (c0 >= k && min(c0 + kTile, f) <= e)) return;
     typename Tile<T>::Smem *sm = reinterpret_cast<typename Tile<T>::Smem *>(tile_raw);
     Tile<T> t;
@@ -508,28 +603,33 @@ __global__ void __launch_bounds__(256) k_row_block(int q0, int k, int nt, int v0
 }
 
 // A_IJ -= C_I R_J on one 64 x 64 tile (rows outside the pivots), A_IK =
-// -C_I X in the pivot columns (R_K = X in place).
+// -C_I X in the pivot columns (R_K = X in place).  Tile 0 of a front is the
+// next step's pivot block, whose inverse this CTA stores in its place.
 template <class T>
 __global__ void __launch_bounds__(256, 3) k_update(int q0, int k, int nt, int v0,
                                                    const int *__restrict__ S_,
                                                    const int *__restrict__ f_,
                                                    const long long *__restrict__ foff,
-                                                   const int *__restrict__ voff, T *F, const T *C)
+                                                   const int *__restrict__ voff, T *F, const T *C,
+                                                   int *flag)
 {
     using P2 = typename Pair<T>::type;
     extern __shared__ __align__(16) unsigned char tile_raw[];
-    const int q = q0 + blockIdx.y;
+    const int q = q0 + blockIdx.x / (nt * nt), t = blockIdx.x % (nt * nt);
     const int S = S_[q], f = f_[q];
     if (S <= k) return;
     const int w = min(kPiv, S - k), e = k + w;
-    const int r0 = (blockIdx.x / nt) * kTile, c0 = (blockIdx.x % nt) * kTile;
+    // tiles in row order, the one of the next pivot block exchanged with the first
+    const int next = e < S ? (e / kTile) * (nt + 1) : -1;
+    const int t0 = next < 0 ? t : (t == 0 ? next : (t == next ? 0 : t));
+    const int r0 = (t0 / nt) * kTile, c0 = (t0 % nt) * kTile;
     if (r0 >= f || c0 >= f || (r0 >= k && min(r0 + kTile, f) <= e)) return;
     T *A = F + foff[q];
     const T *Cq = C + (long long)(voff[q] - v0) * kPiv;
     typename Tile<T>::Smem *sm = reinterpret_cast<typename Tile<T>::Smem *>(tile_raw);
-    Tile<T> t;
+    Tile<T> acc;
     // the old entries, negated: loaded while the operands are on their way
-    t.each([&](int rr, int cc, T (&v)[2]) {
+    acc.each([&](int rr, int cc, T (&v)[2]) {
         const int r = r0 + rr, c = c0 + cc;
         v[0] = v[1] = T(0);
         if (r < f && c < f && !(c >= k && c < e)) {
@@ -538,10 +638,21 @@ __global__ void __launch_bounds__(256, 3) k_update(int q0, int k, int nt, int v0
             v[1] = -o.y;
         }
     });
-    tile_product<T>(t, sm, Cq + (long long)r0 * kPiv, kPiv, min(kTile, f - r0),
+    tile_product<T>(acc, sm, Cq + (long long)r0 * kPiv, kPiv, min(kTile, f - r0),
                     A + (long long)k * f + c0, f, min(kTile, f - c0), w);
-    t.each([&](int rr, int cc, T (&v)[2]) {
+    const bool pivots = t0 == next;
+    const int wn = pivots ? min(kPiv, S - e) : 0;   // the block's pivots
+    PivotSmem &ps = *reinterpret_cast<PivotSmem *>(tile_raw);
+    if (pivots) __syncthreads();   // the operands' buffers are free
+    acc.each([&](int rr, int cc, T (&v)[2]) {
         const int r = r0 + rr, c = c0 + cc;
+        if (pivots) {
+            const bool in = rr < wn && cc < wn;
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                ps.M[rr * kLdX + cc + u] = in ? -(double)v[u] : (rr == cc + u ? 1.0 : 0.0);
+            if (in) return;
+        }
         if (r < f && c < f && !(r >= k && r < e)) {
             P2 o;
             o.x = -v[0];
@@ -549,6 +660,11 @@ __global__ void __launch_bounds__(256, 3) k_update(int q0, int k, int nt, int v0
             *reinterpret_cast<P2 *>(A + (long long)r * f + c) = o;
         }
     });
+    if (!pivots) return;
+    __syncthreads();
+    if (threadIdx.x >= kInvThreads) return;
+    invert_block(ps, wn, flag);
+    store_block(ps, wn, A + (long long)e * f + e, f);
 }
 
 // FP64 factors rounded to FP32 (the solve of the mixed form with FP64

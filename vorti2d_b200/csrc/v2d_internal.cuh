@@ -227,7 +227,7 @@ int mf_time_apply_launches(const MfPlan *P, const MfFactor *M, int reps, size_t 
                            cudaStream_t s, double *ms, int *codes, int cap, int *n);
 // Per-kernel device time of one factorization launched directly (not from
 // its graph), average of reps; codes kind * 1000 + level (kinds 0 rowscale,
-// 1 scatter, 2 extend_add, 3 pivot-block inverse, 4 row block, 6 update,
+// 1 scatter, 2 assembly with the first pivot inverse, 4 row block, 6 update,
 // 11 rounding to FP32).  The factors are recomputed from the same values.
 int mf_time_factor_launches(const MfPlan *P, MfFactor *M, const int *rowptr, const double *val,
                             int reps, cudaStream_t s, double *ms, int *codes, int cap, int *n);

@@ -667,7 +667,7 @@ int mf_plan_build(int imax, int jmax, int n, const int *h_rowptr, const int *h_c
     return V2D_OK;
 }
 
-// The inverse contribution maps (k_extend_add), from the uploaded arrays.
+// The inverse contribution maps (k_assemble), from the uploaded arrays.
 static int invert_cbmap(MfPlan *P)
 {
     const size_t bytes = std::max<size_t>(1, P->vtotal) * sizeof(int);
@@ -1808,8 +1808,8 @@ static int factor_launches(const MfPlan *P, MfFactor *M, const int *rowptr, cons
     long long launches = 0;
     const size_t smem = tile_smem_bytes<T>();
     // with ev: an event is recorded after each kernel (kind * 1000 + level;
-    // kinds 0 rowscale, 1 scatter, 2 extend_add, 3 pivot-block inverse, 4 row
-    // block, 6 update)
+    // kinds 0 rowscale, 1 scatter, 2 assembly with the first pivot inverse,
+    // 4 row block, 6 update)
     int nev = 0;
     auto mark = [&](int code) -> int {
         const cudaError_t le = cudaGetLastError();
@@ -1836,36 +1836,26 @@ static int factor_launches(const MfPlan *P, MfFactor *M, const int *rowptr, cons
                                                       P->d_asm_pos, val, M->rs, F);
     V2D_TRY(mark(1000));
     ++launches;
+    const AssemblyMaps maps{P->d_S, P->d_f, P->d_voff, P->d_child0, P->d_child1, P->d_inv0,
+                            P->d_inv1, P->d_foff};
     for (int L = 0; L < P->nlevel; ++L) {
         const int q0 = P->lvl_off[L], nq = P->lvl_off[L + 1] - q0;
-        const int maxf = P->lvl_maxf[L], nt = (maxf + kTile - 1) / kTile;
-        if (L > 0) {
-            const int gx = (maxf + kExtendWarps - 1) / kExtendWarps;
-            for (int qb = 0; qb < nq; qb += kMaxFrontsY) {
-                k_extend_add<T><<<dim3(gx, std::min(nq - qb, kMaxFrontsY)), 32 * kExtendWarps, 0,
-                                  s>>>(q0 + qb, P->d_S, P->d_f, P->d_foff, P->d_voff, P->d_child0,
-                                       P->d_child1, P->d_inv0, P->d_inv1, F);
-                ++launches;
-            }
-            V2D_TRY(mark(2000 + L));
-        }
+        const int maxf = P->lvl_maxf[L], nt = (maxf + kTile - 1) / kTile, v0 = P->voff[q0];
+        // the extend-add's blocks of a front: none on the leaves
+        const int nc = (maxf + kExtCols - 1) / kExtCols;
+        const int per =
+            1 + (L > 0 ? nc * ((maxf + kExtRows * kExtWarps - 1) / (kExtRows * kExtWarps)) : 0);
+        k_assemble<T><<<nq * per, 32 * kExtWarps, 0, s>>>(q0, per, nc, maps, F, M->flag);
+        V2D_TRY(mark(2000 + L));
+        ++launches;
         for (int k = 0; k < P->lvl_maxS[L]; k += kPiv) {
-            k_pivot_inverse<T><<<nq, kInvThreads, 0, s>>>(q0, k, P->d_S, P->d_f, P->d_foff, F,
-                                                        M->flag);
-            V2D_TRY(mark(3000 + L));
-            ++launches;
-            for (int qb = 0; qb < nq; qb += kMaxFrontsY) {
-                k_row_block<T><<<dim3(2 * nt, std::min(nq - qb, kMaxFrontsY)), 256, smem, s>>>(
-                    q0 + qb, k, nt, P->voff[q0], P->d_S, P->d_f, P->d_foff, P->d_voff, F, C);
-                ++launches;
-            }
+            k_row_block<T><<<nq * 2 * nt, 256, smem, s>>>(q0, k, nt, v0, P->d_S, P->d_f, P->d_foff,
+                                                        P->d_voff, F, C);
             V2D_TRY(mark(4000 + L));
-            for (int qb = 0; qb < nq; qb += kMaxFrontsY) {
-                k_update<T><<<dim3(nt * nt, std::min(nq - qb, kMaxFrontsY)), 256, smem, s>>>(
-                    q0 + qb, k, nt, P->voff[q0], P->d_S, P->d_f, P->d_foff, P->d_voff, F, C);
-                ++launches;
-            }
+            k_update<T><<<nq * nt * nt, 256, smem, s>>>(q0, k, nt, v0, P->d_S, P->d_f, P->d_foff,
+                                                      P->d_voff, F, C, M->flag);
             V2D_TRY(mark(6000 + L));
+            launches += 2;
         }
     }
     if (M->fact64) {   // FP64 factors rounded to FP32 for the solve

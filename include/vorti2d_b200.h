@@ -420,16 +420,16 @@ int v2d_solver_lu_stats(v2d_solver *s, double *out6);
 
 /* Measurement aid (no reference counterpart): one dataflow LU solve of the
  * current factors with a trace of every work item -- global-timer ns at its
- * ticket, at the end of its dependency wait and after its done counters
- * (ticks[3 i + k]) -- and the item table (items: 12 ints per item as in
+ * ticket, when its vector is gathered (its dependencies met) and after its
+ * rows (ticks[3 i + k]) -- and the item table (items: 12 ints per item as in
  * v2d_lu_solve_plan, may be null); cap >= items, *n = items. */
 int v2d_solver_trace_lu_apply(v2d_solver *s, unsigned long long *ticks, int *items, int cap,
                               int *n);
 
 /* Tuning aid (no reference counterpart): the form of the dataflow LU solve
- * kernel -- 0: two resident CTAs per SM with 32 row registers per lane (16 in
- * FP64); 1: three CTAs per SM with 16 (8 in FP64).  form < 0 only reads the
- * current one into *current (may be null). */
+ * kernel -- 0: two resident CTAs per SM (default); 1: three, each with a third
+ * of the SM's shared memory for factor rows on their way.  form < 0 only reads
+ * the current one into *current (may be null). */
 int v2d_solver_lu_flow_form(v2d_solver *s, int form, int *current);
 
 /* Tuning aid (no reference counterpart): the split form of the dataflow LU
@@ -439,15 +439,16 @@ int v2d_solver_lu_flow_form(v2d_solver *s, int form, int *current);
  * front, so that more of their many small work items are in flight per SM;
  * 0: one launch for the whole tree.  level < 0 only reads the current
  * setting into *current (may be null).  Every setting forms the same
- * products. */
+ * products in the same order. */
 int v2d_solver_lu_split(v2d_solver *s, int level, int *current);
 
 /* Tuning aid (no reference counterpart): the work-item granularity of the
  * LU preconditioner solve, rows[L] rows of a front per work item on tree
- * level L (0: whole fronts); rows may be null to only read the current
+ * level L (0: whole fronts; a handle starts with about 300 items per level);
+ * rows may be null to only read the current
  * setting into out_rows (cap >= levels) and *nlevels_out.  Every setting
- * forms the same products; only how the rows are split over CTAs (and the
- * order of a row's partial sums) changes. */
+ * forms the same products in the same order; only how the rows are split over
+ * CTAs changes. */
 int v2d_solver_lu_item_rows(v2d_solver *s, const int *rows, int nlevels, int *out_rows, int cap,
                             int *nlevels_out);
 

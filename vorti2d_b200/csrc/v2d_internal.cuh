@@ -80,6 +80,17 @@ int launch_forces(const GridDev &g, double re, double ref_length, double x0, dou
 // field-blocked 2N system of one O-grid (v2d_mf.cu).  Fronts are numbered
 // level by level; front q holds f[q] local variables (its S[q] fully summed
 // ones first), stored densely (row-major f x f) at foff[q].
+// A work item of the solve as the kernels read it: rows [rb, re) of a front
+// (kind 0 forward rows, 1 backward rows; 2 and 3, gather items, need no work of
+// their own), the front's sizes and offsets and its children's contribution
+// offsets (-1: no such child).
+struct alignas(16) SolveItemDev {
+    int kind, rb, re, S;
+    int f, vo, uo, cu0;
+    long long fo;   // the front's offset in the factors
+    int cu1;
+};
+
 struct MfPlan {
     int N = 0, n = 0, nfront = 0, nlevel = 0, maxS = 0, maxf = 0;
     long long ftotal = 0, nasm = 0;
@@ -110,7 +121,7 @@ struct MfPlan {
                                    // -R rows per item after one gather item per front)
     std::vector<int> lvl_fwd_g, lvl_bwd_g;   // gather items at the start of each level's
                                              // forward / backward range
-    int *d_items = nullptr;
+    SolveItemDev *d_items = nullptr;   // the same items with their fronts' scalars
     long long items_ver = 0;       // bumped whenever d_items is replaced
     // host copies, kept only between the build and the upload
     std::vector<int> h_vars, h_cbmap, h_asm_csr, h_asm_row;
@@ -136,6 +147,13 @@ struct MfBarrier {
     int err, pad;
 };
 
+// One form of the dataflow solve's launch: CTAs, shared memory, of which the
+// item's vector and each of the staged chunks.
+struct FlowShape {
+    int grid = 0, vbytes = 0, cbytes = 0;
+    size_t smem = 0;
+};
+
 // Numeric factors of one plan in one precision.
 struct MfFactor {
     int fp32 = 0;               // precision of the solve (Krylov vectors, applied factors)
@@ -145,18 +163,18 @@ struct MfFactor {
     void *F32 = nullptr;        // fact64: FP32 copy of F that the solve reads
     void *cols = nullptr;       // one elimination step's pivot columns of a level's fronts
     void *wb = nullptr;         // transposed solve: per-front adjoint right-hand sides (vtotal)
-    void *tw = nullptr;         // solve: gathered fronts' t, w and struct x (vtotal)
     double *rs = nullptr;       // row scaling 1 / max |a_r.|
     int *flag = nullptr;
     MfBarrier *bar = nullptr;
-    int *sctr = nullptr;        // dataflow solve: 3 counters per front + the work ticket
-    int flow_grid = 0;          // most CTAs of the dataflow solve resident at once
-    int flow_grid1 = 0;         // the same for its high-occupancy form (0: none)
-    int flow_form = 0;          // 0: 2 CTAs per SM, 32 row registers; 1: 3 CTAs, 16
+    void *msg = nullptr;        // dataflow solve: the tickets, upd and z in one allocation
+    size_t msg_bytes = 0;
+    int *tickets = nullptr;
+    // launches of the dataflow solve: form 0 with two, form 1 with three CTAs
+    // per SM (grid 0: does not fit), [2] the split form's lower levels
+    FlowShape shape[3];
+    int flow_form = 0;
     int split = 0;              // > 0: tree levels [0, split) in launches of their own
                                 // (forward before, backward after the upper levels)
-    int low_grid = 0;           // CTAs of those launches
-    size_t low_smem = 0;        // and their shared memory
     int flow = 1;               // 1: the solve is one dataflow launch; 0: one launch per level
                                 // and sweep
     cudaGraphExec_t graph = nullptr;
@@ -169,9 +187,8 @@ struct MfFactor {
 struct MfDev {
     const int *S, *f, *voff, *uoff, *child0, *child1, *parent;
     const long long *foff;
-    const int *vars, *cbmap;
+    const int *vars, *cbmap, *inv0, *inv1;
     int maxS, maxf;
-    void *tw;   // gathered fronts: t and w (forward), -x on the struct variables (backward)
 };
 
 // Host-only symbolic phase (validates every index it produces).

@@ -52,20 +52,18 @@
 
 #include "v2d_factor.cuh"
 #include "v2d_internal.cuh"
+#include "v2d_solve.cuh"
 
 namespace v2d {
 
 // rows per work item of the solve on levels with few fronts
 constexpr int kSolveRowsHost = 8;
-// threads of a solve work item (8 warps)
-constexpr int kSolveThreadsHost = 256;
 // the default work-item split aims at about this many items per level
 constexpr int kItemsPerLevel = 600;
 
-// Counters of the dataflow solve, three per front q: forward items of q
-// that wrote z rows (fz), the children's forward items that wrote
-// contribution rows (fin), backward items of q (bx); the work ticket after
-// them.
+// Dependency counters of the plan's order check, per front q: forward items of
+// q that wrote z rows (fz), the children's forward items that wrote
+// contribution rows (fin), backward items of q (bx), gather items (fg, bg).
 __host__ __device__ inline int ctr_fz(int q, int nf) { return q; }
 __host__ __device__ inline int ctr_fin(int q, int nf) { return nf + q; }
 __host__ __device__ inline int ctr_bx(int q, int nf) { return 2 * nf + q; }
@@ -219,13 +217,12 @@ void mf_plan_destroy(MfPlan *p)
 //                       done: bx[q]
 // On levels whose rows-per-item entry is negative, a front split into
 // several items gets a gather item first in each sweep:
-//   forward gather of q   waits fin[q]; writes t and the contribution rows'
-//                         w to tw; done: fg[q]; q's forward items wait fg[q]
+//   forward gather of q   waits fin[q]; done: fg[q]; q's forward items wait fg[q]
 //   backward gather of q  waits bx[parent] (which implies that q's own
-//                         contribution rows, the last readers of tw's w part,
-//                         are done); writes -x of q's struct variables to
-//                         tw; done: bg[q]; q's backward items wait fz[q] and
-//                         bg[q]
+//                         contribution rows are done); done: bg[q]; q's
+//                         backward items wait fz[q] and bg[q]
+// The kernels run an item's rows with a gather of their own: gather items are
+// places in the order only.
 // The check: every wait's counter reaches exactly its target in all, and
 // only through items earlier in the order; so the items an item reads have
 // all finished before it starts, and a CTA that takes items in order only
@@ -252,10 +249,8 @@ static int items_build(MfPlan *P)
         }
     }
     // rows per item; a negative entry -R splits fronts of more than R rows
-    // into R-row items after one gather item per front (kind 2 forward: w and
-    // t = P w_FS into tw; kind 3 backward: -x of the struct variables into
-    // tw), so the front's items read one contiguous vector instead of each
-    // repeating the gather
+    // into R-row items after one gather item per front (kind 2 forward, kind 3
+    // backward)
     auto per = [&](int L) {
         const int r = P->item_rows[L];
         return r > 0 ? r : (r < 0 ? -r : INT_MAX);
@@ -667,6 +662,19 @@ int mf_plan_build(int imax, int jmax, int n, const int *h_rowptr, const int *h_c
     return V2D_OK;
 }
 
+// The work items with their fronts' scalars, as the kernels read them.
+static std::vector<SolveItemDev> device_items(const MfPlan *P)
+{
+    std::vector<SolveItemDev> out(P->nitems);
+    for (int k = 0; k < P->nitems; ++k) {
+        const int *v = &P->h_items[12 * (size_t)k], q = v[1];
+        auto cu = [&](int c) { return c >= 0 ? P->uoff[c] : -1; };
+        out[k] = SolveItemDev{v[0], v[2], v[3], P->S[q], P->f[q], P->voff[q], P->uoff[q],
+                              cu(P->child0[q]), P->foff[q], cu(P->child1[q])};
+    }
+    return out;
+}
+
 // The inverse contribution maps (k_assemble), from the uploaded arrays.
 static int invert_cbmap(MfPlan *P)
 {
@@ -683,11 +691,31 @@ static int invert_cbmap(MfPlan *P)
     return V2D_OK;
 }
 
+// The split a device solve starts with: about kItemsDevice items per level --
+// one round of the dataflow solve's CTAs -- of 16 to 256 rows, and whole fronts
+// where they are short and many.  Half the items of the plan's own default:
+// an item's cost is its gather and its hand-over rather than its rows (181 x
+// 181, FP32: 0.113 ms with this split, 0.138 ms with the plan's).
+static void device_item_rows(MfPlan *P)
+{
+    constexpr int kItemsDevice = 300, kWholeFronts = 64, kWholeMaxF = 256;
+    for (int L = 0; L < P->nlevel; ++L) {
+        const int nq = P->lvl_off[L + 1] - P->lvl_off[L];
+        long long rows = 0;
+        for (int q = P->lvl_off[L]; q < P->lvl_off[L + 1]; ++q) rows += P->f[q];
+        int R = 16;
+        while (R < 256 && 2LL * R * kItemsDevice <= rows) R *= 2;
+        const bool whole = P->lvl_maxf[L] <= R || (nq >= kWholeFronts && P->lvl_maxf[L] <= kWholeMaxF);
+        P->item_rows[L] = whole ? 0 : R;
+    }
+}
+
 // Device copies of a host plan's arrays; the host copies of the large index
 // arrays are released.  On failure the plan is destroyed.
 static int mf_plan_upload(MfPlan *P)
 {
-    int st_up = V2D_OK;
+    device_item_rows(P);
+    int st_up = items_build(P);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_S, P->S);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_f, P->f);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_voff, P->voff);
@@ -701,7 +729,7 @@ static int mf_plan_upload(MfPlan *P)
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_asm_csr, P->h_asm_csr);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_asm_row, P->h_asm_row);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_asm_pos, P->h_asm_pos);
-    if (st_up == V2D_OK) st_up = upload_vec(&P->d_items, P->h_items);
+    if (st_up == V2D_OK) st_up = upload_vec(&P->d_items, device_items(P));
     if (st_up == V2D_OK) st_up = invert_cbmap(P);
     if (st_up != V2D_OK) {
         mf_plan_destroy(P);
@@ -747,8 +775,8 @@ int mf_plan_set_item_rows(MfPlan *P, const int *rows, int nlevels)
         items_build(P);
         return V2D_EARG;
     }
-    int *d = nullptr;
-    V2D_TRY(upload_vec(&d, P->h_items));
+    SolveItemDev *d = nullptr;
+    V2D_TRY(upload_vec(&d, device_items(P)));
     if (P->d_items) cudaFree(P->d_items);
     P->d_items = d;
     ++P->items_ver;
@@ -969,594 +997,6 @@ namespace v2d {
 // ================================================================ numeric
 namespace {
 
-// ------------------------------------------------------------------ solve
-// After the factorization each front's storage holds, row-major f x f,
-//   [0,S) x [0,S)   A11^-1,
-//   [S,f) x [0,S)   -G, G = A21 A11^-1,
-//   [0,S) x [S,f)   H = A11^-1 A12,
-// so every row of the solve is one contiguous dot product with a vector
-// gathered once per work item (t = the right-hand side on the pivots):
-//   forward,  r <  S:  z_r = t_r (kept for the backward sweep)
-//             r >= S:  u_r = w_r + F[r, 0:S] . t[0:S]      contribution to the parent
-//   backward, r <  S:  x_r = F[r, 0:f] . v[0:f]            v = (t, -x_struct)
-// A front's forward rows need only its children's contributions and its
-// backward rows only its own z and its ancestors' x: one dependent step per
-// level and sweep.  G and H hold as many entries as A21 and A12, so a solve
-// still reads sum S (2f - S) factor entries.
-
-__device__ __forceinline__ bool stopped(const int *a, const int *b)
-{
-    return (a && *a) || (b && *b);
-}
-
-constexpr int kSolveThreads = kSolveThreadsHost;   // 8 warps per work item
-constexpr int kFlowSlots = 3;   // ticket counters after the dependency counters
-constexpr int kGatherRegs = 4;   // staged gather entries per thread (fronts up to 4 x 256)
-constexpr int kThreadRowMaxF = 256;   // fronts whose forward rows a thread sums alone
-
-// Row registers: a warp that computes a single row of an item loads it into
-// registers before the item's dependency wait; rows up to kRowRegs<T> x 32
-// entries (from a 32-aligned start).
-template <class T> struct RowRegs;
-template <> struct RowRegs<float> { static constexpr int v = 32; };
-template <> struct RowRegs<double> { static constexpr int v = 16; };
-// the three-CTAs-per-SM form of the dataflow solve: fewer row registers
-template <class T> struct RowRegs3;
-template <> struct RowRegs3<float> { static constexpr int v = 16; };
-template <> struct RowRegs3<double> { static constexpr int v = 8; };
-
-template <class T, int R>
-__device__ __forceinline__ void row_load(T (&reg)[R], const T *row, int base, int lo, int hi)
-{
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-        const int c = base + lane + 32 * k;
-        reg[k] = (c >= lo && c < hi) ? row[c] : T(0);
-    }
-}
-
-template <class T, int R>
-__device__ __forceinline__ T row_dot_reg(const T (&reg)[R], const T *v, int base, int lo, int hi)
-{
-    const int lane = threadIdx.x & 31;
-    T a0 = T(0), a1 = T(0);
-#pragma unroll
-    for (int k = 0; k < R; k += 2) {
-        const int c = base + lane + 32 * k;
-        if (c >= lo && c < hi) a0 += reg[k] * v[c];
-        if (c + 32 >= lo && c + 32 < hi) a1 += reg[k + 1] * v[c + 32];
-    }
-    return warp_sum(a0 + a1);
-}
-
-// N rows' dot products by one warp at once: row u's entries [b_u, e_u) with
-// v (an empty range for an absent row), all loads in flight together.  Each
-// row has its own accumulator, so its sum does not depend on N.
-template <class T, int N, int K = (N >= 8 ? 2 : 4)>
-__device__ __forceinline__ void dotN(const T *const (&p)[N], const int (&b)[N], const int (&e)[N],
-                                     const T *v, T (&s)[N])
-{
-    const int lane = threadIdx.x & 31;
-    int lo = b[0], hi = e[0];
-#pragma unroll
-    for (int u = 1; u < N; ++u) {
-        lo = min(lo, b[u]);
-        hi = max(hi, e[u]);
-    }
-    // K column chunks of each of the N rows are loaded before any is used:
-    // N * K loads of the factor rows in flight per lane
-    T a[N];
-#pragma unroll
-    for (int u = 0; u < N; ++u) a[u] = T(0);
-    int c = (lo & ~31) + lane;
-    for (; c + 32 * (K - 1) < hi; c += 32 * K) {
-        T xv[K], rv[N][K];
-#pragma unroll
-        for (int k = 0; k < K; ++k) xv[k] = v[c + 32 * k];
-#pragma unroll
-        for (int u = 0; u < N; ++u)
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const int cc = c + 32 * k;
-                rv[u][k] = (cc >= b[u] && cc < e[u]) ? p[u][cc] : T(0);
-            }
-#pragma unroll
-        for (int u = 0; u < N; ++u)
-#pragma unroll
-            for (int k = 0; k < K; ++k) a[u] += rv[u][k] * xv[k];
-    }
-    for (; c < hi; c += 32) {
-        const T x = v[c];
-#pragma unroll
-        for (int u = 0; u < N; ++u)
-            if (c >= b[u] && c < e[u]) a[u] += p[u][c] * x;
-    }
-#pragma unroll
-    for (int u = 0; u < N; ++u) s[u] = warp_sum(a[u]);
-}
-
-template <class T>
-__device__ __forceinline__ void dot4(const T *const (&p)[4], const int (&b)[4], const int (&e)[4],
-                                     const T *v, T (&s)[4])
-{
-    dotN<T, 4>(p, b, e, v, s);
-}
-
-// Column range of row r of front (S, f) in the forward (fwd) or backward sweep.
-__device__ __forceinline__ void row_range(bool fwd, int r, int S, int f, int &lo, int &hi)
-{
-    if (fwd) {
-        lo = 0;
-        hi = r < S ? 0 : S;
-    } else {
-        lo = 0;
-        hi = f;
-    }
-}
-
-// A work item: rows [rbeg, rend) of front q in one sweep.  The parts that
-// depend on no other item (indices, scaled right-hand side, the single row a
-// warp owns) are loaded by pre(); run() then gathers the vector the rows
-// multiply (after the item's dependencies are met) and computes the rows.
-template <class T, int R = RowRegs<T>::v>
-struct SolveItemCtx {
-    bool fwd;
-    int kind;    // 0 forward rows, 1 backward rows, 2 forward gather, 3 backward gather
-    bool gath;   // rows of a front whose gather item ran (its vectors are in tw)
-    int q, S, f, vo, rbeg, rend;
-    int r0;      // first row with a product (forward: the first contribution row)
-    const T *A;
-    // staged gather (forward: vars and child maps; backward: struct vars)
-    bool staged;
-    int ch[2], m[2], uof[2];
-    int mp[2][kGatherRegs], xi[kGatherRegs];
-    T rsb[kGatherRegs];
-    // this warp's single row, if the item has at most one row per warp
-    bool onerow;
-    int base;
-    T reg[R];
-
-    __device__ __forceinline__ void pre(const MfDev &D, const T *F, const T *b,
-                                        const double *__restrict__ rs, int kind_, int gath_,
-                                        int q_, int rbeg_, int rend_)
-    {
-        kind = kind_;
-        fwd = kind == 0 || kind == 2;
-        gath = gath_ != 0 && kind < 2;
-        q = q_;
-        rbeg = rbeg_;
-        rend = rend_;
-        S = D.S[q];
-        f = D.f[q];
-        vo = D.voff[q];
-        A = F + D.foff[q];
-        const int tid = threadIdx.x, nt = blockDim.x, wid = tid >> 5, nw = nt >> 5;
-        const int *vars = D.vars + vo;
-        r0 = fwd ? max(rbeg, S) : rbeg;
-        onerow = kind < 2 && rend - r0 <= nw;
-        const int r = r0 + wid;
-        if (onerow && r < rend) {
-            int lo, hi;
-            row_range(fwd, r, S, f, lo, hi);
-            base = lo & ~31;
-            if (hi - base <= 32 * R) row_load<T, R>(reg, A + (long long)r * f, base, lo, hi);
-            else onerow = false;
-        } else {
-            onerow = false;
-        }
-        if (gath) {
-            staged = false;   // the rows read the gather item's vectors
-        } else if (fwd) {
-            ch[0] = D.child0[q];
-            ch[1] = D.child1[q];
-            for (int sl = 0; sl < 2; ++sl) {
-                m[sl] = ch[sl] >= 0 ? D.f[ch[sl]] - D.S[ch[sl]] : 0;
-                uof[sl] = ch[sl] >= 0 ? D.uoff[ch[sl]] : 0;
-            }
-            staged = f <= kGatherRegs * nt && m[0] <= kGatherRegs * nt &&
-                     m[1] <= kGatherRegs * nt;
-            if (staged) {
-                int vi[kGatherRegs];
-#pragma unroll
-                for (int k = 0; k < kGatherRegs; ++k) {
-                    const int p = tid + k * nt;
-                    vi[k] = p < S ? vars[p] : -1;
-#pragma unroll
-                    for (int sl = 0; sl < 2; ++sl) mp[sl][k] = p < m[sl] ? D.cbmap[uof[sl] + p] : 0;
-                }
-#pragma unroll
-                for (int k = 0; k < kGatherRegs; ++k)
-                    rsb[k] = vi[k] >= 0 ? (T)(rs[vi[k]] * (double)b[vi[k]]) : T(0);
-            }
-        } else {
-            staged = f - S <= kGatherRegs * nt;
-            if (staged) {
-#pragma unroll
-                for (int k = 0; k < kGatherRegs; ++k) {
-                    const int e = tid + k * nt;
-                    xi[k] = e < f - S ? vars[S + e] : 0;
-                }
-            }
-        }
-    }
-
-    // Forward gather: w (f entries: scaled b on the fully summed rows plus
-    // the children's contributions) in shared memory; t is its first S.
-    __device__ __forceinline__ void gather_w(const MfDev &D, const T *b,
-                                             const double *__restrict__ rs, const T *upd, T *w)
-    {
-        const int tid = threadIdx.x, nt = blockDim.x;
-        if (staged) {
-            T uv[2][kGatherRegs];
-#pragma unroll
-            for (int sl = 0; sl < 2; ++sl)
-#pragma unroll
-                for (int k = 0; k < kGatherRegs; ++k) {
-                    const int e = tid + k * nt;
-                    uv[sl][k] = e < m[sl] ? __ldcg(upd + uof[sl] + e) : T(0);
-                }
-#pragma unroll
-            for (int k = 0; k < kGatherRegs; ++k) {
-                const int p = tid + k * nt;
-                if (p < f) w[p] = rsb[k];
-            }
-            __syncthreads();
-#pragma unroll
-            for (int sl = 0; sl < 2; ++sl) {
-#pragma unroll
-                for (int k = 0; k < kGatherRegs; ++k)
-                    if (tid + k * nt < m[sl]) w[mp[sl][k]] += uv[sl][k];
-                __syncthreads();
-            }
-        } else {
-            // wide fronts: the same in batches of kGatherRegs entries per
-            // thread, each batch's index loads issued before its gathers
-            const int *vars = D.vars + vo;
-            for (int p0 = tid; p0 < f; p0 += kGatherRegs * nt) {
-                int vi[kGatherRegs];
-#pragma unroll
-                for (int k = 0; k < kGatherRegs; ++k) {
-                    const int p = p0 + k * nt;
-                    vi[k] = p < S ? vars[p] : -1;
-                }
-                T val[kGatherRegs];
-#pragma unroll
-                for (int k = 0; k < kGatherRegs; ++k)
-                    val[k] = vi[k] >= 0 ? (T)(rs[vi[k]] * (double)b[vi[k]]) : T(0);
-#pragma unroll
-                for (int k = 0; k < kGatherRegs; ++k)
-                    if (p0 + k * nt < f) w[p0 + k * nt] = val[k];
-            }
-            __syncthreads();
-            for (int sl = 0; sl < 2; ++sl) {
-                const int *map = D.cbmap + uof[sl];
-                const T *u = upd + uof[sl];
-                for (int e0 = tid; e0 < m[sl]; e0 += kGatherRegs * nt) {
-                    int mi[kGatherRegs];
-                    T uv[kGatherRegs];
-#pragma unroll
-                    for (int k = 0; k < kGatherRegs; ++k) {
-                        const int e = e0 + k * nt;
-                        mi[k] = e < m[sl] ? map[e] : -1;
-                        uv[k] = e < m[sl] ? __ldcg(u + e) : T(0);
-                    }
-#pragma unroll
-                    for (int k = 0; k < kGatherRegs; ++k)
-                        if (mi[k] >= 0) w[mi[k]] += uv[k];
-                }
-                __syncthreads();
-            }
-        }
-    }
-
-    // -x on the struct variables [S, f) into dst[0, f - S), in batches of
-    // kGatherRegs entries per thread (index loads first)
-    __device__ __forceinline__ void gather_struct_x(const MfDev &D, const T *x, T *dst) const
-    {
-        const int tid = threadIdx.x, nt = blockDim.x, mm = f - S;
-        if (staged) {
-#pragma unroll
-            for (int k = 0; k < kGatherRegs; ++k) {
-                const int e = tid + k * nt;
-                if (e < mm) dst[e] = -__ldcg(x + xi[k]);
-            }
-            return;
-        }
-        const int *vars = D.vars + vo + S;
-        for (int e0 = tid; e0 < mm; e0 += kGatherRegs * nt) {
-            int vi[kGatherRegs];
-#pragma unroll
-            for (int k = 0; k < kGatherRegs; ++k) vi[k] = e0 + k * nt < mm ? vars[e0 + k * nt] : -1;
-            T xv[kGatherRegs];
-#pragma unroll
-            for (int k = 0; k < kGatherRegs; ++k) xv[k] = vi[k] >= 0 ? __ldcg(x + vi[k]) : T(0);
-#pragma unroll
-            for (int k = 0; k < kGatherRegs; ++k)
-                if (vi[k] >= 0) dst[e0 + k * nt] = -xv[k];
-        }
-    }
-
-    // Forward rows: t from the gather item (gathered fronts) or gathered
-    // here; then z_r = t_r on pivot rows and u_r = w_r - G[r, 0:S] t on
-    // contribution rows.
-    __device__ __forceinline__ void run_fwd(const MfDev &D, const T *b,
-                                            const double *__restrict__ rs, T *zbuf, T *upd, T *w)
-    {
-        T *uo = upd + D.uoff[q] - S;   // row r >= S -> uo[r]
-        const T *tw = (const T *)D.tw + vo;
-        if (gath) {
-            for (int i = threadIdx.x; i < S; i += blockDim.x) w[i] = __ldcg(tw + i);
-            __syncthreads();
-        } else {
-            gather_w(D, b, rs, upd, w);
-        }
-        for (int r = rbeg + (int)threadIdx.x; r < min(rend, S); r += blockDim.x) zbuf[vo + r] = w[r];
-        if (gath) rows(w, [&](int r, T v) { uo[r] = __ldcg(tw + r) + v; });
-        else rows(w, [&](int r, T v) { uo[r] = w[r] + v; });
-    }
-
-    // Forward gather item: t on the pivot positions and w on the
-    // contribution rows into tw, once for all of the front's row items.
-    __device__ __forceinline__ void run_gather_fwd(const MfDev &D, const T *b,
-                                                   const double *__restrict__ rs, const T *upd,
-                                                   T *w)
-    {
-        gather_w(D, b, rs, upd, w);
-        T *tw = (T *)D.tw + vo;
-        for (int i = threadIdx.x; i < f; i += blockDim.x) tw[i] = w[i];
-    }
-
-    // Backward gather item: -x on the front's struct variables into tw.
-    __device__ __forceinline__ void run_gather_bwd(const MfDev &D, const T *x)
-    {
-        gather_struct_x(D, x, (T *)D.tw + vo + S);
-    }
-
-    // Backward: v = (t, -x on the front's struct variables); then the rows.
-    __device__ __forceinline__ void run_bwd(const MfDev &D, const T *zbuf, T *x, T *v)
-    {
-        const int tid = threadIdx.x, nt = blockDim.x, mm = f - S;
-        const int *vars = D.vars + vo;
-        for (int i = tid; i < S; i += nt) v[i] = __ldcg(zbuf + vo + i);
-        if (gath) {
-            const T *tw = (const T *)D.tw + vo + S;
-            for (int e = tid; e < mm; e += nt) v[S + e] = __ldcg(tw + e);
-        } else {
-            gather_struct_x(D, x, v + S);
-        }
-        __syncthreads();
-        rows(v, [&](int r, T val) { x[vars[r]] = val; });
-    }
-
-    // The item's rows: one per thread when a forward item has at least half
-    // as many rows as threads, in fronts of at most kThreadRowMaxF variables
-    // (each thread sums its row left to right, four partial sums;
-    // the row's entries come through L1 line by line and the vector entries
-    // from shared memory); one per warp from registers (at most one row per
-    // warp); otherwise G rows per warp at a time (dotN).
-    template <class Out>
-    __device__ __forceinline__ void rows(const T *vec, Out out)
-    {
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        // one row per thread: short FP32 rows only (a warp's loads touch 32
-        // rows at once, which pays only while the rows stay in L1)
-        if (fwd && f <= kThreadRowMaxF && 2 * (rend - r0) >= (int)blockDim.x) {
-            for (int r = r0 + (int)threadIdx.x; r < rend; r += blockDim.x) {
-                int lo, hi;
-                row_range(fwd, r, S, f, lo, hi);
-                const T *row = A + (long long)r * f;
-                T a0 = T(0), a1 = T(0), a2 = T(0), a3 = T(0);
-                int c = lo;
-#pragma unroll 4
-                for (; c + 3 < hi; c += 4) {
-                    a0 += row[c] * vec[c];
-                    a1 += row[c + 1] * vec[c + 1];
-                    a2 += row[c + 2] * vec[c + 2];
-                    a3 += row[c + 3] * vec[c + 3];
-                }
-                for (; c < hi; ++c) a0 += row[c] * vec[c];
-                out(r, (a0 + a1) + (a2 + a3));
-            }
-            return;
-        }
-        if (rend - r0 <= nw) {
-            const int r = r0 + wid;
-            if (r < rend) {
-                int lo, hi;
-                row_range(fwd, r, S, f, lo, hi);
-                T s = T(0);
-                if (onerow) {
-                    s = row_dot_reg<T, R>(reg, vec, base, lo, hi);
-                } else {
-                    const T *p[4] = {A + (long long)r * f, A, A, A};
-                    const int bb[4] = {lo, 0, 0, 0}, ee[4] = {hi, 0, 0, 0};
-                    T s4[4];
-                    dot4<T>(p, bb, ee, vec, s4);
-                    s = s4[0];
-                }
-                if (lane == 0) out(r, s);
-            }
-            return;
-        }
-        constexpr int G = R >= 32 ? 8 : 4;   // rows per warp in flight (register budget)
-        // column chunks per row in flight: 2 in the small-register forms
-        constexpr int KC = (R < RowRegs<T>::v || G >= 8) ? 2 : 4;
-        for (int r = r0 + wid; r < rend; r += G * nw) {
-            const T *p[G];
-            int bb[G], ee[G], rr[G];
-#pragma unroll
-            for (int u = 0; u < G; ++u) {
-                rr[u] = r + u * nw;
-                if (rr[u] < rend) {
-                    row_range(fwd, rr[u], S, f, bb[u], ee[u]);
-                    p[u] = A + (long long)rr[u] * f;
-                } else {
-                    bb[u] = ee[u] = 0;
-                    p[u] = A;
-                }
-            }
-            T sg[G];
-            dotN<T, G, KC>(p, bb, ee, vec, sg);
-            if (lane == 0) {
-#pragma unroll
-                for (int u = 0; u < G; ++u)
-                    if (rr[u] < rend) out(rr[u], sg[u]);
-            }
-        }
-    }
-};
-
-// Work item table entry: 12 ints.
-//   x: kind (0 forward, 1 backward), front, first row, end row
-//   y: wait counter 0, its target, wait counter 1, its target (-1 / 0: none)
-//   z: done counters 0 and 1 (-1: none), unused, unused
-struct SolveItemDev {
-    int4 x, y, z;
-};
-
-template <class T, int R>
-__device__ __forceinline__ void run_item(SolveItemCtx<T, R> &c, const MfDev &D, const T *b,
-                                         const double *__restrict__ rs, T *zbuf, T *upd, T *x,
-                                         T *smem)
-{
-    // shared memory: w (forward) or v (backward), up to the launch's largest front
-    switch (c.kind) {
-    case 0: c.run_fwd(D, b, rs, zbuf, upd, smem); break;
-    case 1: c.run_bwd(D, zbuf, x, smem); break;
-    case 2: c.run_gather_fwd(D, b, rs, upd, smem); break;
-    default: c.run_gather_bwd(D, x); break;
-    }
-}
-
-// One launch per level and sweep: block i runs item i0 + i (its
-// dependencies are the previous launches).
-template <class T>
-__global__ void __launch_bounds__(kSolveThreads, 2) k_solve_level(
-    const MfDev D, const T *F, const T *b, const double *__restrict__ rs, T *zbuf, T *upd, T *x,
-    const SolveItemDev *__restrict__ items, int i0, const int *stop_a, const int *stop_b)
-{
-    if (stopped(stop_a, stop_b)) return;
-    extern __shared__ unsigned char smem_raw[];
-    T *smem = reinterpret_cast<T *>(smem_raw);
-    const SolveItemDev it = items[i0 + blockIdx.x];
-    SolveItemCtx<T> c;
-    c.pre(D, F, b, rs, it.x.x, it.z.w, it.x.y, it.x.z, it.x.w);
-    run_item(c, D, b, rs, zbuf, upd, x, smem);
-}
-
-// The split form's lower-level launches: CTA size and resident CTAs per SM.
-constexpr int kLowThreads = 128;
-constexpr int kLowMinBlocks = 4;
-
-// Polls of one dependency counter before a CTA of the dataflow solve gives
-// up (each poll sleeps ~40 ns: well under a second in all).
-constexpr long long kFlowSpins = 1LL << 22;
-
-__device__ __forceinline__ int ld_acquire_gpu(const int *p)
-{
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Global nanosecond timer (per-item traces of the dataflow solve).
-__device__ __forceinline__ unsigned long long globaltimer_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Bounded wait until *ctr >= target; false if it ran out or another CTA
-// reported an error meanwhile.
-__device__ __forceinline__ void red_release_gpu(int *p, int v)
-{
-    asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-__device__ __forceinline__ bool wait_count(const int *ctr, int target, volatile int *err)
-{
-    long long spins = 0;
-    while (ld_acquire_gpu(ctr) < target) {
-        if (*err || ++spins > kFlowSpins) return false;
-        __nanosleep(40);
-    }
-    return true;
-}
-
-// The whole solve as one launch of work items in the plan's order (forward
-// bottom-up, then backward top-down).  A CTA takes items by ticket
-// (ctr[nctr]), loads what needs no other item, waits (thread 0, acquire
-// loads) until the item's counters reach their targets, runs the item and,
-// after a barrier, adds one to the item's done counters with release
-// semantics.  The plan checks that
-// every counter an item waits on is advanced only by items before it, so a
-// CTA only ever waits for items held by running CTAs: no co-resident grid is
-// needed.  A wait that runs out (or an error seen while waiting) sets
-// bar->err (bit 2) and *stop_a (so GMRES stops instead of using an
-// unfinished preconditioner) and ends the CTA.  ctr is zeroed before each
-// launch.
-// Two forms (the autotuner picks one): MINB resident CTAs per SM at least,
-// R row registers per lane (rows up to 32 R entries prefetched before the
-// wait).  Form 0: 2 CTAs and RowRegs<T> registers; form 1: 3 CTAs per SM
-// with RowRegs3<T>, more warps in flight for the levels whose items are
-// whole fronts.  A launch runs the items [item0, item1) with ticket counter
-// ctr[nctr + slot]: the whole table, or (split form) the lower levels'
-// forward items, the upper levels, the lower levels' backward items as three
-// launches in stream order -- an item then only waits for items of its own
-// launch or of an earlier, finished one.  The lower launches use NT = 128
-// threads and shared memory for their own largest front, so more of
-// their many small items are in flight per SM.
-template <class T, int R, int MINB, int NT = kSolveThreads>
-__global__ void __launch_bounds__(NT, MINB) k_solve_flow(
-    const MfDev D, const T *F, const T *b, const double *__restrict__ rs, T *zbuf, T *upd, T *x,
-    const SolveItemDev *__restrict__ items, int item0, int item1, int *ctr, int nctr,
-    int slot, MfBarrier *bar, const int *stop_a, const int *stop_b, unsigned long long *trace)
-{
-    if (stopped(stop_a, stop_b)) return;   // the flags are the same for every CTA
-    extern __shared__ unsigned char smem_raw[];
-    T *smem = reinterpret_cast<T *>(smem_raw);
-    __shared__ int item_s, ok_s;
-    volatile int *err = &bar->err;
-    int *ticket = ctr + nctr + slot;
-    int next = threadIdx.x == 0 ? item0 + atomicAdd(ticket, 1) : 0;
-    for (;;) {
-        if (threadIdx.x == 0) item_s = next;
-        __syncthreads();
-        const int i = item_s;
-        if (i >= item1) return;
-        const SolveItemDev it = items[i];
-        if (trace && threadIdx.x == 0) trace[3 * i] = globaltimer_ns();
-        SolveItemCtx<T, R> c;
-        c.pre(D, F, b, rs, it.x.x, it.z.w, it.x.y, it.x.z, it.x.w);
-        if (threadIdx.x == 0) {
-            next = item0 + atomicAdd(ticket, 1);   // in flight during the wait
-            bool ok = true;
-            if (it.y.x >= 0 && it.y.y > 0) ok = wait_count(ctr + it.y.x, it.y.y, err);
-            if (ok && it.y.z >= 0 && it.y.w > 0) ok = wait_count(ctr + it.y.z, it.y.w, err);
-            if (!ok) {
-                atomicOr(&bar->err, 2);
-                if (stop_a) atomicExch(const_cast<int *>(stop_a), 1);
-            }
-            ok_s = ok;
-        }
-        __syncthreads();
-        if (!ok_s) return;
-        if (trace && threadIdx.x == 0) trace[3 * i + 1] = globaltimer_ns();
-        run_item(c, D, b, rs, zbuf, upd, x, smem);
-        // the barrier orders every thread's writes before thread 0's release
-        // additions (cumulative at GPU scope), which the waiters' acquire
-        // loads pair with
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            if (it.z.x >= 0) red_release_gpu(ctr + it.z.x, 1);
-            if (it.z.y >= 0) red_release_gpu(ctr + it.z.y, 1);
-            if (trace) trace[3 * i + 2] = globaltimer_ns();
-        }
-    }
-}
-
 // ---------------------------------------------------------- transposed solve
 // The transposed solve is the adjoint of the solve's steps taken in reverse
 // order.  Bottom-up (adjoint of the backward sweep): the front gathers g on
@@ -1664,6 +1104,58 @@ static cudaError_t raise_dyn_smem(const void *fn, size_t bytes)
     return e;
 }
 
+// The split form's lower-level launches: threads that compute an item and
+// resident CTAs per SM.
+constexpr int kLowThreads = 128;
+constexpr int kLowMinBlocks = 4;
+
+// Shared memory of a dataflow launch whose largest front has maxf variables
+// (es bytes each), `want` CTAs per SM at most: the vector, then kStages chunks
+// of what is left of the SM's share.  A chunk below kMinChunk holds too few
+// rows to stage (each CTA then takes a larger share, or reads its rows from
+// global memory).
+static FlowShape flow_shape(int maxf, size_t es, int want)
+{
+    constexpr int kMinChunk = 8192;
+    FlowShape sh;
+    sh.vbytes = (int)(((size_t)maxf * es + 127) / 128 * 128);
+    for (int d = want; d >= 1; --d) {
+        const int share = std::min(227 * 1024, 228 * 1024 / d - 1024) - (int)sizeof(FlowShared) - 256;
+        sh.cbytes = std::max(0, (share - sh.vbytes) / kStages) / 128 * 128;
+        if (sh.cbytes >= kMinChunk) break;
+    }
+    if (sh.cbytes < 1024) sh.cbytes = 0;
+    sh.smem = (size_t)sh.vbytes + (size_t)kStages * sh.cbytes;
+    return sh;
+}
+
+// The kernel of a form (0, 1; 2: the split form's lower levels) of the
+// dataflow solve.
+template <class T> static const void *flow_kernel(int form)
+{
+    return form == 0 ? (const void *)k_solve_flow<T, 2>
+                     : form == 1 ? (const void *)k_solve_flow<T, 3>
+                                 : (const void *)k_solve_flow<T, kLowMinBlocks, kLowThreads>;
+}
+
+// Sizes one form's launches for fronts of up to maxf variables; per_sm CTAs
+// at most.
+static int flow_setup(const MfFactor *M, int form, int maxf, int per_sm, FlowShape *out)
+{
+    const size_t es = M->fp32 ? sizeof(float) : sizeof(double);
+    const void *fn = M->fp32 ? flow_kernel<float>(form) : flow_kernel<double>(form);
+    FlowShape sh = flow_shape(maxf, es, per_sm);
+    V2D_CUDA_TRY(raise_dyn_smem(fn, sh.smem));
+    int dev = 0, nsm = 0, occ = 0;
+    V2D_CUDA_TRY(cudaGetDevice(&dev));
+    V2D_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    V2D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &occ, fn, 32 + (form == 2 ? kLowThreads : kSolveThreads), sh.smem));
+    sh.grid = nsm * std::min(occ, per_sm);
+    *out = sh;
+    return V2D_OK;
+}
+
 int mf_factor_create(const MfPlan *P, int fp32, int fact64, MfFactor **out)
 {
     *out = nullptr;
@@ -1678,8 +1170,15 @@ int mf_factor_create(const MfPlan *P, int fp32, int fact64, MfFactor **out)
     };
     grab(&M->F, (size_t)P->ftotal * esf);
     if (M->fact64) grab(&M->F32, (size_t)P->ftotal * sizeof(float));
-    grab(&M->upd, (size_t)P->utotal * es);
-    grab(&M->z, (size_t)P->vtotal * es);
+    // tickets, then upd, then z: one fill before each dataflow solve
+    const size_t upd0 = 128, z0 = upd0 + ((size_t)P->utotal * es + 127) / 128 * 128;
+    M->msg_bytes = z0 + (size_t)P->vtotal * es;
+    grab(&M->msg, M->msg_bytes);
+    if (e == cudaSuccess) {
+        M->tickets = (int *)M->msg;
+        M->upd = (char *)M->msg + upd0;
+        M->z = (char *)M->msg + z0;
+    }
     long long cols = 0;   // front variables of the largest level
     for (int L = 0; L < P->nlevel; ++L) {
         long long v = 0;
@@ -1687,9 +1186,7 @@ int mf_factor_create(const MfPlan *P, int fp32, int fact64, MfFactor **out)
         cols = std::max(cols, v);
     }
     grab(&M->cols, (size_t)cols * kPiv * esf);
-    grab((void **)&M->sctr, (size_t)(P->nctr + kFlowSlots) * sizeof(int));
     grab(&M->wb, (size_t)P->vtotal * es);
-    grab(&M->tw, (size_t)P->vtotal * es);
     grab((void **)&M->rs, (size_t)P->n * sizeof(double));
     grab((void **)&M->flag, sizeof(int));
     grab((void **)&M->bar, sizeof(MfBarrier));
@@ -1722,14 +1219,10 @@ int mf_factor_create(const MfPlan *P, int fp32, int fact64, MfFactor **out)
     }
     if (fp32) {
         attr((const void *)k_solve_level<float>, solve);
-        attr((const void *)k_solve_flow<float, RowRegs<float>::v, 2>, solve);
-        attr((const void *)k_solve_flow<float, RowRegs3<float>::v, 3>, solve);
         attr((const void *)k_tup_front<float>, tsolve);
         attr((const void *)k_tdown_front<float>, tsolve);
     } else {
         attr((const void *)k_solve_level<double>, solve);
-        attr((const void *)k_solve_flow<double, RowRegs<double>::v, 2>, solve);
-        attr((const void *)k_solve_flow<double, RowRegs3<double>::v, 3>, solve);
         attr((const void *)k_tup_front<double>, tsolve);
         attr((const void *)k_tdown_front<double>, tsolve);
     }
@@ -1745,33 +1238,20 @@ int mf_factor_create(const MfPlan *P, int fp32, int fact64, MfFactor **out)
         mf_factor_destroy(M);
         return V2D_ECUDA;
     }
-    // dataflow solve: as many CTAs as can be resident at once (two per SM at
-    // most), never more than there are work items
-    int dev = 0, nsm = 0, per_sm = 0;
-    cudaError_t oe = cudaGetDevice(&dev);
-    if (oe == cudaSuccess) oe = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (oe == cudaSuccess)
-        oe = fp32 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                        &per_sm, k_solve_flow<float, RowRegs<float>::v, 2>, kSolveThreads, solve)
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                        &per_sm, k_solve_flow<double, RowRegs<double>::v, 2>, kSolveThreads,
-                        solve);
-    int per_sm1 = 0;
-    if (oe == cudaSuccess)
-        oe = fp32 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                        &per_sm1, k_solve_flow<float, RowRegs3<float>::v, 3>, kSolveThreads,
-                        solve)
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                        &per_sm1, k_solve_flow<double, RowRegs3<double>::v, 3>, kSolveThreads,
-                        solve);
-    if (oe != cudaSuccess || per_sm <= 0) {
-        set_error("mf_factor: occupancy of the dataflow solve: %s",
-                  oe != cudaSuccess ? cudaGetErrorString(oe) : "no CTA fits on an SM");
+    // dataflow solve: as many CTAs as can be resident at once, two (form 0) or
+    // three (form 1) per SM
+    for (int form = 0; form < 2; ++form) {
+        const int st = flow_setup(M, form, P->maxf, 2 + form, &M->shape[form]);
+        if (st != V2D_OK) {
+            mf_factor_destroy(M);
+            return st;
+        }
+    }
+    if (M->shape[0].grid <= 0) {
+        set_error("mf_factor: no CTA of the dataflow solve fits on an SM");
         mf_factor_destroy(M);
         return V2D_ECUDA;
     }
-    M->flow_grid = std::max(1, nsm * std::min(per_sm, 2));
-    M->flow_grid1 = per_sm1 > 0 ? nsm * std::min(per_sm1, 3) : 0;
     cudaGetLastError();
     *out = M;
     return V2D_OK;
@@ -1781,8 +1261,7 @@ void mf_factor_destroy(MfFactor *M)
 {
     if (!M) return;
     if (M->graph) cudaGraphExecDestroy(M->graph);
-    void *ptrs[] = {M->F,  M->F32, M->upd,  M->z,   M->cols, M->wb,
-                    M->tw, M->rs,  M->flag, M->bar, M->sctr};
+    void *ptrs[] = {M->F, M->F32, M->msg, M->cols, M->wb, M->rs, M->flag, M->bar};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     delete M;
@@ -1794,8 +1273,8 @@ MfDev mf_dev(const MfPlan *P, const MfFactor *M)
     D.S = P->d_S; D.f = P->d_f; D.voff = P->d_voff; D.uoff = P->d_uoff;
     D.child0 = P->d_child0; D.child1 = P->d_child1; D.parent = P->d_parent; D.foff = P->d_foff;
     D.vars = P->d_vars; D.cbmap = P->d_cbmap;
+    D.inv0 = P->d_inv0; D.inv1 = P->d_inv1;
     D.maxS = P->maxS; D.maxf = P->maxf;
-    D.tw = M->tw;
     return D;
 }
 
@@ -1939,32 +1418,33 @@ static int apply_launches(const MfPlan *P, const MfFactor *M, const T *b, T *x, 
     const MfDev D = mf_dev(P, M);
     const T *F = (const T *)(M->fact64 ? M->F32 : M->F);
     T *z = (T *)M->z, *upd = (T *)M->upd;
-    const SolveItemDev *items = (const SolveItemDev *)P->d_items;
+    const SolveItemDev *items = P->d_items;
     const size_t smf = (size_t)P->maxf * sizeof(T);
     long long launches = 0;
     if (M->flow) {
-        V2D_CUDA_TRY(cudaMemsetAsync(M->sctr, 0, (size_t)(P->nctr + kFlowSlots) * sizeof(int), s));
+        // every message unset (0xff bytes: a NaN no arithmetic gives), tickets -1
+        V2D_CUDA_TRY(cudaMemsetAsync(M->msg, 0xff, M->msg_bytes, s));
+        V2D_CUDA_TRY(cudaMemsetAsync(x, 0xff, (size_t)P->n * sizeof(T), s));
+        const FlowShape &up = M->shape[M->flow_form], &lo = M->shape[2];
         auto upper = [&](int i0, int i1, int slot) {
-            const int n = std::max(1, i1 - i0);
-            if (M->flow_form == 1 && M->flow_grid1 > 0)
-                k_solve_flow<T, RowRegs3<T>::v, 3><<<std::min(n, M->flow_grid1), kSolveThreads, smf,
-                                                     s>>>(D, F, b, M->rs, z, upd, x, items, i0, i1,
-                                                          M->sctr, P->nctr, slot, M->bar,
-                                                          stop_a, stop_b, trace);
+            const int n = std::max(1, std::min(i1 - i0, up.grid));
+            if (M->flow_form == 1)
+                k_solve_flow<T, 3><<<n, kSolveThreads + 32, up.smem, s>>>(
+                    D, F, b, M->rs, z, upd, x, items, i0, i1, up.vbytes, up.cbytes,
+                    M->tickets, slot, M->bar, stop_a, stop_b, trace);
             else
-                k_solve_flow<T, RowRegs<T>::v, 2><<<std::min(n, M->flow_grid), kSolveThreads, smf,
-                                                    s>>>(D, F, b, M->rs, z, upd, x, items, i0, i1,
-                                                         M->sctr, P->nctr, slot, M->bar,
-                                                         stop_a, stop_b, trace);
+                k_solve_flow<T, 2><<<n, kSolveThreads + 32, up.smem, s>>>(
+                    D, F, b, M->rs, z, upd, x, items, i0, i1, up.vbytes, up.cbytes,
+                    M->tickets, slot, M->bar, stop_a, stop_b, trace);
         };
         auto lower = [&](int i0, int i1, int slot) {
-            k_solve_flow<T, RowRegs<T>::v, kLowMinBlocks, kLowThreads>
-                <<<std::max(1, std::min(i1 - i0, M->low_grid)), kLowThreads, M->low_smem, s>>>(
-                    D, F, b, M->rs, z, upd, x, items, i0, i1, M->sctr, P->nctr, slot,
-                    M->bar, stop_a, stop_b, trace);
+            k_solve_flow<T, kLowMinBlocks, kLowThreads>
+                <<<std::max(1, std::min(i1 - i0, lo.grid)), kLowThreads + 32, lo.smem, s>>>(
+                    D, F, b, M->rs, z, upd, x, items, i0, i1, lo.vbytes, lo.cbytes,
+                    M->tickets, slot, M->bar, stop_a, stop_b, trace);
         };
         const int Ls = M->split;
-        if (Ls > 0 && Ls < P->nlevel && M->low_grid > 0) {
+        if (Ls > 0 && Ls < P->nlevel && lo.grid > 0) {
             lower(P->lvl_fwd[0], P->lvl_fwd[Ls], 0);
             V2D_TRY(solve_launch("k_solve_flow (lower levels, forward)", 0));
             V2D_TRY(mark(kCodeFlow * 1000));
@@ -1982,30 +1462,22 @@ static int apply_launches(const MfPlan *P, const MfFactor *M, const T *b, T *x, 
             launches = 1;
         }
     } else {
-        // a level's gather items (first in its range) are a launch of their own
+        // a level's gather items (first in its range) need no launch
         for (int L = 0; L < P->nlevel; ++L) {
-            const int i0 = P->lvl_fwd[L], ni = P->lvl_fwd[L + 1] - i0, ng = P->lvl_fwd_g[L];
-            for (const int part : {0, 1}) {
-                const int a = part == 0 ? i0 : i0 + ng, n = part == 0 ? ng : ni - ng;
-                if (n == 0) continue;
-                k_solve_level<T><<<n, kSolveThreads, smf, s>>>(D, F, b, M->rs, z, upd, x, items,
-                                                              a, stop_a, stop_b);
-                V2D_TRY(solve_launch("k_solve_level (forward)", L));
-                V2D_TRY(mark(kCodeFwdLevel * 1000 + L));
-                ++launches;
-            }
+            const int i0 = P->lvl_fwd[L] + P->lvl_fwd_g[L], n = P->lvl_fwd[L + 1] - i0;
+            k_solve_level<T><<<n, kSolveThreads, smf, s>>>(D, F, b, M->rs, z, upd, x, items, i0,
+                                                          stop_a, stop_b);
+            V2D_TRY(solve_launch("k_solve_level (forward)", L));
+            V2D_TRY(mark(kCodeFwdLevel * 1000 + L));
+            ++launches;
         }
         for (int L = P->nlevel - 1; L >= 0; --L) {
-            const int i0 = P->lvl_bwd[L + 1], ni = P->lvl_bwd[L] - i0, ng = P->lvl_bwd_g[L];
-            for (const int part : {0, 1}) {
-                const int a = part == 0 ? i0 : i0 + ng, n = part == 0 ? ng : ni - ng;
-                if (n == 0) continue;
-                k_solve_level<T><<<n, kSolveThreads, smf, s>>>(D, F, b, M->rs, z, upd, x, items,
-                                                              a, stop_a, stop_b);
-                V2D_TRY(solve_launch("k_solve_level (backward)", L));
-                V2D_TRY(mark(kCodeBwdLevel * 1000 + L));
-                ++launches;
-            }
+            const int i0 = P->lvl_bwd[L + 1] + P->lvl_bwd_g[L], n = P->lvl_bwd[L] - i0;
+            k_solve_level<T><<<n, kSolveThreads, smf, s>>>(D, F, b, M->rs, z, upd, x, items, i0,
+                                                          stop_a, stop_b);
+            V2D_TRY(solve_launch("k_solve_level (backward)", L));
+            V2D_TRY(mark(kCodeBwdLevel * 1000 + L));
+            ++launches;
         }
     }
     V2D_CUDA_TRY(cudaGetLastError());
@@ -2071,21 +1543,10 @@ int mf_set_split(const MfPlan *P, MfFactor *M, int split)
     }
     int wcap = 0;
     for (int L = 0; L < split; ++L) wcap = std::max(wcap, P->lvl_maxf[L]);
-    const size_t es = M->fp32 ? sizeof(float) : sizeof(double);
-    const size_t bytes = (size_t)wcap * es;
-    const void *fn = M->fp32
-                         ? (const void *)k_solve_flow<float, RowRegs<float>::v, kLowMinBlocks,
-                                                      kLowThreads>
-                         : (const void *)k_solve_flow<double, RowRegs<double>::v, kLowMinBlocks,
-                                                      kLowThreads>;
-    V2D_CUDA_TRY(raise_dyn_smem(fn, bytes));
-    int dev = 0, nsm = 0, per_sm = 0;
-    V2D_CUDA_TRY(cudaGetDevice(&dev));
-    V2D_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    V2D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLowThreads, bytes));
-    V2D_ARG_CHECK(per_sm > 0, "lu split: no CTA of the lower-level launch fits on an SM");
-    M->low_smem = bytes;
-    M->low_grid = nsm * per_sm;
+    FlowShape sh;
+    V2D_TRY(flow_setup(M, 2, wcap, kLowMinBlocks, &sh));
+    V2D_ARG_CHECK(sh.grid > 0, "lu split: no CTA of the lower-level launch fits on an SM");
+    M->shape[2] = sh;
     M->split = split;
     return V2D_OK;
 }

@@ -1,24 +1,22 @@
 """In-house autotuner of the LU preconditioner solve's work-item granularity.
 
 The solve (one dataflow launch over the front tree) runs in one of two
-kernel forms (more resident CTAs per SM, or more row registers per lane) and
-splits each front's rows
+kernel forms (two resident CTAs per SM, or three with less shared memory each)
+and splits each front's rows
 into work items; on tree level L an item is ``rows[L]`` rows of one front, or
-the whole front (0), or, for ``rows[L] = -R``, R rows after one gather item
-per front that collects the front's right-hand side once for all of its
-items.  Small items spread a level's rows over more CTAs and shorten the
-chain of dependent steps; large ones gather each front's right-hand side once
-and keep a CTA's rows together; gather items add one dependent step but
-spare every item the indexed gather.  Which wins depends on
+the whole front (0); ``rows[L] = -R`` is the split of R with a place for one
+gather item per split front in the plan, which the kernels skip (every item
+gathers its own right-hand side).  Small items spread a level's rows over more
+CTAs and shorten the chain of dependent steps; large ones gather each front's
+right-hand side once and keep a CTA's rows together.  Which wins depends on
 the grid, the precision and the GPU, so it is measured: a coordinate search
 over the levels (each level's candidates tried with the others fixed, two
 sweeps), then the split form (the lower levels as launches of their own with
 smaller CTAs, ``split`` levels, followed by one more sweep over those
 levels' rows), every trial timed as the average of warm applications of the
 current factors (``v2d_solver_time_lu_apply``, factors in L2 as inside
-GMRES).  Every setting forms the same products; a row's partial sums are
-added in an order that depends on the split, so results agree to rounding
-and each Krylov solve still meets its tolerance.
+GMRES).  Every setting forms the same products and adds a row's in the same
+order.
 
 The result can be written to a JSON file keyed by grid shape, precision and
 leaf size, and read back (``Config.lu_item_rows``, ``load_tuning``).
@@ -34,8 +32,8 @@ import numpy as np
 from . import _lib
 from ._lib import check, lib
 
-# rows per item: 0 whole fronts, R > 0 R-row items, R < 0 (-R)-row items
-# after one gather item per split front
+# rows per item: 0 whole fronts, R > 0 R-row items, R < 0 (-R)-row items with
+# a gather item per split front in the plan
 CANDIDATES = (0, 8, 16, 32, 64, 128, 256, -8, -16, -32, -64, -128, -256)
 
 

@@ -447,7 +447,7 @@ def factor_rate(torch, _lib, s):
     codes = (ctypes.c_int * cap)()
     n = ctypes.c_int()
     _lib.check(_lib.lib().v2d_solver_time_lu_factor(s.dev.h, 1, ms, codes, cap, ctypes.byref(n)))
-    fkinds = ["rowscale", "scatter", "assemble", "-", "row_block", "-", "update",
+    fkinds = ["rowscale", "scatter", "assemble", "leaves", "row_block", "-", "update",
               "-", "-", "-", "-", "round_f32"]
     by_kind = {}
     for k in range(n.value):
@@ -729,7 +729,7 @@ def profile_lu_launches(args):
                       "per_launch_us": [[kind, lvl, round(1e3 * t, 2)] for kind, lvl, t in rows]}
     if SOLVER.get("lu_solve", "flow") == "flow":
         out["dataflow_trace"] = lu_trace_summary(s)
-    fkinds = ["rowscale", "scatter", "assemble", "-", "row_block", "-", "update",
+    fkinds = ["rowscale", "scatter", "assemble", "leaves", "row_block", "-", "update",
               "-", "-", "-", "-", "round_f32"]
     cap = 16384
     ms = (ctypes.c_double * cap)()

@@ -462,8 +462,8 @@ int v2d_solver_time_lu_launches(v2d_solver *s, int reps, long long flush_bytes, 
 /* Measurement aid (no reference counterpart): the device time of each kernel
  * of one LU factorization of the last assembled Jacobian, launched directly,
  * averaged over `reps` (codes kind * 1000 + level; kinds 0 row scaling,
- * 1 scatter, 2 extend-add with the first pivot-block inverse, 4 row block of
- * a step, 6 update of the front with the next step's pivot-block inverse,
+ * 1 scatter, 2 extend-add with the first pivot-block inverse, 3 leaves, 4 row
+ * block of a step, 6 update of the front with the next step's pivot-block inverse,
  * 11 rounding to FP32). */
 int v2d_solver_time_lu_factor(v2d_solver *s, int reps, double *ms, int *codes, int cap, int *n);
 

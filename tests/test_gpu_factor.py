@@ -23,15 +23,12 @@ WIDTHS = [(15, 13), (16, 13), (17, 13), (31, 17), (32, 17), (33, 17), (48, 33), 
           (64, 32), (65, 33), (127, 64), (129, 67)]
 
 
-@pytest.mark.parametrize("imax,jmax", WIDTHS)
-@pytest.mark.parametrize("precision,factors,limit", [("fp64", "fp32", 3), ("mixed", "fp32", 7),
-                                                     ("mixed", "fp64", 7)])
-def test_elimination_widths(v2d, oracle_mod, imax, jmax, precision, factors, limit):
+def one_update(v2d, oracle_mod, imax, jmax, limit, **config):
+    """One Newton update on an imax x jmax grid against SciPy's direct solve."""
     xg, yg = oracle_mod.generate_cylinder(imax, jmax)
     s = v2d.Solver(v2d.Config(verbose=False, write_csv=False, write_xdmf=False, re=80.0,
                               steady=False, dt_phys=0.2, farfield_bc="outflow", alpha_deg=4.0,
-                              ksp_rtol=1e-12, ksp_restart=30, precision=precision,
-                              lu_factors=factors), mesh=(xg, yg))
+                              ksp_rtol=1e-12, ksp_restart=30, **config), mesh=(xg, yg))
     M = oracle_mod.core().compute_metrics(1 / (imax - 1), 1 / (jmax - 1), xg, yg)
     st = smooth_state(M[8], M[9])
     s.set_state(*st)
@@ -47,3 +44,29 @@ def test_elimination_widths(v2d, oracle_mod, imax, jmax, precision, factors, lim
     s.close()
     assert np.max(np.abs(got - dq)) <= 1e-9 * max(1.0, np.max(np.abs(dq)))
     assert lin.converged and lin.iterations <= limit, lin.iterations
+
+
+@pytest.mark.parametrize("imax,jmax", WIDTHS)
+@pytest.mark.parametrize("precision,factors,limit", [("fp64", "fp32", 3), ("mixed", "fp32", 7),
+                                                     ("mixed", "fp64", 7)])
+def test_elimination_widths(v2d, oracle_mod, imax, jmax, precision, factors, limit):
+    one_update(v2d, oracle_mod, imax, jmax, limit, precision=precision, lu_factors=factors)
+
+
+# The leaf kernel's blocks of 32 and 8 pivots (at most 128 = 64 nodes) and the
+# leaves beyond it, eliminated like the other fronts; the whole grid one leaf
+@pytest.mark.parametrize("leaf,imax,jmax", [(4, 23, 19), (9, 23, 19), (16, 33, 33), (17, 33, 29),
+                                            (33, 41, 27), (48, 41, 35), (63, 63, 31), (64, 33, 33),
+                                            (64, 8, 8), (65, 33, 33), (100, 37, 33), (512, 16, 16)])
+@pytest.mark.parametrize("precision,factors,limit", [("fp64", "fp32", 3), ("mixed", "fp32", 7),
+                                                     ("mixed", "fp64", 7)])
+def test_leaf_sizes(v2d, oracle_mod, monkeypatch, leaf, imax, jmax, precision, factors, limit):
+    defaults = v2d._lib.krylov_defaults
+
+    def with_leaf():   # a parameter of the C interface only
+        k = defaults()
+        k.lu_leaf = leaf
+        return k
+
+    monkeypatch.setattr(v2d._lib, "krylov_defaults", with_leaf)
+    one_update(v2d, oracle_mod, imax, jmax, limit, precision=precision, lu_factors=factors)

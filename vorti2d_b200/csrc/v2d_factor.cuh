@@ -51,15 +51,38 @@ __global__ void k_rowscale(int n, const int *__restrict__ rowptr, const double *
     }
 }
 
-// Every front's own matrix entries, row-scaled, into the zeroed fronts.
+// Every front's own matrix entries, row-scaled, into the zeroed fronts: one
+// entry per position, so a plain store (a read of the zero would cost a second
+// trip to memory), four entries of a thread in flight (513 x 513 FP64: 0.56 ms
+// with += and one entry at a time).
+constexpr int kScatterEntries = 4;
+
 template <class T>
-__global__ void k_scatter(long long n, const int *__restrict__ csr, const int *__restrict__ row,
-                          const long long *__restrict__ pos, const double *__restrict__ val,
-                          const double *__restrict__ rs, T *F)
+__global__ void __launch_bounds__(256) k_scatter(long long n, const int *__restrict__ csr,
+                                                 const int *__restrict__ row,
+                                                 const long long *__restrict__ pos,
+                                                 const double *__restrict__ val,
+                                                 const double *__restrict__ rs, T *F)
 {
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n;
-         e += (long long)gridDim.x * blockDim.x)
-        F[pos[e]] += (T)(val[csr[e]] * rs[row[e]]);
+    const long long e0 = (long long)blockIdx.x * (256 * kScatterEntries) + threadIdx.x;
+    int c[kScatterEntries], r[kScatterEntries];
+    long long p[kScatterEntries];
+#pragma unroll
+    for (int k = 0; k < kScatterEntries; ++k) {
+        const long long e = e0 + 256 * k;
+        c[k] = e < n ? csr[e] : -1;
+        r[k] = e < n ? row[e] : 0;
+        p[k] = e < n ? pos[e] : 0;
+    }
+    double v[kScatterEntries], s[kScatterEntries];
+#pragma unroll
+    for (int k = 0; k < kScatterEntries; ++k) {
+        v[k] = c[k] >= 0 ? val[c[k]] : 0.0;
+        s[k] = c[k] >= 0 ? rs[r[k]] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kScatterEntries; ++k)
+        if (c[k] >= 0) F[p[k]] = (T)(v[k] * s[k]);
 }
 
 // inv[slot][voff[P] + cbmap[e]] = e for each front's contribution variables:
@@ -227,7 +250,8 @@ __device__ __forceinline__ double reciprocal(double x)
     return fma(y, fma(-x, y, 1.0), y);
 }
 
-// In-place inverse of the 32 x 32 block at M by four warps: lane = row,
+// In-place inverse of the n x n block at M (n <= 32, rows ld apart; padded by
+// the identity in registers) by four warps: lane = row,
 // column 4 i + w in register i of warp w.  Gauss-Jordan in panels of four
 // columns, one of each warp: the warps exchange the panel through shared
 // memory (one barrier) and each eliminates its four columns on its own copy
@@ -242,13 +266,17 @@ __device__ __forceinline__ double reciprocal(double x)
 // column s.  9.0e3 clocks; one warp with whole rows in registers 1.8e4, a
 // barrier per column instead of per panel 1.0e4.  Returns whether a pivot
 // column was zero.
-__device__ __forceinline__ bool invert32(double *M, double (*col)[kPanel][kHalf], int *piv)
+__device__ __forceinline__ bool invert32(double *M, int ld, int n, double (*col)[kPanel][kHalf],
+                                         int *piv)
 {
     constexpr int R = kHalf / kPanel;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double a[R];
 #pragma unroll
-    for (int i = 0; i < R; ++i) a[i] = M[lane * kLdX + kPanel * i + w];
+    for (int i = 0; i < R; ++i) {
+        const int c = kPanel * i + w;
+        a[i] = lane < n && c < n ? M[lane * ld + c] : (lane == c ? 1.0 : 0.0);
+    }
     bool bad = false, used = false;
     int step = 0;
     double scale = 0.0;
@@ -294,7 +322,10 @@ __device__ __forceinline__ bool invert32(double *M, double (*col)[kPanel][kHalf]
     }
     pivot_sync();
 #pragma unroll
-    for (int i = 0; i < R; ++i) M[step * kLdX + piv[kPanel * i + w]] = a[i] * scale;
+    for (int i = 0; i < R; ++i) {
+        const int c = piv[kPanel * i + w];
+        if (step < n && c < n) M[step * ld + c] = a[i] * scale;
+    }
     return bad;
 }
 
@@ -310,7 +341,7 @@ __device__ __forceinline__ void invert_block(PivotSmem &sm, int w, int *flag)
         // the step's block X, its row O, its column C and the rest Y
         double *X = sm.M + h * (kHalf * kLdX + kHalf), *Y = sm.M + (1 - h) * (kHalf * kLdX + kHalf);
         double *O = sm.M + (h ? kHalf * kLdX : kHalf), *C = sm.M + (h ? kHalf : kHalf * kLdX);
-        bad |= invert32(X, sm.col, sm.piv);
+        bad |= invert32(X, kLdX, kHalf, sm.col, sm.piv);
         pivot_sync();
         if (nh == 1) break;
 #pragma unroll 1
@@ -567,9 +598,9 @@ __global__ void __launch_bounds__(256) k_row_block(int q0, int k, int nt, int v0
     extern __shared__ __align__(16) unsigned char tile_raw[];
     const int q = q0 + blockIdx.x / (2 * nt), tile = blockIdx.x % (2 * nt);
     const int S = S_[q], f = f_[q];
-    if (S <= k) return;
-    const int w = min(kPiv, S - k), e = k + w;
     T *A = F + foff[q];
+    const int w = min(kPiv, S - k), e = k + w;
+    if (S <= k) return;
     if (tile >= nt) {
         const int r0 = (tile - nt) * kTile;
         const int nr = min(kTile, f - r0);
@@ -617,15 +648,15 @@ __global__ void __launch_bounds__(256, 3) k_update(int q0, int k, int nt, int v0
     extern __shared__ __align__(16) unsigned char tile_raw[];
     const int q = q0 + blockIdx.x / (nt * nt), t = blockIdx.x % (nt * nt);
     const int S = S_[q], f = f_[q];
-    if (S <= k) return;
     const int w = min(kPiv, S - k), e = k + w;
+    T *A = F + foff[q];
+    const T *Cq = C + (long long)(voff[q] - v0) * kPiv;
+    if (S <= k) return;
     // tiles in row order, the one of the next pivot block exchanged with the first
     const int next = e < S ? (e / kTile) * (nt + 1) : -1;
     const int t0 = next < 0 ? t : (t == 0 ? next : (t == next ? 0 : t));
     const int r0 = (t0 / nt) * kTile, c0 = (t0 % nt) * kTile;
     if (r0 >= f || c0 >= f || (r0 >= k && min(r0 + kTile, f) <= e)) return;
-    T *A = F + foff[q];
-    const T *Cq = C + (long long)(voff[q] - v0) * kPiv;
     typename Tile<T>::Smem *sm = reinterpret_cast<typename Tile<T>::Smem *>(tile_raw);
     Tile<T> acc;
     // the old entries, negated: loaded while the operands are on their way
@@ -665,6 +696,253 @@ __global__ void __launch_bounds__(256, 3) k_update(int q0, int k, int nt, int v0
     if (threadIdx.x >= kInvThreads) return;
     invert_block(ps, wn, flag);
     store_block(ps, wn, A + (long long)e * f + e, f);
+}
+
+// ------------------------------------------------------------------ leaves
+// A front without children holds matrix entries only: A12 and A21 are sparse (a
+// struct variable couples to a few pivots next to it) and A22 is zero.  So only
+// A11 is eliminated densely, and H = A11^-1 A12, G = A21 A11^-1 and the Schur
+// complement -G A12 are sums over those few entries: 2 S^3 flops and one write
+// of the front instead of 2 S f^2 and a read and a write of it per step, and no
+// zero fill and scatter before.
+//
+// Setup (k_leaf_lists, once per plan): each leaf's A12 entries by column and
+// A21 entries by row, as (CSR entry, pivot index) in `list` at the leaf's range
+// of assembly entries; ptr12[uoff + q + j] / ptr21[...] the first entry of
+// struct variable j, j = 0 .. m.  stat[0]: the most A12 entries of a leaf;
+// stat[1]: leaves with more than the setup's arrays hold.
+constexpr int kLeafMaxS = 128;
+constexpr int kLeafMaxEntries = 2048;   // A12 or A21 entries of a leaf
+
+__global__ void __launch_bounds__(256) k_leaf_lists(const int *__restrict__ S_,
+                                                    const int *__restrict__ f_,
+                                                    const long long *__restrict__ foff,
+                                                    const int *__restrict__ uoff,
+                                                    const long long *__restrict__ aoff,
+                                                    const int *__restrict__ csr,
+                                                    const long long *__restrict__ pos, int2 *list,
+                                                    long long *ptr12, long long *ptr21, int *stat)
+{
+    __shared__ int key[2][kLeafMaxEntries], id[2][kLeafMaxEntries], cnt[2];
+    const int q = blockIdx.x, S = S_[q], f = f_[q], m = f - S;
+    const long long a0 = aoff[q], a1 = aoff[q + 1];
+    if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
+    __syncthreads();
+    for (long long e = a0 + threadIdx.x; e < a1; e += blockDim.x) {
+        const int p = (int)(pos[e] - foff[q]), r = p / f, c = p - r * f;
+        if (r < S && c < S) continue;
+        const int h = r < S ? 0 : 1;   // A12, keyed by (column, row); A21 by (row, column)
+        const int k = atomicAdd(&cnt[h], 1);
+        if (k < kLeafMaxEntries) {
+            key[h][k] = h == 0 ? c * f + r : p;
+            id[h][k] = csr[e];
+        }
+    }
+    __syncthreads();
+    const int n0 = cnt[0], n1 = cnt[1];
+    if (n0 > kLeafMaxEntries || n1 > kLeafMaxEntries) {
+        if (threadIdx.x == 0) atomicAdd(&stat[1], 1);
+        return;
+    }
+    if (threadIdx.x == 0) atomicMax(&stat[0], n0);
+    // every entry's place by counting: the keys differ, so it is the same in
+    // every run whatever order the entries came in
+    for (int h = 0; h < 2; ++h) {
+        const int n = h == 0 ? n0 : n1;
+        const long long base = a0 + (h == 0 ? 0 : n0);
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            int rank = 0;
+            for (int j = 0; j < n; ++j) rank += key[h][j] < key[h][i];
+            list[base + rank] = make_int2(id[h][i], key[h][i] % f);
+        }
+        for (int j = threadIdx.x; j <= m; j += blockDim.x) {
+            int before = 0;
+            for (int i = 0; i < n; ++i) before += key[h][i] / f < S + j;
+            (h == 0 ? ptr12 : ptr21)[uoff[q] + q + j] = base + before;
+        }
+    }
+}
+
+struct LeafMaps {
+    const int *S, *f, *voff, *uoff, *vars, *csr, *row;
+    const long long *foff, *aoff, *pos, *ptr12, *ptr21;
+    const int2 *list;
+};
+
+// Leading dimension of a leaf's pivot block in shared memory: 2 modulo 16, so
+// that a fragment read takes two wavefronts, the least for 256 bytes.
+__host__ __device__ inline int leaf_ld(int S) { return (S + 13) / 16 * 16 + 2; }
+inline size_t leaf_smem(int maxS, int maxf, int maxe, int gwarps)
+{
+    const int rows = (maxS + 7) / 8 * 8;
+    return ((size_t)rows * leaf_ld(rows) + gwarps * (size_t)rows + maxe) * sizeof(double) +
+           (size_t)(maxf + 1) * sizeof(int) + (size_t)maxe * sizeof(short);
+}
+
+// sum of x[c] v over a list's entries, four loads in flight
+__device__ __forceinline__ double sparse_dot(const double *x, const short *c, const double *v,
+                                             int b, int e)
+{
+    double s0 = 0.0, s1 = 0.0;
+    for (; b < e; b += 4) {
+        int k[4];
+        double a[4], y[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            k[u] = b + u < e ? c[b + u] : 0;
+            a[u] = b + u < e ? v[b + u] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) y[u] = b + u < e ? x[k[u]] : 0.0;
+        s0 += y[0] * a[0] + y[2] * a[2];
+        s1 += y[1] * a[1] + y[3] * a[3];
+    }
+    return s0 + s1;
+}
+
+// One CTA per leaf.  A11 in shared memory is inverted in FP64 by Gauss-Jordan
+// blocks of 32 (invert32 by four warps, the products by all eight on the FP64
+// tensor cores, a block row of eight rows per warp); then the sparse sums, one
+// front row per warp.  maxrows, maxf, maxe: the level's largest pivot count
+// (rounded up to 8), front and number of A12 entries; gwarps: the warps that have
+// room for a row of G (fewer than eight where that lets two CTAs share an SM).
+template <class T>
+__global__ void __launch_bounds__(256, 2) k_leaf(const LeafMaps L, int maxrows, int maxf, int maxe,
+                                                 int gwarps,
+                                                 const double *__restrict__ val,
+                                                 const double *__restrict__ rs, T *F, int *flag)
+{
+    extern __shared__ __align__(16) unsigned char leaf_raw[];
+    __shared__ double col[2][kPanel][kHalf];
+    __shared__ int piv[kHalf];
+    const int q = blockIdx.x, S = L.S[q], f = L.f[q], vo = L.voff[q], m = f - S;
+    const int n8 = (S + 7) / 8, ld = leaf_ld(8 * n8);
+    double *M = reinterpret_cast<double *>(leaf_raw);
+    double *grow = M + (size_t)maxrows * leaf_ld(maxrows);   // a row of G per warp
+    double *ev = grow + gwarps * (size_t)maxrows;
+    int *p12 = reinterpret_cast<int *>(ev + maxe);           // column j's entries [p12[j], p12[j+1])
+    short *ec = reinterpret_cast<short *>(p12 + maxf + 1);   // an entry's pivot
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const long long a0 = L.aoff[q], a1 = L.aoff[q + 1], u0 = L.uoff[q] + q;
+    for (int i = tid; i < 8 * n8 * ld; i += 256) M[i] = 0.0;
+    // the A12 values (row scaled), in list order
+    const long long e12 = L.ptr12[u0], e21 = L.ptr21[u0];
+    for (int j = tid; j <= m; j += 256) p12[j] = (int)(L.ptr12[u0 + j] - e12);
+    for (long long e = e12 + tid; e < e21; e += 256) {
+        const int2 x = L.list[e];
+        ev[e - e12] = val[x.x] * rs[L.vars[vo + x.y]];
+        ec[e - e12] = (short)x.y;
+    }
+    __syncthreads();
+    const long long fo = L.foff[q];
+    for (long long e = a0 + tid; e < a1; e += 256) {
+        const int p = (int)(L.pos[e] - fo), r = p / f, c = p - r * f;
+        if (r < S && c < S) M[r * ld + c] = val[L.csr[e]] * rs[L.row[e]];
+    }
+    __syncthreads();
+    bool bad = false;
+#pragma unroll 1
+    for (int k = 0; k < S; k += kHalf) {
+        const int w = min(kHalf, S - k), b0 = k / 8, b1 = b0 + (w + 7) / 8;   // its 8-blocks
+        if (tid < kInvThreads) bad |= invert32(M + k * ld + k, ld, w, col, piv);
+        __syncthreads();
+        // R = X A_KJ, a warp's 8-column blocks (two at most), in place
+        double r[2][4][2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int nb = wid + 8 * u;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[u][i][0] = r[u][i][1] = 0.0;
+            if (nb >= n8 || (nb >= b0 && nb < b1)) continue;
+#pragma unroll 2
+            for (int k4 = 0; k4 < w; k4 += 4) {
+                const double b = M[(k + k4 + t) * ld + 8 * nb + g];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (8 * i < w)
+                        dmma_8x8x4(r[u][i][0], r[u][i][1], M[(k + 8 * i + g) * ld + k + k4 + t], b);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int nb = wid + 8 * u;
+            if (nb >= n8 || (nb >= b0 && nb < b1)) continue;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (8 * i < w)
+                    *reinterpret_cast<double2 *>(&M[(k + 8 * i + g) * ld + 8 * nb + 2 * t]) =
+                        make_double2(r[u][i][0], r[u][i][1]);
+        }
+        __syncthreads();
+        // the other rows: A_IJ -= A_IK R, then A_IK = -A_IK X
+        for (int mb = wid; mb < n8; mb += 8) {
+            if (mb >= b0 && mb < b1) continue;
+            double a[kHalf / 4];
+#pragma unroll
+            for (int k4 = 0; k4 < kHalf / 4; ++k4)
+                a[k4] = 4 * k4 < w ? M[(8 * mb + g) * ld + k + 4 * k4 + t] : 0.0;
+            __syncwarp();   // the row's A_IK is in registers
+#pragma unroll 1
+            for (int nb = 0; nb < n8; nb += 4) {
+                double acc[4][2];
+                double *d = &M[(8 * mb + g) * ld + 8 * nb + 2 * t];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const bool old = nb + u < n8 && !(nb + u >= b0 && nb + u < b1);
+                    acc[u][0] = old ? -d[8 * u] : 0.0;
+                    acc[u][1] = old ? -d[8 * u + 1] : 0.0;
+                }
+#pragma unroll
+                for (int k4 = 0; k4 < kHalf / 4; ++k4)
+                    if (4 * k4 < w) {
+                        const double *b = &M[(k + 4 * k4 + t) * ld + 8 * nb + g];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (nb + u < n8) dmma_8x8x4(acc[u][0], acc[u][1], a[k4], b[8 * u]);
+                    }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (nb + u < n8)
+                        *reinterpret_cast<double2 *>(d + 8 * u) = make_double2(-acc[u][0], -acc[u][1]);
+            }
+        }
+        __syncthreads();
+    }
+    if (bad && tid == 0) atomicOr(flag, 1);
+    T *A = F + fo;
+    // A11^-1 and H, a front row per warp
+    for (int i = wid; i < S; i += 8) {
+        const double *x = M + i * ld;
+        T *d = A + (long long)i * f;
+        for (int c = lane; c < S; c += 32) d[c] = (T)x[c];
+        for (int j = lane; j < m; j += 32) d[S + j] = (T)sparse_dot(x, ec, ev, p12[j], p12[j + 1]);
+    }
+    // -G and -G A12: a row of A21 has few entries, the same for the whole warp
+    if (wid >= gwarps) return;
+    double *gr = grow + (size_t)wid * maxrows;
+    for (int i = wid; i < m; i += gwarps) {
+        T *d = A + (long long)(S + i) * f;
+        const long long e0 = L.ptr21[u0 + i], e1 = L.ptr21[u0 + i + 1];
+        const double s = rs[L.vars[vo + S + i]];
+        double v[kLeafMaxS / 32] = {};
+        for (long long e = e0; e < e1; ++e) {
+            const int2 x = L.list[e];
+            const double a = val[x.x] * s;
+#pragma unroll
+            for (int u = 0; u < kLeafMaxS / 32; ++u)
+                if (lane + 32 * u < S) v[u] -= a * M[x.y * ld + lane + 32 * u];
+        }
+#pragma unroll
+        for (int u = 0; u < kLeafMaxS / 32; ++u)
+            if (lane + 32 * u < S) {
+                gr[lane + 32 * u] = v[u];
+                d[lane + 32 * u] = (T)v[u];
+            }
+        __syncwarp();
+        for (int j = lane; j < m; j += 32) d[S + j] = (T)sparse_dot(gr, ec, ev, p12[j], p12[j + 1]);
+        __syncwarp();
+    }
 }
 
 // FP64 factors rounded to FP32 (the solve of the mixed form with FP64

@@ -101,7 +101,7 @@ struct MfPlan {
     std::vector<int> S, f, voff, uoff, child0, child1, parent;
     std::vector<long long> foff;
     std::vector<int> lvl_off, lvl_maxS, lvl_maxf;
-    std::vector<long long> lvl_abeg, lvl_aend;   // assembly entries of each level (forest plans)
+    std::vector<long long> lvl_abeg, lvl_aend;   // assembly entries of each level
     int *d_S = nullptr, *d_f = nullptr, *d_voff = nullptr, *d_uoff = nullptr;
     int *d_child0 = nullptr, *d_child1 = nullptr, *d_parent = nullptr;
     long long *d_foff = nullptr;
@@ -109,6 +109,11 @@ struct MfPlan {
     int *d_inv0 = nullptr, *d_inv1 = nullptr;
     int *d_vars = nullptr, *d_cbmap = nullptr, *d_asm_csr = nullptr, *d_asm_row = nullptr;
     long long *d_asm_pos = nullptr;
+    // the leaves' entry lists (k_leaf); leaf_smem 0: they are eliminated like other fronts
+    long long *d_leaf_off = nullptr, *d_leaf12 = nullptr, *d_leaf21 = nullptr;
+    int2 *d_leaf_list = nullptr;
+    int leaf_entries = 0, leaf_warps = 0;
+    size_t leaf_smem = 0;
     // work items of the solve (12 ints each: kind, front, rows [beg, end),
     // two (counter, target) waits, two done counters), forward items level by
     // level bottom-up, then backward items top-down; the items of level L's
@@ -244,8 +249,8 @@ int mf_time_apply_launches(const MfPlan *P, const MfFactor *M, int reps, size_t 
                            cudaStream_t s, double *ms, int *codes, int cap, int *n);
 // Per-kernel device time of one factorization launched directly (not from
 // its graph), average of reps; codes kind * 1000 + level (kinds 0 rowscale,
-// 1 scatter, 2 assembly with the first pivot inverse, 4 row block, 6 update,
-// 11 rounding to FP32).  The factors are recomputed from the same values.
+// 1 scatter, 2 assembly with the first pivot inverse, 3 leaves, 4 row block,
+// 6 update, 11 rounding to FP32).  The factors are recomputed from the same values.
 int mf_time_factor_launches(const MfPlan *P, MfFactor *M, const int *rowptr, const double *val,
                             int reps, cudaStream_t s, double *ms, int *codes, int cap, int *n);
 

@@ -198,7 +198,8 @@ void mf_plan_destroy(MfPlan *p)
     if (!p) return;
     void *ptrs[] = {p->d_S, p->d_f, p->d_voff, p->d_uoff, p->d_child0, p->d_child1, p->d_parent,
                     p->d_foff, p->d_vars, p->d_cbmap, p->d_inv0, p->d_inv1, p->d_asm_csr,
-                    p->d_asm_row, p->d_asm_pos, p->d_items};
+                    p->d_asm_row, p->d_asm_pos, p->d_items, p->d_leaf_off, p->d_leaf12,
+                    p->d_leaf21, p->d_leaf_list};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     delete p;
@@ -691,6 +692,50 @@ static int invert_cbmap(MfPlan *P)
     return V2D_OK;
 }
 
+// The leaves' entry lists (k_leaf_lists) from the uploaded arrays; leaf_smem
+// stays 0, and the leaves are eliminated like other fronts, when one of them is
+// too wide or has too many entries for the leaf kernel.
+static int leaf_setup(MfPlan *P)
+{
+    const int nq = P->lvl_off[1], maxS = P->lvl_maxS[0];
+    if (maxS > kLeafMaxS) return V2D_OK;
+    const long long ne = P->lvl_aend[0];
+    std::vector<long long> off(nq + 1, 0);
+    int q = 0;
+    for (long long e = 0; e < ne; ++e) {
+        while (q + 1 < nq && P->h_asm_pos[e] >= P->foff[q + 1]) off[++q] = e;
+    }
+    while (q < nq) off[++q] = ne;
+    const size_t np = (size_t)(nq < P->nfront ? P->uoff[nq] : P->utotal) + nq + 1;
+    int *stat = nullptr, h[2] = {0, 0};
+    V2D_TRY(upload_vec(&P->d_leaf_off, off));
+    V2D_CUDA_TRY(cudaMalloc((void **)&P->d_leaf12, np * sizeof(long long)));
+    V2D_CUDA_TRY(cudaMalloc((void **)&P->d_leaf21, np * sizeof(long long)));
+    V2D_CUDA_TRY(cudaMalloc((void **)&P->d_leaf_list, std::max<size_t>(1, ne) * sizeof(int2)));
+    V2D_CUDA_TRY(cudaMalloc((void **)&stat, sizeof(h)));
+    cudaError_t e = cudaMemset(stat, 0, sizeof(h));
+    if (e == cudaSuccess) {
+        k_leaf_lists<<<nq, 256>>>(P->d_S, P->d_f, P->d_foff, P->d_uoff, P->d_leaf_off, P->d_asm_csr,
+                                  P->d_asm_pos, P->d_leaf_list, P->d_leaf12, P->d_leaf21, stat);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(h, stat, sizeof(h), cudaMemcpyDeviceToHost);
+    cudaFree(stat);
+    V2D_CUDA_TRY(e);
+    // eight warps for the G rows, or fewer if then two CTAs fit on an SM
+    constexpr size_t kPair = 228 * 1024 / 2 - 1024 - 2304;   // a CTA's half, less its static arrays
+    int gw = 8;
+    while (gw > 4 && leaf_smem(maxS, P->lvl_maxf[0], h[0], gw) > kPair) --gw;
+    if (leaf_smem(maxS, P->lvl_maxf[0], h[0], gw) > kPair) gw = 8;
+    const size_t bytes = leaf_smem(maxS, P->lvl_maxf[0], h[0], gw);
+    if (h[1] == 0 && bytes <= 220 * 1024) {
+        P->leaf_entries = h[0];
+        P->leaf_warps = gw;
+        P->leaf_smem = bytes;
+    }
+    return V2D_OK;
+}
+
 // The split a device solve starts with: about kItemsDevice items per level --
 // one round of the dataflow solve's CTAs -- of 16 to 256 rows, and whole fronts
 // where they are short and many.  Half the items of the plan's own default:
@@ -731,6 +776,7 @@ static int mf_plan_upload(MfPlan *P)
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_asm_pos, P->h_asm_pos);
     if (st_up == V2D_OK) st_up = upload_vec(&P->d_items, device_items(P));
     if (st_up == V2D_OK) st_up = invert_cbmap(P);
+    if (st_up == V2D_OK) st_up = leaf_setup(P);
     if (st_up != V2D_OK) {
         mf_plan_destroy(P);
         return st_up;
@@ -1227,9 +1273,11 @@ int mf_factor_create(const MfPlan *P, int fp32, int fact64, MfFactor **out)
         attr((const void *)k_tdown_front<double>, tsolve);
     }
     if (esf == sizeof(float)) {
+        attr((const void *)k_leaf<float>, P->leaf_smem);
         attr((const void *)k_row_block<float>, tile_smem_bytes<float>());
         attr((const void *)k_update<float>, tile_smem_bytes<float>());
     } else {
+        attr((const void *)k_leaf<double>, P->leaf_smem);
         attr((const void *)k_row_block<double>, tile_smem_bytes<double>());
         attr((const void *)k_update<double>, tile_smem_bytes<double>());
     }
@@ -1288,7 +1336,7 @@ static int factor_launches(const MfPlan *P, MfFactor *M, const int *rowptr, cons
     const size_t smem = tile_smem_bytes<T>();
     // with ev: an event is recorded after each kernel (kind * 1000 + level;
     // kinds 0 rowscale, 1 scatter, 2 assembly with the first pivot inverse,
-    // 4 row block, 6 update)
+    // 3 leaves, 4 row block, 6 update)
     int nev = 0;
     auto mark = [&](int code) -> int {
         const cudaError_t le = cudaGetLastError();
@@ -1310,14 +1358,32 @@ static int factor_launches(const MfPlan *P, MfFactor *M, const int *rowptr, cons
     k_rowscale<<<grid_for(P->n, 256), 256, 0, s>>>(P->n, rowptr, val, M->rs);
     V2D_TRY(mark(0));
     ++launches;
-    V2D_CUDA_TRY(cudaMemsetAsync(F, 0, (size_t)P->ftotal * sizeof(T), s));
-    k_scatter<T><<<grid_for(P->nasm, 256), 256, 0, s>>>(P->nasm, P->d_asm_csr, P->d_asm_row,
-                                                      P->d_asm_pos, val, M->rs, F);
-    V2D_TRY(mark(1000));
-    ++launches;
+    // the leaves by their own kernel; matrix entries into the other fronts
+    const int first = P->leaf_smem > 0 ? 1 : 0;
+    const long long f0 = first == 0 ? 0 : first < P->nlevel ? P->foff[P->lvl_off[1]] : P->ftotal;
+    const long long e0 = first ? P->lvl_aend[0] : 0, ne = P->nasm - e0;
+    if (f0 < P->ftotal)
+        V2D_CUDA_TRY(cudaMemsetAsync(F + f0, 0, (size_t)(P->ftotal - f0) * sizeof(T), s));
+    if (ne > 0) {
+        constexpr int per_block = 256 * kScatterEntries;
+        k_scatter<T><<<(int)((ne + per_block - 1) / per_block), 256, 0, s>>>(
+            ne, P->d_asm_csr + e0, P->d_asm_row + e0, P->d_asm_pos + e0, val, M->rs, F);
+        V2D_TRY(mark(1000));
+        ++launches;
+    }
+    if (first) {
+        const LeafMaps lm{P->d_S, P->d_f, P->d_voff, P->d_uoff, P->d_vars, P->d_asm_csr,
+                          P->d_asm_row, P->d_foff, P->d_leaf_off, P->d_asm_pos, P->d_leaf12,
+                          P->d_leaf21, P->d_leaf_list};
+        k_leaf<T><<<P->lvl_off[1], 256, P->leaf_smem, s>>>(lm, (P->lvl_maxS[0] + 7) / 8 * 8,
+                                                          P->lvl_maxf[0], P->leaf_entries, P->leaf_warps, val,
+                                                          M->rs, F, M->flag);
+        V2D_TRY(mark(3000));
+        ++launches;
+    }
     const AssemblyMaps maps{P->d_S, P->d_f, P->d_voff, P->d_child0, P->d_child1, P->d_inv0,
                             P->d_inv1, P->d_foff};
-    for (int L = 0; L < P->nlevel; ++L) {
+    for (int L = first; L < P->nlevel; ++L) {
         const int q0 = P->lvl_off[L], nq = P->lvl_off[L + 1] - q0;
         const int maxf = P->lvl_maxf[L], nt = (maxf + kTile - 1) / kTile, v0 = P->voff[q0];
         // the extend-add's blocks of a front: none on the leaves

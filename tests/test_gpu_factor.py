@@ -23,8 +23,8 @@ WIDTHS = [(15, 13), (16, 13), (17, 13), (31, 17), (32, 17), (33, 17), (48, 33), 
           (64, 32), (65, 33), (127, 64), (129, 67)]
 
 
-def one_update(v2d, oracle_mod, imax, jmax, limit, **config):
-    """One Newton update on an imax x jmax grid against SciPy's direct solve."""
+def one_update(v2d, oracle_mod, imax, jmax, limit, tol=1e-9, **config):
+    """One Newton update on an imax x jmax grid against SciPy's direct solve, refined."""
     xg, yg = oracle_mod.generate_cylinder(imax, jmax)
     s = v2d.Solver(v2d.Config(verbose=False, write_csv=False, write_xdmf=False, re=80.0,
                               steady=False, dt_phys=0.2, farfield_bc="outflow", alpha_deg=4.0,
@@ -37,12 +37,14 @@ def one_update(v2d, oracle_mod, imax, jmax, limit, **config):
         imax, jmax, 80.0, 0.0, 2.5, 0.3, 1 / (imax - 1), 1 / (jmax - 1), *M, *st, 0, 2 * N,
         26 * N, 1, np.cos(np.radians(4.0)), np.sin(np.radians(4.0)))
     A = sp.csr_matrix((cv[:nnz], (ci[:nnz], cj[:nnz])), shape=(2 * N, 2 * N))
-    dq = spla.spsolve(A.tocsc(), b)
+    lu = spla.splu(A.tocsc())
+    dq = lu.solve(b)
+    dq += lu.solve(b - A @ dq)   # refined: the direct solve alone is 3e-6 off at 257 x 257
     code, _, lin = s.dev.newton(0.3)
     assert code == 0, v2d._lib.last_error()
     got = np.concatenate(s.dev.get_state()[:2]) - np.concatenate(st[:2])
     s.close()
-    assert np.max(np.abs(got - dq)) <= 1e-9 * max(1.0, np.max(np.abs(dq)))
+    assert np.max(np.abs(got - dq)) <= tol * max(1.0, np.max(np.abs(dq)))
     assert lin.converged and lin.iterations <= limit, lin.iterations
 
 
@@ -70,3 +72,15 @@ def test_leaf_sizes(v2d, oracle_mod, monkeypatch, leaf, imax, jmax, precision, f
 
     monkeypatch.setattr(v2d._lib, "krylov_defaults", with_leaf)
     one_update(v2d, oracle_mod, imax, jmax, limit, precision=precision, lu_factors=factors)
+
+
+# Levels wide enough for the pipelined update (592 tiles of fronts with 64
+# pivots or more): fronts of different sizes with a part step after the full
+# one (78 to 90 pivots), of exactly one step (64), of three full steps and a
+# part (254, 256).  The update's error grows with the condition, here up to
+# eight times the nodes and so at most ten times that of the grids above: 1e-8.
+@pytest.mark.parametrize("imax,jmax", [(181, 181), (193, 161), (513, 33), (257, 257)])
+@pytest.mark.parametrize("precision,factors,limit", [("fp64", "fp32", 3), ("mixed", "fp64", 7)])
+def test_wide_update(v2d, oracle_mod, imax, jmax, precision, factors, limit):
+    one_update(v2d, oracle_mod, imax, jmax, limit, tol=1e-8, precision=precision,
+               lu_factors=factors)

@@ -31,6 +31,7 @@
 
 #include <algorithm>
 
+#include "v2d_async.cuh"
 #include "v2d_internal.cuh"
 
 namespace v2d {
@@ -454,7 +455,25 @@ template <> struct Tile<double> {
         const int wr = (w >> 2) * 32, wc = (w & 3) * 16;
         if (wc >= nc) return;
         nr -= wr;
+        // whole rows without a test between the products, so that the
+        // fragment loads of the next ones are issued ahead
+        if (nr > 24) {
 #pragma unroll
+            for (int k = 0; k < kSlice; k += 4) {
+                double a[4], b[2];
+#pragma unroll
+                for (int ni = 0; ni < 2; ++ni) b[ni] = s.B[k + t][wc + 8 * ni + g];
+#pragma unroll
+                for (int mi = 0; mi < 4; ++mi) a[mi] = s.A[wr + 8 * mi + g][k + t];
+#pragma unroll
+                for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+                    for (int ni = 0; ni < 2; ++ni)
+                        dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], a[mi], b[ni]);
+            }
+            return;
+        }
+#pragma unroll 2
         for (int k = 0; k < kSlice; k += 4) {
             double b[2];
 #pragma unroll
@@ -696,6 +715,183 @@ __global__ void __launch_bounds__(256, 3) k_update(int q0, int k, int nt, int v0
     if (threadIdx.x >= kInvThreads) return;
     invert_block(ps, wn, flag);
     store_block(ps, wn, A + (long long)e * f + e, f);
+}
+
+// The update of a full step (64 pivots in every front) with FP64 fronts and
+// many tiles: one CTA per SM, four producer warps that fetch the next tile's
+// operands and old entries while eight warps multiply the current one.  A CTA
+// takes strips of `len` tiles of a row of tiles from a counter, the next pivot
+// blocks first; a strip's C_I is fetched once.  The FP64 tensor cores bound it
+// (37 TF/s, 2.1 us per tile and SM): 16 fronts of 2562 take 0.53 ms, 24.9 TF/s,
+// against 0.64 ms in k_update, whose reads of the old entries (64 bytes in each
+// of 8 rows per load) hold up the products whether they come early or late.
+// Measured and not taken, on the same fronts: bulk copies per row (0.85 ms),
+// two groups of four warps in turn (0.59), two of eight that read the old
+// entries themselves (0.65), strips with two CTAs per SM (0.76).
+constexpr int kWideWarps = 8, kWideProducers = 128;
+
+struct WideShared {
+    struct Stage {
+        double B[kPiv][kTile + 8], C[kTile][kTile + 8];
+    } st[2];
+    double A[2][kTile][kPiv + 4];
+    unsigned long long full[2], empty[2];
+    struct Work {
+        int q, r0, c0, a;   // front (-1: no more), first row and column, A's buffer
+    } tile[2];
+    int ticket[2];
+};
+static_assert(sizeof(PivotSmem) <= sizeof(WideShared::Stage), "the inversion uses a stage");
+
+__global__ void __launch_bounds__(32 * kWideWarps + kWideProducers, 1)
+    k_update_wide(int q0, int nq, int k, int nt, int len, int v0, const int *__restrict__ S_,
+                  const int *__restrict__ f_, const long long *__restrict__ foff,
+                  const int *__restrict__ voff, double *F, const double *C, int *ticket, int *flag)
+{
+    extern __shared__ __align__(16) unsigned char tile_raw[];
+    WideShared &sh = *reinterpret_cast<WideShared *>(tile_raw);
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&sh.full[s], kWideProducers + 1);
+            mbar_init(&sh.empty[s], kWideWarps);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    const int kt = k / kTile;   // the pivots' tile row and column
+    if (wid >= kWideWarps) {
+        const int ns = (nt + len - 1) / len, p = threadIdx.x - 32 * kWideWarps;
+        const long long total = nq + (long long)nq * nt * ns;
+        int n = 0, a = 0;
+        // the stage of the next tile once it is free; false: given up
+        auto stage = [&](int q, int r0, int c0) {
+            const int s = n & 1;
+            if (n >= 2 && !mbar_wait(&sh.empty[s], ((n >> 1) - 1) & 1, nullptr)) {
+                atomicOr(flag, 1);
+                return false;
+            }
+            if (p == 0) {
+                sh.tile[s] = {q, r0, c0, a};
+                mbar_arrive(&sh.full[s]);
+            }
+            return true;
+        };
+        int next = p == 0 ? atomicAdd(ticket, 1) : 0;
+        for (int i = 0;; ++i) {
+            if (p == 0) sh.ticket[i & 1] = next;
+            asm volatile("bar.sync 3, %0;" ::"n"(kWideProducers) : "memory");
+            const int t = sh.ticket[i & 1];
+            if (t >= total) break;
+            if (p == 0) next = atomicAdd(ticket, 1);
+            const bool pivots = t < nq;
+            const int u = t - nq, q = q0 + (pivots ? t : u / (nt * ns));
+            const int S = S_[q], f = f_[q], rt = pivots ? kt + 1 : u / ns % nt;
+            const int r0 = rt * kTile, nr = min(kTile, f - r0);
+            if (nr <= 0 || rt == kt || (pivots && k + kPiv >= S)) continue;
+            const double *A = F + foff[q], *R = A + (long long)k * f;
+            const double *Ci = C + ((long long)(voff[q] - v0) + r0) * kPiv;
+            const int j0 = pivots ? rt : u % ns * len, j1 = pivots ? rt + 1 : min(nt, j0 + len);
+            const int pr = p / (kTile / 2), pc = 2 * (p % (kTile / 2));   // its rows, columns
+            constexpr int step = kWideProducers / (kTile / 2);
+            bool first = true;
+            for (int j = j0; j < j1; ++j) {
+                const int c0 = j * kTile, nc = min(kTile, f - c0);
+                if (nc <= 0 || (!pivots && rt == kt + 1 && j == rt && k + kPiv < S)) continue;
+                if (!stage(q, r0, c0)) return;
+                WideShared::Stage &st = sh.st[n & 1];
+                if (first)
+#pragma unroll 4
+                    for (int r = pr; r < nr; r += step)
+                        cp_async<16>(&sh.A[a][r][pc], Ci + r * kPiv + pc, true);
+                if (pc < nc) {
+#pragma unroll 4
+                    for (int r = pr; r < kPiv; r += step)
+                        cp_async<16>(&st.B[r][pc], R + (long long)r * f + c0 + pc, true);
+                    if (j != kt)   // the pivot columns are overwritten
+#pragma unroll 4
+                        for (int r = pr; r < nr; r += step)
+                            cp_async<16>(&st.C[r][pc], A + (long long)(r0 + r) * f + c0 + pc, true);
+                }
+                mbar_arrive_copies(&sh.full[n & 1]);
+                first = false;
+                ++n;
+            }
+            if (!first) a ^= 1;   // the other buffer's strip is done two tiles on
+        }
+        if (stage(-1, 0, 0)) mbar_arrive(&sh.full[n & 1]);
+        return;
+    }
+    const int g = lane >> 2, t = lane & 3, wr = (wid >> 2) * 32, wc = (wid & 3) * 16;
+    for (int n = 0;; ++n) {
+        const int s = n & 1;
+        if (!mbar_wait(&sh.full[s], (n >> 1) & 1, nullptr)) {
+            atomicOr(flag, 1);
+            return;
+        }
+        const WideShared::Work w = sh.tile[s];
+        if (w.q < 0) return;
+        WideShared::Stage &st = sh.st[s];
+        const int S = S_[w.q], f = f_[w.q], r0 = w.r0 + wr + g, c0 = w.c0 + wc + 2 * t;
+        double *A = F + foff[w.q];
+        const bool old = w.c0 != k, pivots = w.r0 == k + kPiv && w.c0 == w.r0 && w.r0 < S;
+        double acc[4][2][2];
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < 2; ++ni) {
+                double2 v = *reinterpret_cast<const double2 *>(
+                    &st.C[wr + 8 * mi + g][wc + 8 * ni + 2 * t]);
+                if (!old) v = make_double2(0.0, 0.0);
+                acc[mi][ni][0] = -v.x;
+                acc[mi][ni][1] = -v.y;
+            }
+        if (w.r0 + wr < f && w.c0 + wc < f) {
+            const double(*sa)[kPiv + 4] = sh.A[w.a];
+#pragma unroll 8
+            for (int kk = 0; kk < kPiv; kk += 4) {
+                double a[4], b[2];
+#pragma unroll
+                for (int ni = 0; ni < 2; ++ni) b[ni] = st.B[kk + t][wc + 8 * ni + g];
+#pragma unroll
+                for (int mi = 0; mi < 4; ++mi) a[mi] = sa[wr + 8 * mi + g][kk + t];
+#pragma unroll
+                for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+                    for (int ni = 0; ni < 2; ++ni)
+                        dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], a[mi], b[ni]);
+            }
+        }
+        __syncwarp();
+        if (!pivots && lane == 0) mbar_arrive(&sh.empty[s]);
+        const int wn = pivots ? min(kPiv, S - w.r0) : 0;   // the next block's pivots
+        PivotSmem &ps = *reinterpret_cast<PivotSmem *>(&st);
+        if (pivots) asm volatile("bar.sync 2, %0;" ::"n"(32 * kWideWarps) : "memory");
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < 2; ++ni) {
+                const int r = r0 + 8 * mi, c = c0 + 8 * ni, rr = r - w.r0, cc = c - w.c0;
+                const bool in = rr < wn && cc < wn;
+                if (pivots) {
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+                        ps.M[rr * kLdX + cc + u] =
+                            in ? -acc[mi][ni][u] : (rr == cc + u ? 1.0 : 0.0);
+                }
+                if (!in && r < f && c < f)
+                    *reinterpret_cast<double2 *>(A + (long long)r * f + c) =
+                        make_double2(-acc[mi][ni][0], -acc[mi][ni][1]);
+            }
+        if (!pivots) continue;
+        asm volatile("bar.sync 2, %0;" ::"n"(32 * kWideWarps) : "memory");
+        if (threadIdx.x < kInvThreads) {
+            invert_block(ps, wn, flag);
+            store_block(ps, wn, A + (long long)w.r0 * f + w.r0, f);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.empty[s]);
+    }
 }
 
 // ------------------------------------------------------------------ leaves

@@ -169,7 +169,8 @@ struct MfFactor {
     void *cols = nullptr;       // one elimination step's pivot columns of a level's fronts
     void *wb = nullptr;         // transposed solve: per-front adjoint right-hand sides (vtotal)
     double *rs = nullptr;       // row scaling 1 / max |a_r.|
-    int *flag = nullptr;
+    int *flag = nullptr;        // singular pivot block; then a tile counter per elimination step
+    int steps = 0;
     MfBarrier *bar = nullptr;
     void *msg = nullptr;        // dataflow solve: the tickets, upd and z in one allocation
     size_t msg_bytes = 0;

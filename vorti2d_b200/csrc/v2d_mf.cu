@@ -285,7 +285,8 @@ static int items_build(MfPlan *P)
     for (int L = nl - 1; L >= 0; --L) {
         P->lvl_bwd[L + 1] = (int)it.size() / 12;
         cur_level = L;
-        const int R = per(L);
+        const int R = (int)P->item_rows_b.size() == nl && P->item_rows[L] > 0 ? P->item_rows_b[L]
+                                                                              : per(L);
         for (int q = P->lvl_off[L]; q < P->lvl_off[L + 1]; ++q)
             if (gath_b(L, q)) {
                 push(3, q, 0, P->S[q], 1);
@@ -740,18 +741,31 @@ static int leaf_setup(MfPlan *P)
 // one round of the dataflow solve's CTAs -- of 16 to 256 rows, and whole fronts
 // where they are short and many.  Half the items of the plan's own default:
 // an item's cost is its gather and its hand-over rather than its rows (181 x
-// 181, FP32: 0.113 ms with this split, 0.138 ms with the plan's).
+// 181, FP32: 0.113 ms with this split, 0.138 ms with the plan's).  From 1024
+// columns on the rows are the larger part: 8 rows at least, twice the forward
+// items (half of them only hand z on).  Backward items are counted by the
+// level's pivots, not its variables: with the forward items' rows a level of
+// four fronts of 2048 kept 64 of 296 CTAs busy (FP64: 513 x 513 0.66 ms so,
+// 0.58 with the backward count, 0.54 with both; 1025 x 1025 2.45, 2.01, 1.95).
 static void device_item_rows(MfPlan *P)
 {
-    constexpr int kItemsDevice = 300, kWholeFronts = 64, kWholeMaxF = 256;
+    constexpr int kItemsDevice = 300, kWholeFronts = 64, kWholeMaxF = 256, kLongRows = 1024;
+    P->item_rows.assign(P->nlevel, 0);
+    P->item_rows_b.assign(P->nlevel, 0);
     for (int L = 0; L < P->nlevel; ++L) {
-        const int nq = P->lvl_off[L + 1] - P->lvl_off[L];
-        long long rows = 0;
-        for (int q = P->lvl_off[L]; q < P->lvl_off[L + 1]; ++q) rows += P->f[q];
-        int R = 16;
-        while (R < 256 && 2LL * R * kItemsDevice <= rows) R *= 2;
-        const bool whole = P->lvl_maxf[L] <= R || (nq >= kWholeFronts && P->lvl_maxf[L] <= kWholeMaxF);
+        const int nq = P->lvl_off[L + 1] - P->lvl_off[L], maxf = P->lvl_maxf[L];
+        const bool wide = maxf >= kLongRows;
+        long long rows = 0, pivots = 0;
+        for (int q = P->lvl_off[L]; q < P->lvl_off[L + 1]; ++q) {
+            rows += P->f[q];
+            pivots += P->S[q];
+        }
+        int R = wide ? 8 : 16, Rb = R;
+        while (R < 256 && (wide ? 4LL : 2LL) * R * kItemsDevice <= rows) R *= 2;
+        while (Rb < R && 2LL * Rb * kItemsDevice <= pivots) Rb *= 2;
+        const bool whole = maxf <= R || (nq >= kWholeFronts && maxf <= kWholeMaxF);
         P->item_rows[L] = whole ? 0 : R;
+        P->item_rows_b[L] = Rb;
     }
 }
 
@@ -814,10 +828,15 @@ int mf_plan_set_item_rows(MfPlan *P, const int *rows, int nlevels)
     for (int L = 0; L < nlevels; ++L)
         V2D_ARG_CHECK(rows[L] >= -4096 && rows[L] <= 4096, "lu item rows: level %d: %d", L,
                       rows[L]);
-    std::vector<int> keep = P->item_rows;
-    P->item_rows.assign(rows, rows + nlevels);
+    const std::vector<int> keep = P->item_rows, keep_b = P->item_rows_b;
+    device_item_rows(P);   // the rows of the default split mean that split
+    if (!std::equal(rows, rows + nlevels, P->item_rows.begin())) {
+        P->item_rows.assign(rows, rows + nlevels);
+        P->item_rows_b.clear();
+    }
     if (items_build(P) != V2D_OK) {
         P->item_rows = keep;
+        P->item_rows_b = keep_b;
         items_build(P);
         return V2D_EARG;
     }

@@ -236,6 +236,8 @@ int mf_flag(const MfFactor *M, int *flag, cudaStream_t s);
 // V2D_ETIMEOUT (and a reset error state) if a dependency wait of the
 // dataflow solve timed out since the last check.
 int mf_check_barrier(MfFactor *M, cudaStream_t s);
+// The device word behind it.
+const int *mf_error_word(const MfFactor *M);
 // Average device time (ms) of `reps` LU applies to a zero vector, each after a
 // write of flush_bytes (evicts L2); CUDA events on stream s.
 int mf_time_apply(const MfPlan *P, const MfFactor *M, int reps, size_t flush_bytes, cudaStream_t s,
@@ -280,9 +282,16 @@ struct KrylovWork;  // defined in v2d_krylov.cu
 
 int krylov_create(KrylovWork **out, int n, int restart, cudaStream_t s);
 void krylov_destroy(KrylovWork *w);
+// Work enqueued behind each end of a restart cycle, before the host waits for
+// it: it runs to effect once *ok (a device word) says that the solve converged.
+struct KrylovTail {
+    int (*enqueue)(void *self, const int *ok, cudaStream_t s);
+    void *self;
+};
 // Solves A x = b (x is overwritten, starting from zero).  d_b, d_x device.
 int krylov_solve(KrylovWork *w, const CsrOp &A, const double *d_b, double *d_x,
-                 const v2d_krylov_params &prm, v2d_lin_stats *st, cudaStream_t s);
+                 const v2d_krylov_params &prm, v2d_lin_stats *st, cudaStream_t s,
+                 const KrylovTail *tail = nullptr);
 
 int time_spmv(const CsrOp &A, bool fp32, int reps, size_t flush_bytes, cudaStream_t s,
               double *ms_avg);

@@ -46,6 +46,7 @@ struct Ctl {
     double tol_abs;      // convergence target for the true residual
     double inner_rtol;   // FP32 cycles: relative tolerance per cycle
     double res0;
+    double atol;         // absolute floor of tol_abs
     int conv;            // converged: every kernel exits
     int cyc_stop;        // the current cycle's Arnoldi loop ended
     int jdone;           // Arnoldi columns completed in this cycle
@@ -54,6 +55,7 @@ struct Ctl {
     int breakdown;
     int cycles;
     int nonfinite;
+    int ok;              // conv, and the true residual reached its target (or stagnated near it)
     int stagnated;       // a cycle failed to halve the residual near the target
     double prev_beta;
     unsigned int cnt[4]; // last-block counters
@@ -390,9 +392,11 @@ __global__ void __launch_bounds__(kRedThreads) k_update(const Desc *d, Ctl *ctl,
 }
 
 // End of a cycle: back-substitution R y = g over the completed columns.
-__global__ void k_backsolve(const Desc *d, Ctl *ctl, const double *H, const double *g, double *y)
+// (guard: only if the cycle's last step has stopped it; here and in the next two)
+__global__ void k_backsolve(const Desc *d, Ctl *ctl, const double *H, const double *g, double *y,
+                            int guard)
 {
-    if (ctl->conv) return;
+    if (ctl->conv || (guard && !ctl->cyc_stop)) return;
     if (threadIdx.x != 0) return;
     const int m = d->m, jj = ctl->jdone;
     for (int i = jj - 1; i >= 0; --i) {
@@ -406,9 +410,9 @@ __global__ void k_backsolve(const Desc *d, Ctl *ctl, const double *H, const doub
 // x += M^-1 (V y), x in FP64.
 template <class T>
 __global__ void __launch_bounds__(256) k_correct(const Desc *d, Ctl *ctl, const T *V, const double *y,
-                                                 T *t_scratch, double *x, const T *Z)
+                                                 T *t_scratch, double *x, const T *Z, int guard)
 {
-    if (ctl->conv) return;
+    if (ctl->conv || (guard && !ctl->cyc_stop)) return;
     const int n = d->n, jj = ctl->jdone;
     if (d->precond == V2D_PC_LU) {   // x += Z y
         V2D_GRID_STRIDE(r, n)
@@ -461,9 +465,10 @@ __global__ void __launch_bounds__(256) k_correct(const Desc *d, Ctl *ctl, const 
 // FP64 true residual r = b - A x and its norm; the last block decides
 // convergence and resets the cycle state.
 __global__ void __launch_bounds__(kSpmvThreads) k_residual(const Desc *d, Ctl *ctl, double *r,
-                                                           double *partial, double *g, int first)
+                                                           double *partial, double *g, int first,
+                                                           int guard)
 {
-    if (ctl->conv) return;
+    if (ctl->conv || (guard && !ctl->cyc_stop)) return;
     __shared__ double red[32];
     const int n = d->n, m = d->m;
     const int lane = threadIdx.x & (kTPR - 1);
@@ -496,9 +501,11 @@ __global__ void __launch_bounds__(kSpmvThreads) k_residual(const Desc *d, Ctl *c
         if (threadIdx.x == 0) {
             double beta = sqrt(s);
             ctl->beta = beta;
+            double tc = ctl->tol_abs;
             if (first) {
                 ctl->res0 = beta;
-                ctl->tol_abs = ctl->tol_abs * beta;  // rtol * ||b||
+                tc *= beta;  // rtol * ||b||; the first cycle aims at that also under an atol
+                ctl->tol_abs = fmax(tc, ctl->atol);
             }
             ctl->resid = beta;
             ctl->cycles += first ? 0 : 1;
@@ -514,18 +521,28 @@ __global__ void __launch_bounds__(kSpmvThreads) k_residual(const Desc *d, Ctl *c
             } else if (ctl->its >= ctl->max_it || ctl->breakdown) {
                 ctl->conv = 1;  // stop: not converged (host reads beta)
             }
+            ctl->ok = ctl->conv && !ctl->nonfinite && (beta <= ctl->tol_abs || ctl->stagnated);
             ctl->prev_beta = beta;
             // next cycle
             g[0] = beta;
             for (int i = 1; i <= m; ++i) g[i] = 0.0;
             ctl->jdone = 0;
             ctl->cyc_stop = 0;
-            double tc = ctl->tol_abs;
             if (ctl->inner_rtol > 0.0) tc = fmax(tc, ctl->inner_rtol * beta);
             ctl->tol_cycle = tc;
             ctl->cnt[2] = 0;
         }
     }
+}
+
+// The solve's operator and control block, and x = 0, in one launch.
+__global__ void k_begin(Desc hd, Ctl c, Desc *d, Ctl *ctl)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *d = hd;
+        *ctl = c;
+    }
+    V2D_GRID_STRIDE(t, hd.n) { hd.x[t] = 0.0; }
 }
 
 // ------------------------------------------------------------------ host
@@ -566,7 +583,8 @@ static int tile_grid(long long n)
 static std::vector<int> segment_bounds(int m)
 {
     std::vector<int> b{0};
-    const int len[] = {2, 4, 4, 4};
+    // one step first: with fresh FP64 factors it is the only one
+    const int len[] = {1, 3, 4, 4};
     for (int q = 0; b.back() < m; ++q)
         b.push_back(std::min(m, b.back() + (q < 4 ? len[q] : 8)));
     return b;
@@ -637,6 +655,12 @@ static int capture_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, doub
     drop_graphs(w, which);
     w->seg_launches[which].clear();
     const std::vector<int> bnd = segment_bounds(w->m);
+    auto finish = [&](int guard) {
+        k_backsolve<<<1, 32, 0, s>>>(w->desc, w->ctl, w->H, w->g, w->y, guard);
+        k_correct<T><<<gp, 256, 0, s>>>(w->desc, w->ctl, V, w->y, z, x, Z, guard);
+        k_residual<<<res_grid(n), kSpmvThreads, 0, s>>>(w->desc, w->ctl, w->r, w->partial, w->g, 0,
+                                                        guard);
+    };
     for (size_t q = 0; q + 1 < bnd.size(); ++q) {
         long long nl = 0;
         V2D_CUDA_TRY(cudaGetLastError());
@@ -674,15 +698,17 @@ static int capture_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, doub
                 if (capture_launch_failed(s, "k_update", j)) return V2D_ECUDA;
             }
         }
+        if (q == 0) {   // the first step often is the last: its end without a round trip
+            finish(1);
+            nl += 3;
+        }
         cudaGraphExec_t ge = nullptr;
         V2D_TRY(end_capture(s, &ge));
         w->seg[which].push_back(ge);
         w->seg_launches[which].push_back(nl);
     }
     V2D_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    k_backsolve<<<1, 32, 0, s>>>(w->desc, w->ctl, w->H, w->g, w->y);
-    k_correct<T><<<gp, 256, 0, s>>>(w->desc, w->ctl, V, w->y, z, x, Z);
-    k_residual<<<res_grid(n), kSpmvThreads, 0, s>>>(w->desc, w->ctl, w->r, w->partial, w->g, 0);
+    finish(0);
     V2D_TRY(end_capture(s, &w->fin[which]));
     w->seg_bounds[which] = bnd;
     w->graph_m[which] = w->m;
@@ -697,7 +723,7 @@ static int capture_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, doub
 // One restart cycle; *h receives the control block at its end.
 template <class T>
 static int run_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, double *x, const CsrOp &A,
-                     int precond, cudaStream_t s, Ctl *h)
+                     int precond, cudaStream_t s, Ctl *h, const KrylovTail *tail)
 {
     const bool lu = precond == V2D_PC_LU;
     if (w->seg[which].empty() || !w->fin[which] || w->graph_m[which] != w->m ||
@@ -707,17 +733,26 @@ static int run_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, double *
         w->graph_lu_items[which] != (lu ? A.lu_plan->items_ver : -1) ||
         w->graph_x[which] != x)
         V2D_TRY(capture_cycle<T>(w, which, V, wv, z, Z, x, A, precond, s));
+    auto read = [&](bool end) -> int {
+        if (end && tail) V2D_TRY(tail->enqueue(tail->self, &w->ctl->ok, s));
+        V2D_CUDA_TRY(cudaMemcpyAsync(w->ctl_host, w->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
+        V2D_CUDA_TRY(cudaStreamSynchronize(s));
+        return V2D_OK;
+    };
+    const int cycles = h->cycles;
     for (size_t q = 0; q < w->seg[which].size(); ++q) {
         V2D_CUDA_TRY(cudaGraphLaunch(w->seg[which][q], s));
         count_launches(w->seg_launches[which][q]);
-        V2D_CUDA_TRY(cudaMemcpyAsync(w->ctl_host, w->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
-        V2D_CUDA_TRY(cudaStreamSynchronize(s));
-        if (w->ctl_host->cyc_stop || w->ctl_host->conv) break;
+        V2D_TRY(read(q == 0));
+        if (w->ctl_host->conv || w->ctl_host->cycles != cycles) {   // its end was in segment 0
+            *h = *w->ctl_host;
+            return V2D_OK;
+        }
+        if (w->ctl_host->cyc_stop) break;
     }
     V2D_CUDA_TRY(cudaGraphLaunch(w->fin[which], s));
     count_launches(3);
-    V2D_CUDA_TRY(cudaMemcpyAsync(w->ctl_host, w->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
-    V2D_CUDA_TRY(cudaStreamSynchronize(s));
+    V2D_TRY(read(true));
     *h = *w->ctl_host;
     return V2D_OK;
 }
@@ -787,7 +822,8 @@ static int ensure_basis(KrylovWork *w, bool fp32, bool lu)
 }
 
 int krylov_solve(KrylovWork *w, const CsrOp &A, const double *d_b, double *d_x,
-                 const v2d_krylov_params &prm, v2d_lin_stats *st, cudaStream_t s)
+                 const v2d_krylov_params &prm, v2d_lin_stats *st, cudaStream_t s,
+                 const KrylovTail *tail)
 {
     V2D_ARG_CHECK(A.n == w->n, "krylov_solve: operator size %d != workspace size %d", A.n, w->n);
     V2D_ARG_CHECK(prm.restart == w->m, "krylov_solve: restart changed (%d != %d)", prm.restart, w->m);
@@ -804,36 +840,28 @@ int krylov_solve(KrylovWork *w, const CsrOp &A, const double *d_b, double *d_x,
     hd.dinv = A.dinv; hd.dinv32 = A.dinv32; hd.b = d_b; hd.x = d_x;
     hd.precond = (prm.precond == V2D_PC_BJACOBI || prm.precond == V2D_PC_LU) ? prm.precond
                                                                               : V2D_PC_NONE;
-    V2D_CUDA_TRY(cudaMemcpyAsync(w->desc, &hd, sizeof(Desc), cudaMemcpyHostToDevice, s));
     Ctl c{};
-    c.tol_abs = prm.rtol;  // scaled by ||b|| in the first residual pass (atol applied below)
+    c.tol_abs = prm.rtol;  // scaled by ||b|| in the first residual pass
+    c.atol = prm.atol;
     c.max_it = prm.max_it;
     c.inner_rtol = fp32 ? prm.inner_rtol : 0.0;
-    V2D_CUDA_TRY(cudaMemcpyAsync(w->ctl, &c, sizeof(Ctl), cudaMemcpyHostToDevice, s));
-    V2D_CUDA_TRY(cudaMemsetAsync(d_x, 0, (size_t)A.n * sizeof(double), s));
-    const int gr = red_grid(A.n);
-    k_residual<<<res_grid(A.n), kSpmvThreads, 0, s>>>(w->desc, w->ctl, w->r, w->partial, w->g, 1);
+    k_begin<<<grid_for(A.n, 256), 256, 0, s>>>(hd, c, w->desc, w->ctl);
+    k_residual<<<res_grid(A.n), kSpmvThreads, 0, s>>>(w->desc, w->ctl, w->r, w->partial, w->g, 1, 0);
     V2D_CUDA_TRY(cudaGetLastError());
-    count_launches(1);
-    // atol: tol_abs = max(rtol * ||b||, atol) -- applied on the host after the first pass
-    V2D_CUDA_TRY(cudaMemcpyAsync(w->ctl_host, w->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
-    V2D_CUDA_TRY(cudaStreamSynchronize(s));
-    Ctl h = *w->ctl_host;
-    if (!h.conv && prm.atol > h.tol_abs) {
-        double ta = prm.atol;
-        V2D_CUDA_TRY(cudaMemcpyAsync(&w->ctl->tol_abs, &ta, sizeof(double), cudaMemcpyHostToDevice, s));
-        if (h.beta <= ta) h.conv = 1;
-    }
+    count_launches(2);
+    // the first cycle is launched before the first residual is known here: its
+    // kernels end at once where that has met the tolerance already
+    Ctl h = c;
     int guard = 0;
-    while (!h.conv) {
+    do {
         int status = fp32 ? run_cycle<float>(w, 1, w->V32, w->w32, w->z32, w->Z32, d_x, A,
-                                             hd.precond, s, &h)
+                                             hd.precond, s, &h, tail)
                           : run_cycle<double>(w, 0, w->V64, w->w64, w->z64, w->Z64, d_x, A,
-                                              hd.precond, s, &h);
+                                              hd.precond, s, &h, tail);
         if (status != V2D_OK) return status;
         if (++guard > 1000000) break;
-    }
-    const bool converged = (h.beta <= fmax(h.tol_abs, prm.atol) || h.stagnated) && !h.nonfinite;
+    } while (!h.conv);
+    const bool converged = h.ok != 0;
     if (st) {
         st->iterations = h.its;
         st->restarts = h.cycles;

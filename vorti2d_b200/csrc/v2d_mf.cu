@@ -1793,6 +1793,8 @@ int mf_time_factor_launches(const MfPlan *P, MfFactor *M, const int *rowptr, con
     return V2D_OK;
 }
 
+const int *mf_error_word(const MfFactor *M) { return M->bar ? &M->bar->err : nullptr; }
+
 int mf_check_barrier(MfFactor *M, cudaStream_t s)
 {
     if (!M->bar) return V2D_OK;

@@ -572,21 +572,23 @@ static int tile_grid(long long n)
     return (int)std::max(1LL, std::min<long long>(kTileBlocks, g));
 }
 
-// A restart cycle runs as a few captured segments of Arnoldi steps
-// ([0,2), [2,6), [6,10), [10,14), then 8 at a time), then a finishing graph
-// (back-substitution, correction, FP64 residual).  The host reads the control
-// block after each segment and skips the remaining segments once the cycle
-// has stopped, so a cycle that converges in a few steps (the usual case with
-// the LU preconditioner: 6-12 with factors kept across Newton iterations)
-// launches few steps past its last one; each step after the stop is a chain
-// of launches that return at once.
-static std::vector<int> segment_bounds(int m)
+// A restart cycle runs as a few captured segments of Arnoldi steps (FP64:
+// [0,1), [1,4), FP32: [0,2), [2,6), then 4, 4 and 8 at a time), the first with
+// the cycle's end behind it, then a finishing graph (back-substitution,
+// correction, FP64 residual).  The host reads the control block after each
+// segment and skips the remaining segments once the cycle has stopped, so a
+// cycle that converges in a few steps (the usual case with the LU
+// preconditioner: 6-12 with factors kept across Newton iterations) launches few
+// steps past its last one; each step after the stop is a chain of launches that
+// return at once.  With fresh FP64 factors the first step is the only one (25 x
+// 17: 1.22 ms a pass against 1.27 with two); FP32 cycles need two or more (181 x
+// 181 mixed: 28.1 ms against 29.3 with one).
+static std::vector<int> segment_bounds(int m, bool fp32)
 {
     std::vector<int> b{0};
-    // one step first: with fresh FP64 factors it is the only one
-    const int len[] = {1, 3, 4, 4};
+    const int len[2][4] = {{1, 3, 4, 4}, {2, 4, 4, 4}};
     for (int q = 0; b.back() < m; ++q)
-        b.push_back(std::min(m, b.back() + (q < 4 ? len[q] : 8)));
+        b.push_back(std::min(m, b.back() + (q < 4 ? len[fp32][q] : 8)));
     return b;
 }
 
@@ -654,7 +656,7 @@ static int capture_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, doub
     const bool lu = precond == V2D_PC_LU;
     drop_graphs(w, which);
     w->seg_launches[which].clear();
-    const std::vector<int> bnd = segment_bounds(w->m);
+    const std::vector<int> bnd = segment_bounds(w->m, which == 1);
     auto finish = [&](int guard) {
         k_backsolve<<<1, 32, 0, s>>>(w->desc, w->ctl, w->H, w->g, w->y, guard);
         k_correct<T><<<gp, 256, 0, s>>>(w->desc, w->ctl, V, w->y, z, x, Z, guard);

@@ -74,9 +74,10 @@ __device__ __forceinline__ void plan_chunks(SolveItem &it, int bytes, int nw)
 }
 
 // Values on their way between items carry their own readiness: before a
-// dataflow solve z, upd and x are filled with kUnset, a NaN that no arithmetic
-// produces (results are the canonical NaN), and an item reads an entry again
-// until it is set.  One word is one message, so neither side needs an ordering
+// dataflow solve z, upd and x are filled with 0xff bytes (unset: a NaN that no
+// arithmetic makes), and an item reads an entry again until it is set.  FP64
+// arithmetic may hand on an operand's NaN, so a store replaces this one, which a
+// caller's matrix could hold, by the ordinary NaN (no measurable cost).  One word is one message, so neither side needs an ordering
 // between words: no counter, no release fence after an item's writes (about 0.8
 // us) and no separate poll before its gather (about 0.6 us).
 template <class T> struct Unset;
@@ -109,10 +110,12 @@ __device__ __forceinline__ double ld_relaxed(const double *p)
 
 __device__ __forceinline__ void st_relaxed(float *p, float v)
 {
+    if (Unset<float>::is(v)) v = __int_as_float(0x7fffffff);
     asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
 }
 __device__ __forceinline__ void st_relaxed(double *p, double v)
 {
+    if (Unset<double>::is(v)) v = __longlong_as_double(0x7ff8000000000000LL);
     asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
 

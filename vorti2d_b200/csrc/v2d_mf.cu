@@ -1144,6 +1144,11 @@ __global__ void __launch_bounds__(kSolveThreads) k_tdown_front(int q0, const MfD
 }  // namespace
 
 // ------------------------------------------------------------ host drivers
+// Shared memory of the transposed solve's launches, es bytes per entry: an f
+// and an S vector going up, an f vector going down.
+static size_t tup_smem(const MfPlan *P, size_t es) { return ((size_t)P->maxf + P->maxS) * es; }
+static size_t tdown_smem(const MfPlan *P, size_t es) { return (size_t)P->maxf * es; }
+
 // The dynamic shared memory limit of a kernel (cudaFuncSetAttribute) holds
 // per function and device for the whole process, so every handle shares it:
 // it is only ever raised, to the largest size any handle launches with.
@@ -1277,8 +1282,7 @@ int mf_factor_create(const MfPlan *P, int fp32, int fact64, MfFactor **out)
     auto attr = [&](const void *fn, size_t bytes) {
         if (e == cudaSuccess) e = raise_dyn_smem(fn, bytes);
     };
-    // transposed solve: an f and an S vector (limit kept at two f vectors)
-    const size_t tsolve = (size_t)(P->maxf + P->maxS) * es;
+    // the largest front accepted: two f vectors
     if (2 * P->maxf * es > 227 * 1024) {
         set_error("mf_factor: front of %d unknowns exceeds shared memory (transposed solve)",
                   P->maxf);
@@ -1287,12 +1291,12 @@ int mf_factor_create(const MfPlan *P, int fp32, int fact64, MfFactor **out)
     }
     if (fp32) {
         attr((const void *)k_solve_level<float>, solve);
-        attr((const void *)k_tup_front<float>, tsolve);
-        attr((const void *)k_tdown_front<float>, tsolve);
+        attr((const void *)k_tup_front<float>, tup_smem(P, es));
+        attr((const void *)k_tdown_front<float>, tdown_smem(P, es));
     } else {
         attr((const void *)k_solve_level<double>, solve);
-        attr((const void *)k_tup_front<double>, tsolve);
-        attr((const void *)k_tdown_front<double>, tsolve);
+        attr((const void *)k_tup_front<double>, tup_smem(P, es));
+        attr((const void *)k_tdown_front<double>, tdown_smem(P, es));
     }
     if (esf == sizeof(float)) {
         attr((const void *)k_leaf<float>, P->leaf_smem);
@@ -1605,14 +1609,14 @@ static int apply_transpose_launches(const MfPlan *P, MfFactor *M, const T *g, T 
 {
     const MfDev D = mf_dev(P, M);
     const T *F = (const T *)(M->fact64 ? M->F32 : M->F);
-    const size_t smf = (size_t)2 * P->maxf * sizeof(T);
+    const size_t up = tup_smem(P, sizeof(T)), down = tdown_smem(P, sizeof(T));
     for (int L = 0; L < P->nlevel; ++L) {
         const int q0 = P->lvl_off[L], nq = P->lvl_off[L + 1] - q0;
-        k_tup_front<T><<<nq, kSolveThreads, smf, s>>>(q0, D, F, g, (T *)M->z, (T *)M->upd);
+        k_tup_front<T><<<nq, kSolveThreads, up, s>>>(q0, D, F, g, (T *)M->z, (T *)M->upd);
     }
     for (int L = P->nlevel - 1; L >= 0; --L) {
         const int q0 = P->lvl_off[L], nq = P->lvl_off[L + 1] - q0;
-        k_tdown_front<T><<<nq, kSolveThreads, smf, s>>>(q0, D, F, M->rs, (const T *)M->z,
+        k_tdown_front<T><<<nq, kSolveThreads, down, s>>>(q0, D, F, M->rs, (const T *)M->z,
                                                         (T *)M->wb, lam);
     }
     V2D_CUDA_TRY(cudaGetLastError());

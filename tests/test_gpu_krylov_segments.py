@@ -1,0 +1,54 @@
+"""The captured pieces of a GMRES cycle, by the kernels launched: with kept
+factors the host looks after steps 2, 6, 10, 14, 22 and 30, with the cycle's end
+behind steps 1 and 2; with fresh FP64 factors after step 1 too."""
+import numpy as np
+import pytest
+
+from cases import smooth_state
+
+pytestmark = pytest.mark.gpu
+
+STEP = 7          # scaling, LU solve, product, two passes of projection and update
+BEGIN, END, TAIL = 2, 3, 1   # set-up and first residual; a cycle's end; the Newton update
+
+
+def kept_launches(its, restart=30):
+    bound = next(b for b in (2, 6, 10, 14, 22, 30) if b >= its)
+    ends = 1 if its <= 2 else 2
+    return BEGIN + STEP * bound + END + ends * (END + TAIL)
+
+
+def factorizations(v2d, s):
+    out = np.zeros(6)
+    v2d._lib.check(v2d._lib.lib().v2d_solver_phase_times(s.dev.h, v2d._lib.dptr(out), 0))
+    return int(out[5])
+
+
+def test_launches_with_kept_and_fresh_factors(v2d, oracle_mod):
+    imax, jmax = 65, 49
+    xg, yg = oracle_mod.generate_cylinder(imax, jmax)
+    count = v2d._lib.lib().v2d_launch_count
+    M = oracle_mod.core().compute_metrics(1 / (imax - 1), 1 / (jmax - 1), xg, yg)
+    st = [np.array(a) for a in smooth_state(M[8], M[9])]
+    seen = set()
+    for rtol in (1e-2, 1e-4, 1e-6, 1e-8, 1e-10):
+        s = v2d.Solver(v2d.Config(verbose=False, write_csv=False, write_xdmf=False, re=80.0,
+                                  steady=False, dt_phys=0.2, ksp_restart=30, ksp_rtol=rtol,
+                                  lu_reuse_its=30, lu_reuse_steps=True, precision="fp64"),
+                       mesh=(xg, yg))
+        s.set_state(*st)
+        n0 = count()
+        s.dev.system(urot=0.0)
+        assembly = count() - n0
+        code, _, lin = s.dev.newton(0.0)     # factors this Jacobian; captures the cycle
+        assert code == 0 and lin.iterations == 1
+        for amount in (1e-3, 1e-2, 1e-1):
+            s.set_state(*[a * (1.0 + amount) for a in st])
+            f0, n0 = factorizations(v2d, s), count()
+            code, _, lin = s.dev.newton(0.0)
+            assert code == 0 and lin.converged and factorizations(v2d, s) == f0
+            assert count() - n0 - assembly <= kept_launches(lin.iterations), (rtol, lin.iterations)
+            seen.add(lin.iterations)
+        s.close()
+    # step counts at which a first piece of one step would have cost a piece more
+    assert seen & {2, 5, 6, 9, 10}, seen

@@ -399,6 +399,7 @@ extern "C" int v2d_batch_newton(v2d_batch *B, double *res, int *flags, v2d_lin_s
     if (refactor) {
         V2D_TRY(mf_factor(B->plan, B->lu, B->rowptr, B->val, s));
         ++B->factorizations;
+        A.lu_fresh = true;
         V2D_TRY(krylov_solve(B->kw, A, B->b, B->x, kp, &ls, s));
     } else {
         v2d_krylov_params k2 = kp;
@@ -409,7 +410,7 @@ extern "C" int v2d_batch_newton(v2d_batch *B, double *res, int *flags, v2d_lin_s
             const int its0 = ls.iterations;
             V2D_TRY(mf_factor(B->plan, B->lu, B->rowptr, B->val, s));
             ++B->factorizations;
-            refactor = true;
+            refactor = A.lu_fresh = true;
             V2D_TRY(krylov_solve(B->kw, A, B->b, B->x, kp, &ls, s));
             ls.iterations += its0;
         }

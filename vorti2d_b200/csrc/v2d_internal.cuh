@@ -274,6 +274,7 @@ struct CsrOp {
     int nblk = 0;  // number of 2x2 blocks (or n for point layout)
     const MfPlan *lu_plan = nullptr;   // V2D_PC_LU: factors of this operator
     const MfFactor *lu = nullptr;
+    bool lu_fresh = false;             // lu are the factors of these very values
     bool lu_transpose = false;         // the operator is J^T and lu factors J: the
                                        // preconditioner is the transposed solve
 };

@@ -56,6 +56,7 @@ struct Ctl {
     int cycles;
     int nonfinite;
     int ok;              // conv, and the true residual reached its target (or stagnated near it)
+    int hold;            // steps 0 and 1 run as one: no end between them
     int stagnated;       // a cycle failed to halve the residual near the target
     double prev_beta;
     unsigned int cnt[4]; // last-block counters
@@ -391,12 +392,18 @@ __global__ void __launch_bounds__(kRedThreads) k_update(const Desc *d, Ctl *ctl,
     }
 }
 
+// The kernels of a cycle's end, queued before it is known whether the cycle has
+// ended (guard 1; 2 after step 0, where it is left for step 1's under hold).
+__device__ __forceinline__ bool no_end(const Ctl *ctl, int guard)
+{
+    return guard && (!ctl->cyc_stop || (guard == 2 && ctl->hold));
+}
+
 // End of a cycle: back-substitution R y = g over the completed columns.
-// (guard: only if the cycle's last step has stopped it; here and in the next two)
 __global__ void k_backsolve(const Desc *d, Ctl *ctl, const double *H, const double *g, double *y,
                             int guard)
 {
-    if (ctl->conv || (guard && !ctl->cyc_stop)) return;
+    if (ctl->conv || no_end(ctl, guard)) return;
     if (threadIdx.x != 0) return;
     const int m = d->m, jj = ctl->jdone;
     for (int i = jj - 1; i >= 0; --i) {
@@ -412,7 +419,7 @@ template <class T>
 __global__ void __launch_bounds__(256) k_correct(const Desc *d, Ctl *ctl, const T *V, const double *y,
                                                  T *t_scratch, double *x, const T *Z, int guard)
 {
-    if (ctl->conv || (guard && !ctl->cyc_stop)) return;
+    if (ctl->conv || no_end(ctl, guard)) return;
     const int n = d->n, jj = ctl->jdone;
     if (d->precond == V2D_PC_LU) {   // x += Z y
         V2D_GRID_STRIDE(r, n)
@@ -468,7 +475,7 @@ __global__ void __launch_bounds__(kSpmvThreads) k_residual(const Desc *d, Ctl *c
                                                            double *partial, double *g, int first,
                                                            int guard)
 {
-    if (ctl->conv || (guard && !ctl->cyc_stop)) return;
+    if (ctl->conv || no_end(ctl, guard)) return;
     __shared__ double red[32];
     const int n = d->n, m = d->m;
     const int lane = threadIdx.x & (kTPR - 1);
@@ -572,23 +579,26 @@ static int tile_grid(long long n)
     return (int)std::max(1LL, std::min<long long>(kTileBlocks, g));
 }
 
-// A restart cycle runs as a few captured segments of Arnoldi steps (FP64:
-// [0,1), [1,4), FP32: [0,2), [2,6), then 4, 4 and 8 at a time), the first with
-// the cycle's end behind it, then a finishing graph (back-substitution,
-// correction, FP64 residual).  The host reads the control block after each
-// segment and skips the remaining segments once the cycle has stopped, so a
-// cycle that converges in a few steps (the usual case with the LU
+// A restart cycle runs as a few captured segments of Arnoldi steps ([0,2),
+// [2,6), [6,10), [10,14), then 8 at a time; steps 0 and 1 apart in FP64), the
+// ones up to step 1 with the cycle's end behind them, then a finishing graph
+// (back-substitution, correction, FP64 residual).  The host reads the control
+// block after each segment and skips the remaining segments once the cycle has
+// stopped, so a cycle that converges in a few steps (the usual case with the LU
 // preconditioner: 6-12 with factors kept across Newton iterations) launches few
 // steps past its last one; each step after the stop is a chain of launches that
-// return at once.  With fresh FP64 factors the first step is the only one (25 x
-// 17: 1.22 ms a pass against 1.27 with two); FP32 cycles need two or more (181 x
-// 181 mixed: 28.1 ms against 29.3 with one).
+// return at once.  With fresh FP64 factors one step is enough up to about 257 x
+// 257 and two beyond: there the host reads after step 0 too (25 x 17: 1.22 ms a
+// pass against 1.27 without).  FP32 cycles need two or more (181 x 181 mixed:
+// 28.1 ms against 29.3 with a read after step 0).
 static std::vector<int> segment_bounds(int m, bool fp32)
 {
     std::vector<int> b{0};
-    const int len[2][4] = {{1, 3, 4, 4}, {2, 4, 4, 4}};
-    for (int q = 0; b.back() < m; ++q)
-        b.push_back(std::min(m, b.back() + (q < 4 ? len[fp32][q] : 8)));
+    if (!fp32) b.push_back(1);
+    for (int len : {2, 4, 4, 4}) b.push_back(b.back() == 1 ? 2 : b.back() + len);
+    while (b.back() < m) b.push_back(b.back() + 8);
+    while (b.size() > 2 && b[b.size() - 2] >= m) b.pop_back();
+    b.back() = std::min(b.back(), m);
     return b;
 }
 
@@ -700,8 +710,8 @@ static int capture_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, doub
                 if (capture_launch_failed(s, "k_update", j)) return V2D_ECUDA;
             }
         }
-        if (q == 0) {   // the first step often is the last: its end without a round trip
-            finish(1);
+        if (bnd[q] < 2) {   // the first steps often are the last: their end without a round trip
+            finish(bnd[q + 1] == 1 ? 2 : 1);
             nl += 3;
         }
         cudaGraphExec_t ge = nullptr;
@@ -745,8 +755,10 @@ static int run_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, double *
     for (size_t q = 0; q < w->seg[which].size(); ++q) {
         V2D_CUDA_TRY(cudaGraphLaunch(w->seg[which][q], s));
         count_launches(w->seg_launches[which][q]);
-        V2D_TRY(read(q == 0));
-        if (w->ctl_host->conv || w->ctl_host->cycles != cycles) {   // its end was in segment 0
+        const bool first = w->seg_bounds[which][q] < 2;
+        if (q == 0 && which == 0 && !A.lu_fresh && w->seg[which].size() > 1) continue;
+        V2D_TRY(read(first));
+        if (w->ctl_host->conv || w->ctl_host->cycles != cycles) {   // it ended in the first steps
             *h = *w->ctl_host;
             return V2D_OK;
         }
@@ -847,6 +859,7 @@ int krylov_solve(KrylovWork *w, const CsrOp &A, const double *d_b, double *d_x,
     c.atol = prm.atol;
     c.max_it = prm.max_it;
     c.inner_rtol = fp32 ? prm.inner_rtol : 0.0;
+    c.hold = !A.lu_fresh;
     k_begin<<<grid_for(A.n, 256), 256, 0, s>>>(hd, c, w->desc, w->ctl);
     k_residual<<<res_grid(A.n), kSpmvThreads, 0, s>>>(w->desc, w->ctl, w->r, w->partial, w->g, 1, 0);
     V2D_CUDA_TRY(cudaGetLastError());

@@ -437,6 +437,7 @@ extern "C" int v2d_linsys_solve(v2d_linsys *L, double *x, v2d_lin_stats *st)
             }
         }
         if (fresh) {
+            A.lu_fresh = true;
             V2D_TRY(krylov_solve(L->kw, A, L->b, L->x, kp, &ls, L->s));
             V2D_TRY(mf_check_barrier(L->lu, L->s));
             ls.iterations += its0;

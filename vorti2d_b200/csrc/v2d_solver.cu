@@ -445,7 +445,7 @@ extern "C" int v2d_solver_newton(v2d_solver *S, double urot, double *res, v2d_li
         if (!mixed) ++S->lu0_ver;
         ++S->lu_factorizations;
         S->lu_ready = true;
-        refactored = true;
+        refactored = A.lu_fresh = true;
         return V2D_OK;
     };
     if (lu) {
@@ -937,7 +937,7 @@ extern "C" int v2d_solver_adjoint(v2d_solver *S, double urot, const double *g_ho
     AT.nblk = g.n;
     AT.lu_plan = S->plan;
     AT.lu = S->lu[0];
-    AT.lu_transpose = true;
+    AT.lu_transpose = AT.lu_fresh = true;
     v2d_krylov_params kp;
     v2d_krylov_defaults(&kp);
     kp.restart = kAdjRestart;

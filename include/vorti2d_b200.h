@@ -444,8 +444,11 @@ int v2d_solver_lu_split(v2d_solver *s, int level, int *current);
 
 /* Tuning aid (no reference counterpart): the work-item granularity of the
  * LU preconditioner solve, rows[L] rows of a front per work item on tree
- * level L (0: whole fronts; a handle starts with about 300 items per level);
- * rows may be null to only read the current
+ * level L (0: whole fronts).  A handle starts with about 300 items per level,
+ * counted by the variables of the level's fronts forward and by their pivots
+ * backward: rows and out_rows hold the forward counts, and a level at its
+ * starting count keeps the backward one that belongs to it; any other count
+ * holds for both sweeps of its level.  rows may be null to only read the current
  * setting into out_rows (cap >= levels) and *nlevels_out.  Every setting
  * forms the same products in the same order; only how the rows are split over
  * CTAs changes. */

@@ -122,7 +122,7 @@ struct MfPlan {
     // checked when the plan is built (see items_build).
     int nitems = 0, nctr = 0;
     std::vector<int> h_items, lvl_fwd, lvl_bwd;
-    std::vector<int> item_rows_b;  // the default split's backward rows per item (empty: item_rows)
+    std::vector<int> item_rows_b;  // backward rows per item of the device's split (empty: item_rows)
     std::vector<int> item_rows;    // rows per item of each level (0: whole fronts; R < 0:
                                    // -R rows per item after one gather item per front)
     std::vector<int> lvl_fwd_g, lvl_bwd_g;   // gather items at the start of each level's

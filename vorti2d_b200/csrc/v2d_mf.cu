@@ -816,8 +816,9 @@ int mf_plan_create(int imax, int jmax, int n, const int *h_rowptr, const int *h_
 }
 
 // New work-item granularity for the solve: rows[L] rows per item on level L
-// (0: whole fronts; R > 0: R rows; R < 0: -R rows after one gather item per
-// front).  Rebuilds and
+// (0: whole fronts; R > 0: R rows; R < 0: -R rows).  A level at its default
+// count keeps the default's backward rows, whatever the others are set to; on
+// another level the count holds for both sweeps.  Rebuilds and
 // re-uploads the item table (its order is checked again); the device pointer
 // changes, so solves captured in graphs before must be captured again
 // (items_ver counts the tables).
@@ -829,11 +830,9 @@ int mf_plan_set_item_rows(MfPlan *P, const int *rows, int nlevels)
         V2D_ARG_CHECK(rows[L] >= -4096 && rows[L] <= 4096, "lu item rows: level %d: %d", L,
                       rows[L]);
     const std::vector<int> keep = P->item_rows, keep_b = P->item_rows_b;
-    device_item_rows(P);   // the rows of the default split mean that split
-    if (!std::equal(rows, rows + nlevels, P->item_rows.begin())) {
-        P->item_rows.assign(rows, rows + nlevels);
-        P->item_rows_b.clear();
-    }
+    device_item_rows(P);
+    for (int L = 0; L < nlevels; ++L)
+        if (rows[L] != P->item_rows[L]) P->item_rows[L] = P->item_rows_b[L] = rows[L];
     if (items_build(P) != V2D_OK) {
         P->item_rows = keep;
         P->item_rows_b = keep_b;

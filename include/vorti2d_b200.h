@@ -442,6 +442,14 @@ int v2d_solver_lu_flow_form(v2d_solver *s, int form, int *current);
  * products in the same order. */
 int v2d_solver_lu_split(v2d_solver *s, int level, int *current);
 
+/* Test aid (no reference counterpart): how many tests a device wait of the LU
+ * factorization and solve makes before it runs out -- gather: of the solve's
+ * values from other blocks, pipe: between the threads of one block, after a
+ * first few; negative: the default (about a second, several seconds), which is
+ * also the most.  A wait
+ * that runs out ends the call with V2D_ETIMEOUT. */
+int v2d_solver_lu_wait_limits(v2d_solver *s, int gather, int pipe);
+
 /* Tuning aid (no reference counterpart): the work-item granularity of the
  * LU preconditioner solve, rows[L] rows of a front per work item on tree
  * level L (0: whole fronts).  A handle starts with about 300 items per level,

@@ -42,19 +42,27 @@ __device__ __forceinline__ bool mbar_test(unsigned long long *b, unsigned parity
                  : "memory");
     return ok != 0;
 }
-// Waits between the threads of a CTA: they end when the CTA gives up (quit,
-// after kFlowSpins of its own waits on others) or after this many tests, which
-// take longer than those.
+// Waits between the threads of a CTA: they end when the CTA gives up (quit) or
+// after 32 tests in a row and `limit` slower ones: false.  kPipeSpins of them
+// take longer than kFlowSpins of the solve's waits on other CTAs, which a thread
+// of this one may be in.
 constexpr int kPipeSpins = 1 << 27;
 __device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity,
-                                          volatile int *quit)
+                                          volatile int *quit, int limit)
 {
-    for (int n = 0; n < kPipeSpins; ++n) {
+    for (int n = 0; n < 32; ++n)
         if (mbar_test(b, parity)) return true;
-        if (n > 32) __nanosleep(32);
-        if (quit && *quit) return false;
+    for (int n = 0; n < limit && !(quit && *quit); ++n) {
+        __nanosleep(32);
+        if (mbar_test(b, parity)) return true;
     }
     return false;
+}
+// The same by a whole warp, with one answer for all of its lanes.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long *b, unsigned parity,
+                                               volatile int *quit, int limit)
+{
+    return __all_sync(0xffffffffu, mbar_wait(b, parity, quit, limit));
 }
 // bytes (a multiple of 16) from src to dst, both 16-byte aligned; completes on b.
 __device__ __forceinline__ void bulk_copy(void *dst, const void *src, unsigned bytes,

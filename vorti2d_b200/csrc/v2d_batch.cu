@@ -396,6 +396,7 @@ extern "C" int v2d_batch_newton(v2d_batch *B, double *res, int *flags, v2d_lin_s
     kp.rtol = B->kp.rtol / std::sqrt((double)std::max(1, nact));
     bool refactor = !(kp.lu_reuse_its > 0 && B->lu_valid && B->lu_last_its <= kp.lu_reuse_its);
     v2d_lin_stats ls{};
+    B->lu_valid = false;   // until this iteration's waits are known to have ended
     if (refactor) {
         V2D_TRY(mf_factor(B->plan, B->lu, B->rowptr, B->val, s));
         ++B->factorizations;

@@ -728,6 +728,12 @@ __global__ void __launch_bounds__(256, 3) k_update(int q0, int k, int nt, int v0
 // Measured and not taken, on the same fronts: bulk copies per row (0.85 ms),
 // two groups of four warps in turn (0.59), two of eight that read the old
 // entries themselves (0.65), strips with two CTAs per SM (0.76).
+//
+// No wait depends on another CTA, so none should run out; if one does, bit 4 of
+// *err is set and the CTA ends.  Each side then leaves through a barrier that all
+// of its threads reach: the producers' at the next ticket (stop, by the ticket's
+// parity, so that a thread already past it cannot change what a slower one reads),
+// the multiplying warps' at the next pivot tile or at the end (leave).
 constexpr int kWideWarps = 8, kWideProducers = 128;
 
 struct WideShared {
@@ -740,13 +746,16 @@ struct WideShared {
         int q, r0, c0, a;   // front (-1: no more), first row and column, A's buffer
     } tile[2];
     int ticket[2];
+    volatile int quit;   // a wait ran out: the others end
+    int stop[2], leave;  // ... and the producers, the multiplying warps leave together
 };
 static_assert(sizeof(PivotSmem) <= sizeof(WideShared::Stage), "the inversion uses a stage");
 
 __global__ void __launch_bounds__(32 * kWideWarps + kWideProducers, 1)
     k_update_wide(int q0, int nq, int k, int nt, int len, int v0, const int *__restrict__ S_,
                   const int *__restrict__ f_, const long long *__restrict__ foff,
-                  const int *__restrict__ voff, double *F, const double *C, int *ticket, int *flag)
+                  const int *__restrict__ voff, double *F, const double *C, int *ticket, int *flag,
+                  int limit, int *err)
 {
     extern __shared__ __align__(16) unsigned char tile_raw[];
     WideShared &sh = *reinterpret_cast<WideShared *>(tile_raw);
@@ -755,7 +764,9 @@ __global__ void __launch_bounds__(32 * kWideWarps + kWideProducers, 1)
         for (int s = 0; s < 2; ++s) {
             mbar_init(&sh.full[s], kWideProducers + 1);
             mbar_init(&sh.empty[s], kWideWarps);
+            sh.stop[s] = 0;
         }
+        sh.quit = sh.leave = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -764,11 +775,14 @@ __global__ void __launch_bounds__(32 * kWideWarps + kWideProducers, 1)
         const int ns = (nt + len - 1) / len, p = threadIdx.x - 32 * kWideWarps;
         const long long total = nq + (long long)nq * nt * ns;
         int n = 0, a = 0;
+        bool failed = false;
         // the stage of the next tile once it is free; false: given up
         auto stage = [&](int q, int r0, int c0) {
             const int s = n & 1;
-            if (n >= 2 && !mbar_wait(&sh.empty[s], ((n >> 1) - 1) & 1, nullptr)) {
-                atomicOr(flag, 1);
+            if (n >= 2 && !mbar_wait(&sh.empty[s], ((n >> 1) - 1) & 1, &sh.quit, limit)) {
+                atomicOr(err, 4);
+                sh.quit = 1;
+                failed = true;
                 return false;
             }
             if (p == 0) {
@@ -780,9 +794,11 @@ __global__ void __launch_bounds__(32 * kWideWarps + kWideProducers, 1)
         int next = p == 0 ? atomicAdd(ticket, 1) : 0;
         for (int i = 0;; ++i) {
             if (p == 0) sh.ticket[i & 1] = next;
+            if (failed) sh.stop[i & 1] = 1;
             asm volatile("bar.sync 3, %0;" ::"n"(kWideProducers) : "memory");
             const int t = sh.ticket[i & 1];
-            if (t >= total) break;
+            failed = sh.stop[i & 1];
+            if (failed || t >= total) break;
             if (p == 0) next = atomicAdd(ticket, 1);
             const bool pivots = t < nq;
             const int u = t - nq, q = q0 + (pivots ? t : u / (nt * ns));
@@ -798,7 +814,7 @@ __global__ void __launch_bounds__(32 * kWideWarps + kWideProducers, 1)
             for (int j = j0; j < j1; ++j) {
                 const int c0 = j * kTile, nc = min(kTile, f - c0);
                 if (nc <= 0 || (!pivots && rt == kt + 1 && j == rt && k + kPiv < S)) continue;
-                if (!stage(q, r0, c0)) return;
+                if (!stage(q, r0, c0)) break;
                 WideShared::Stage &st = sh.st[n & 1];
                 if (first)
 #pragma unroll 4
@@ -819,18 +835,23 @@ __global__ void __launch_bounds__(32 * kWideWarps + kWideProducers, 1)
             }
             if (!first) a ^= 1;   // the other buffer's strip is done two tiles on
         }
-        if (stage(-1, 0, 0)) mbar_arrive(&sh.full[n & 1]);
+        if (!failed && stage(-1, 0, 0)) mbar_arrive(&sh.full[n & 1]);
+        asm volatile("cp.async.wait_all;" ::: "memory");   // no copy outlives its thread
         return;
     }
     const int g = lane >> 2, t = lane & 3, wr = (wid >> 2) * 32, wc = (wid & 3) * 16;
     for (int n = 0;; ++n) {
         const int s = n & 1;
-        if (!mbar_wait(&sh.full[s], (n >> 1) & 1, nullptr)) {
-            atomicOr(flag, 1);
-            return;
+        const bool ok = mbar_wait_warp(&sh.full[s], (n >> 1) & 1, &sh.quit, limit);
+        if (!ok && lane == 0) {
+            atomicOr(err, 4);
+            sh.quit = sh.leave = 1;
         }
         const WideShared::Work w = sh.tile[s];
-        if (w.q < 0) return;
+        if (!ok || w.q < 0) {
+            asm volatile("bar.sync 2, %0;" ::"n"(32 * kWideWarps) : "memory");
+            return;
+        }
         WideShared::Stage &st = sh.st[s];
         const int S = S_[w.q], f = f_[w.q], r0 = w.r0 + wr + g, c0 = w.c0 + wc + 2 * t;
         double *A = F + foff[w.q];
@@ -866,7 +887,10 @@ __global__ void __launch_bounds__(32 * kWideWarps + kWideProducers, 1)
         if (!pivots && lane == 0) mbar_arrive(&sh.empty[s]);
         const int wn = pivots ? min(kPiv, S - w.r0) : 0;   // the next block's pivots
         PivotSmem &ps = *reinterpret_cast<PivotSmem *>(&st);
-        if (pivots) asm volatile("bar.sync 2, %0;" ::"n"(32 * kWideWarps) : "memory");
+        if (pivots) {
+            asm volatile("bar.sync 2, %0;" ::"n"(32 * kWideWarps) : "memory");
+            if (sh.leave) return;
+        }
 #pragma unroll
         for (int mi = 0; mi < 4; ++mi)
 #pragma unroll

@@ -146,11 +146,17 @@ inline double front_flops(int S, int f)
     return 2.0 * (sq(f - 1.0) - sq(m - 1.0)) + 2.0 * S * (double)S * S / 3.0 + 2.0 * m * S * S;
 }
 
-// Error state of the dataflow solve: err is set when a dependency wait ran
-// out (read and reset by mf_check_barrier).
+// Error state: err is set when a wait ran out, bit 2 by the dataflow solve, bit 4
+// by the factorization's wide update (read and reset by mf_check_barrier).
 struct MfBarrier {
     unsigned int count, gen;
     int err, pad;
+};
+
+// Tests of one wait before it runs out: the solve's waits for other CTAs' values
+// and the waits between the threads of a CTA.
+struct WaitLimits {
+    int gather, pipe;
 };
 
 // One form of the dataflow solve's launch: CTAs, shared memory, of which the
@@ -184,6 +190,7 @@ struct MfFactor {
                                 // (forward before, backward after the upper levels)
     int flow = 1;               // 1: the solve is one dataflow launch; 0: one launch per level
                                 // and sweep
+    WaitLimits limits{0, 0};
     cudaGraphExec_t graph = nullptr;
     const double *graph_val = nullptr;
     const int *graph_rowptr = nullptr;
@@ -228,13 +235,16 @@ int mf_factor(const MfPlan *P, MfFactor *M, const int *rowptr, const double *val
 // *n_launches (if given) receives the number of kernels launched.
 int mf_apply(const MfPlan *P, const MfFactor *M, const void *b, void *x, const int *stop_a,
              const int *stop_b, cudaStream_t s, long long *n_launches);
+// The tests of a wait before it runs out (negative: the default); solves captured
+// in graphs must be captured again (the plan's items_ver counts this too).
+int mf_set_wait_limits(MfPlan *P, MfFactor *M, int gather, int pipe);
 // lambda = A^-T g with the factors (the transposed solve: a bottom-up sweep
 // with A11^-T / H^T, then a top-down sweep with G^T).
 int mf_apply_transpose(const MfPlan *P, MfFactor *M, const void *g, void *lambda, cudaStream_t s,
                        long long *launches = nullptr);
 int mf_flag(const MfFactor *M, int *flag, cudaStream_t s);
-// V2D_ETIMEOUT (and a reset error state) if a dependency wait of the
-// dataflow solve timed out since the last check.
+// V2D_ETIMEOUT (and a reset error state) if a wait of the dataflow solve or of
+// the factorization ran out since the last check.
 int mf_check_barrier(MfFactor *M, cudaStream_t s);
 // The device word behind it.
 const int *mf_error_word(const MfFactor *M);

@@ -418,6 +418,15 @@ extern "C" int v2d_linsys_solve(v2d_linsys *L, double *x, v2d_lin_stats *st)
         A.lu_plan = L->plan;
         A.lu = L->lu;
         bool fresh = L->lu_fresh;
+        // a wait that ran out: the factors are not used again
+        auto check = [&]() -> int {
+            const int status = mf_check_barrier(L->lu, L->s);
+            if (status != V2D_OK) {
+                L->lu_fresh = false;
+                L->lu_last_its = -1;
+            }
+            return status;
+        };
         const bool reuse = !fresh && kp.lu_reuse_its > 0 && L->lu_last_its >= 0 &&
                            L->lu_last_its <= kp.lu_reuse_its;
         if (!fresh && !reuse) {
@@ -429,7 +438,7 @@ extern "C" int v2d_linsys_solve(v2d_linsys *L, double *x, v2d_lin_stats *st)
             v2d_krylov_params k2 = kp;
             k2.max_it = std::min(kp.max_it, kp.lu_reuse_its + 5);
             V2D_TRY(krylov_solve(L->kw, A, L->b, L->x, k2, &ls, L->s));
-            V2D_TRY(mf_check_barrier(L->lu, L->s));
+            V2D_TRY(check());
             if (!ls.converged) {
                 its0 = ls.iterations;
                 V2D_TRY(mf_factor(L->plan, L->lu, L->indptr, L->data, L->s));
@@ -439,7 +448,7 @@ extern "C" int v2d_linsys_solve(v2d_linsys *L, double *x, v2d_lin_stats *st)
         if (fresh) {
             A.lu_fresh = true;
             V2D_TRY(krylov_solve(L->kw, A, L->b, L->x, kp, &ls, L->s));
-            V2D_TRY(mf_check_barrier(L->lu, L->s));
+            V2D_TRY(check());
             ls.iterations += its0;
         }
         const bool refactored = fresh && !L->lu_fresh;

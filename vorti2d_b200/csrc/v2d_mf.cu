@@ -1231,6 +1231,7 @@ int mf_factor_create(const MfPlan *P, int fp32, int fact64, MfFactor **out)
     MfFactor *M = new MfFactor();
     M->fp32 = fp32;
     M->fact64 = fp32 && fact64 ? 1 : 0;
+    M->limits = WaitLimits{kFlowSpins, kPipeSpins};
     const size_t es = fp32 ? sizeof(float) : sizeof(double);          // solve
     const size_t esf = fp32 && !M->fact64 ? sizeof(float) : sizeof(double);   // factorization
     cudaError_t e = cudaSuccess;
@@ -1435,7 +1436,7 @@ static int factor_launches(const MfPlan *P, MfFactor *M, const int *rowptr, cons
                 const int len = (int)std::max(1LL, std::min(8LL, tiles / (4 * kSMs)));
                 k_update_wide<<<kSMs, 32 * kWideWarps + kWideProducers, sizeof(WideShared), s>>>(
                     q0, nq, k, nt, len, v0, P->d_S, P->d_f, P->d_foff, P->d_voff, (double *)F,
-                    (const double *)C, ticket++, M->flag);
+                    (const double *)C, ticket++, M->flag, M->limits.pipe, &M->bar->err);
             } else {
                 k_update<T><<<nq * nt * nt, 256, smem, s>>>(q0, k, nt, v0, P->d_S, P->d_f,
                                                             P->d_foff, P->d_voff, F, C, M->flag);
@@ -1538,17 +1539,17 @@ static int apply_launches(const MfPlan *P, const MfFactor *M, const T *b, T *x, 
             if (M->flow_form == 1)
                 k_solve_flow<T, 3><<<n, kSolveThreads + 32, up.smem, s>>>(
                     D, F, b, M->rs, z, upd, x, items, i0, i1, up.vbytes, up.cbytes,
-                    M->tickets, slot, M->bar, stop_a, stop_b, trace);
+                    M->tickets, slot, M->bar, stop_a, stop_b, M->limits, trace);
             else
                 k_solve_flow<T, 2><<<n, kSolveThreads + 32, up.smem, s>>>(
                     D, F, b, M->rs, z, upd, x, items, i0, i1, up.vbytes, up.cbytes,
-                    M->tickets, slot, M->bar, stop_a, stop_b, trace);
+                    M->tickets, slot, M->bar, stop_a, stop_b, M->limits, trace);
         };
         auto lower = [&](int i0, int i1, int slot) {
             k_solve_flow<T, kLowMinBlocks, kLowThreads>
                 <<<std::max(1, std::min(i1 - i0, lo.grid)), kLowThreads + 32, lo.smem, s>>>(
                     D, F, b, M->rs, z, upd, x, items, i0, i1, lo.vbytes, lo.cbytes,
-                    M->tickets, slot, M->bar, stop_a, stop_b, trace);
+                    M->tickets, slot, M->bar, stop_a, stop_b, M->limits, trace);
         };
         const int Ls = M->split;
         if (Ls > 0 && Ls < P->nlevel && lo.grid > 0) {
@@ -1637,6 +1638,16 @@ int mf_apply_transpose(const MfPlan *P, MfFactor *M, const void *g, void *lambda
 int mf_flag(const MfFactor *M, int *flag, cudaStream_t s)
 {
     V2D_CUDA_TRY(cudaMemcpyAsync(flag, M->flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    return V2D_OK;
+}
+
+int mf_set_wait_limits(MfPlan *P, MfFactor *M, int gather, int pipe)
+{
+    M->limits.gather = gather < 0 ? kFlowSpins : std::min(gather, kFlowSpins);
+    M->limits.pipe = pipe < 0 ? kPipeSpins : std::min(pipe, kPipeSpins);
+    if (M->graph) V2D_CUDA_TRY(cudaGraphExecDestroy(M->graph));
+    M->graph = nullptr;
+    ++P->items_ver;
     return V2D_OK;
 }
 
@@ -1791,6 +1802,7 @@ int mf_time_factor_launches(const MfPlan *P, MfFactor *M, const int *rowptr, con
     for (auto &e : ev)
         if (e) cudaEventDestroy(e);
     if (st != V2D_OK) return st;
+    V2D_TRY(mf_check_barrier(M, s));
     for (int k = 0; k < nl; ++k) ms[k] = acc[k] / reps;
     *n = nl;
     return V2D_OK;
@@ -1806,7 +1818,8 @@ int mf_check_barrier(MfFactor *M, cudaStream_t s)
     V2D_CUDA_TRY(cudaStreamSynchronize(s));
     if (err) {
         V2D_CUDA_TRY(cudaMemsetAsync(M->bar, 0, sizeof(MfBarrier), s));
-        set_error("LU solve: a dependency wait of the dataflow solve timed out");
+        set_error(err & 4 ? "LU factor: a wait of the wide update timed out"
+                          : "LU solve: a dependency wait of the dataflow solve timed out");
         return V2D_ETIMEOUT;
     }
     return V2D_OK;

@@ -92,7 +92,7 @@ template <> struct Unset<double> {
 };
 
 // Reads of one entry before a CTA gives up (each sleeps 50 ns: about a second
-// in all).
+// in all), unless WaitLimits says otherwise.
 constexpr int kFlowSpins = 1 << 21;
 
 __device__ __forceinline__ float ld_relaxed(const float *p)
@@ -168,7 +168,7 @@ template <class T, int NT> struct SolveGather {
     template <bool Wait>
     __device__ __forceinline__ bool run(const SolveItem &it, const MfDev &D, const T *rhs,
                                         const double *__restrict__ rs, const T *zbuf, const T *upd,
-                                        const T *x, T *dst, volatile int *err)
+                                        const T *x, T *dst, volatile int *err, int limit)
     {
         const int n = count(it);
         for (int e0 = threadIdx.x; e0 < n; e0 += kGatherRegs * NT) {
@@ -204,7 +204,7 @@ template <class T, int NT> struct SolveGather {
 #pragma unroll
                     for (int k = 0; k < kGatherRegs; ++k) unset = unset || Unset<T>::is(u[h][k]);
                 if (!Wait || !unset) break;
-                if (spin >= kFlowSpins || ((spin & 63) == 63 && *err)) return false;
+                if (spin >= limit || ((spin & 63) == 63 && *err)) return false;
                 __nanosleep(50);
             }
 #pragma unroll
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(kSolveThreads, 2) k_solve_level(
     const SolveItem it = load_item(items, i0 + blockIdx.x);
     SolveGather<T, NT> g;
     g.pre(it, D, rhs, rs);
-    g.template run<false>(it, D, rhs, rs, zbuf, upd, x, vec, nullptr);
+    g.template run<false>(it, D, rhs, rs, zbuf, upd, x, vec, nullptr, 0);
     __syncthreads();
     if (it.kind == 0)
         for (int r = it.rb + (int)threadIdx.x; r < min(it.re, it.S); r += NT)
@@ -323,8 +323,8 @@ __device__ __forceinline__ unsigned long long globaltimer_ns()
 struct FlowShared {
     unsigned long long full[kStages], empty[kStages], dfull[2], dempty[2];
     SolveItem item[2];
-    volatile int quit;
-    int ok;
+    volatile int quit;   // a wait ran out: the others end
+    int ok, leave;       // leave: the threads that compute end after the next barrier
 };
 
 // The whole solve as one launch of work items in the plan's order (forward
@@ -335,7 +335,9 @@ struct FlowShared {
 // always one whose CTA is at it and whose dependencies are met: no co-resident
 // grid is needed.  A wait that runs out (or an error seen while waiting) sets
 // bar->err (bit 2) and *stop_a (so GMRES stops instead of using an unfinished
-// preconditioner) and ends the CTA.
+// preconditioner) and ends the CTA: the threads that compute leave together, by
+// `leave`, which is only set between an item's start and its first barrier, and
+// the producer warp once its copies have landed.
 //
 // What an item reads besides the vectors of other items -- its table entry and
 // the factor rows, most of the solve's bytes -- depends on no other item, so a
@@ -359,7 +361,7 @@ __global__ void __launch_bounds__(NT + 32, MINB) k_solve_flow(
     const MfDev D, const T *F, const T *rhs, const double *__restrict__ rs, T *zbuf, T *upd, T *x,
     const SolveItemDev *__restrict__ items, int item0, int item1, int vbytes, int cbytes,
     int *tickets, int slot, MfBarrier *bar, const int *stop_a, const int *stop_b,
-    unsigned long long *trace)
+    const WaitLimits limits, unsigned long long *trace)
 {
     constexpr int nw = NT / 32;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -375,12 +377,17 @@ __global__ void __launch_bounds__(NT + 32, MINB) k_solve_flow(
             mbar_init(&sh.dfull[s], 1);
             mbar_init(&sh.dempty[s], 1);
         }
-        sh.quit = 0;
+        sh.quit = sh.leave = 0;
         sh.ok = !stopped(stop_a, stop_b);   // read once: all of the CTA's threads agree
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
     if (!sh.ok) return;
+    auto give_up = [&]() {
+        atomicOr(&bar->err, 2);
+        if (stop_a) atomicExch(const_cast<int *>(stop_a), 1);
+        sh.quit = 1;
+    };
     if (threadIdx.x >= NT) {   // ---------------------------------- producer
         const int lane = threadIdx.x & 31;
         // the next item's ticket and table entry are fetched while this one's
@@ -398,6 +405,11 @@ __global__ void __launch_bounds__(NT + 32, MINB) k_solve_flow(
             } while (it.kind > 1);   // the items gather for themselves
             return it;
         };
+        // b's phase n has ended (a reader that gave up ends it too)
+        auto freed = [&](unsigned long long *b, int n) {
+            const bool done = mbar_wait(b, n & 1, &sh.quit, limits.pipe);
+            return __all_sync(0xffffffffu, done && !sh.quit) != 0;
+        };
         int ks = 0;   // chunks issued
         bool ok = true;
         SolveItem next = take();
@@ -407,19 +419,19 @@ __global__ void __launch_bounds__(NT + 32, MINB) k_solve_flow(
                 next = take();
                 plan_chunks<T>(it, cbytes, nw);
             }
-            if (k >= 2 && !mbar_wait(&sh.dempty[k & 1], ((k >> 1) - 1) & 1, &sh.quit)) break;
+            ok = k < 2 || freed(&sh.dempty[k & 1], (k >> 1) - 1);
+            if (!ok) break;
             if (lane == 0) {
                 sh.item[k & 1] = it;
                 mbar_arrive(&sh.dfull[k & 1]);
             }
-            if (it.index < 0) return;   // every chunk issued is awaited by the readers
+            if (it.index < 0) break;
             const int len = it.kind == 0 ? it.S : it.f;
             const T *A = F + it.fo + (long long)it.r0 * it.f;
             // the chunk's stage once its readers are done with it
             auto stage = [&]() -> unsigned char * {
                 const int s = ks % kStages;
-                if (ks >= kStages && !mbar_wait(&sh.empty[s], (ks / kStages - 1) & 1, &sh.quit))
-                    return nullptr;
+                if (ks >= kStages && !freed(&sh.empty[s], ks / kStages - 1)) return nullptr;
                 return chunk0 + (size_t)s * cbytes;
             };
             if (it.group > 0) {
@@ -481,27 +493,28 @@ __global__ void __launch_bounds__(NT + 32, MINB) k_solve_flow(
                 }
             }
         }
-        // gave up: let the copies in flight land before the CTA ends
+        if (!ok && lane == 0) give_up();
+        // the CTA may end before its readers have awaited every copy: let them land
         for (int c = max(0, ks - kStages); c < ks; ++c)
-            mbar_wait(&sh.full[c % kStages], (c / kStages) & 1, nullptr);
+            mbar_wait(&sh.full[c % kStages], (c / kStages) & 1, nullptr, kPipeSpins);
         return;
     }
     // -------------------------------------------------------------- the items
     auto sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); };
     int ks = 0;
     for (int k = 0;; ++k) {
-        if (!mbar_wait(&sh.dfull[k & 1], (k >> 1) & 1, nullptr)) return;
+        if (!mbar_wait_warp(&sh.dfull[k & 1], (k >> 1) & 1, &sh.quit, limits.pipe)) goto gone;
         const SolveItem &it = sh.item[k & 1];   // stays until dempty
-        if (it.index < 0) return;
+        if (it.index < 0) {
+            sync();
+            return;
+        }
         SolveGather<T, NT> g;
         g.pre(it, D, rhs, rs);
-        if (!g.template run<true>(it, D, rhs, rs, zbuf, upd, x, vec, &bar->err)) {
-            atomicOr(&bar->err, 2);
-            if (stop_a) atomicExch(const_cast<int *>(stop_a), 1);
-            sh.quit = 1;
-        }
+        if (!g.template run<true>(it, D, rhs, rs, zbuf, upd, x, vec, &bar->err, limits.gather))
+            sh.leave = 1;
         sync();
-        if (sh.quit) return;
+        if (sh.leave) goto left;
         if (trace && threadIdx.x == 0) trace[3 * it.index + 1] = globaltimer_ns();
         if (it.kind == 0)
             for (int r = it.rb + (int)threadIdx.x; r < min(it.re, it.S); r += NT)
@@ -509,11 +522,13 @@ __global__ void __launch_bounds__(NT + 32, MINB) k_solve_flow(
         const int len = it.kind == 0 ? it.S : it.f;
         const T *A = F + it.fo + (long long)it.r0 * it.f;
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        // chunk ks in shared memory; the producer may refill its stage after release()
+        // chunk ks in shared memory; the producer may refill its stage after release().
+        // Where the wait runs out the rows go on with what is there: nobody uses
+        // the result, and a way out of here would cost every chunk a vote.
         auto chunk = [&]() -> const T * {
             const int s = ks % kStages;
-            return mbar_wait(&sh.full[s], (ks / kStages) & 1, nullptr)
-                       ? reinterpret_cast<const T *>(chunk0 + (size_t)s * cbytes) : nullptr;
+            if (!mbar_wait(&sh.full[s], (ks / kStages) & 1, &sh.quit, limits.pipe)) give_up();
+            return reinterpret_cast<const T *>(chunk0 + (size_t)s * cbytes);
         };
         auto release = [&]() {
             __syncwarp();
@@ -524,7 +539,6 @@ __global__ void __launch_bounds__(NT + 32, MINB) k_solve_flow(
         if (it.group > 0) {
             for (int c = 0; c < it.rows; c += it.group, ++ks) {
                 const T *B = chunk();
-                if (!B) return;
                 const T *first = A + (long long)c * it.f;
                 sum_rows<T, NT>(
                     min(it.group, it.rows - c), len, vec,
@@ -543,7 +557,6 @@ __global__ void __launch_bounds__(NT + 32, MINB) k_solve_flow(
                 T a[4] = {};
                 for (int b = 0; b < len; b += it.segment, ++ks) {
                     const T *B = chunk();
-                    if (!B) return;
                     if (r < it.rows) {
                         B += (size_t)wid * it.pitch + offset(A + (long long)r * it.f + b);
                         const int w = min(it.segment, len - b);
@@ -565,6 +578,11 @@ __global__ void __launch_bounds__(NT + 32, MINB) k_solve_flow(
             mbar_arrive(&sh.dempty[k & 1]);
         }
     }
+gone:
+    sh.leave = 1;
+    sync();
+left:
+    give_up();
 }
 
 }  // namespace

@@ -469,7 +469,12 @@ extern "C" int v2d_solver_newton(v2d_solver *S, double urot, double *res, v2d_li
             if (refactored) S->lu_valid = false;
             return flag_error(rep->flag, "newton assembly");
         }
-        if (status == V2D_OK && rep->bad) return mf_check_barrier(S->lu[mixed], S->s);
+        // (a wait may also have run out behind the last report: GMRES stops then)
+        if (status == V2D_OK && lu && (rep->bad || !ls.converged)) {
+            const int timeout = mf_check_barrier(S->lu[mixed], S->s);
+            if (timeout != V2D_OK) S->lu_valid = false;
+            return timeout;
+        }
         return status;
     };
     if (lu && !refactored) {
@@ -867,6 +872,17 @@ extern "C" int v2d_solver_lu_split(v2d_solver *S, int level, int *current)
     return V2D_OK;
 }
 
+extern "C" int v2d_solver_lu_wait_limits(v2d_solver *S, int gather, int pipe)
+{
+    V2D_ARG_CHECK(S, "null solver");
+    V2D_ARG_CHECK(S->plan && (S->lu[0] || S->lu[1]),
+                  "lu_wait_limits: no LU factors (precond must be V2D_PC_LU)");
+    V2D_CUDA_TRY(cudaStreamSynchronize(S->s));
+    for (MfFactor *M : S->lu)
+        if (M) V2D_TRY(mf_set_wait_limits(S->plan, M, gather, pipe));
+    return V2D_OK;
+}
+
 extern "C" int v2d_solver_lu_item_rows(v2d_solver *S, const int *rows, int nlevels, int *out_rows,
                                        int cap, int *nlevels_out)
 {
@@ -909,6 +925,7 @@ extern "C" int v2d_solver_adjoint(v2d_solver *S, double urot, const double *g_ho
         V2D_TRY(mf_factor(S->plan, S->lu[0], g.rowptr, g.val, S->s));
         ++S->lu0_ver;
         S->lu_valid = false;   // lu[0] no longer holds the Newton solve's factors
+        V2D_TRY(mf_check_barrier(S->lu[0], S->s));
         S->adj_key[0] = S->state_ver;
         S->adj_key[1] = S->val_ver;
         S->adj_key[2] = S->lu0_ver;

@@ -393,6 +393,10 @@ int v2d_lu_solve_plan_split(int imax, int jmax, const int *indptr, const int *in
                             const int *rows, int nrows, int *info4, int *items, int cap_items,
                             int *fronts3, int cap_fronts);
 
+/* Test aid (no reference counterpart): y[i] = 1 / x[i] as the factorization takes
+ * it of a pivot (host arrays; x finite and not zero). */
+int v2d_lu_reciprocals(int n, const double *x, double *y);
+
 /* Measurement aid (no reference counterpart): device time in ms, summed over
  * the Newton iterations since the last reset, of the four phases of a Newton
  * iteration (CUDA events on the handle's stream): out6 = assembly,

@@ -128,6 +128,7 @@ _SIGS = {
     "v2d_solver_residual_mesh": (_i, [_vp, _dp, _dp, _d, _d, _d, _d, _d, _d, _dp, _i, _dp]),
     "v2d_solver_trace_lu_apply": (_i, [_vp, ctypes.POINTER(ctypes.c_ulonglong), _ip, _i, _ip]),
     "v2d_solver_lu_flow_form": (_i, [_vp, _i, _ip]),
+    "v2d_lu_reciprocals": (_i, [_i, _dp, _dp]),
     "v2d_solver_lu_wait_limits": (_i, [_vp, _i, _i]),
     "v2d_solver_lu_item_rows": (_i, [_vp, _ip, _i, _ip, _i, _ip]),
     "v2d_solver_shape_tangent": (_i, [_vp, _dp, _dp, _dp, _dp, _d, _d, _d, _d, _d, _d, _d, _d,

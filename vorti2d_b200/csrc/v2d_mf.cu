@@ -1005,6 +1005,22 @@ extern "C" int v2d_lu_plan_info(int imax, int jmax, const int *indptr, const int
     return V2D_OK;
 }
 
+extern "C" int v2d_lu_reciprocals(int n, const double *x, double *y)
+{
+    using namespace v2d;
+    V2D_ARG_CHECK(n > 0, "lu_reciprocals: n = %d", n);
+    V2D_ARG_CHECK(x && y, "lu_reciprocals: null pointer");
+    DevBuf<double> d;
+    V2D_TRY(d.alloc(2 * (size_t)n, 0));
+    V2D_CUDA_TRY(cudaMemcpyAsync(d.p, x, n * sizeof(double), cudaMemcpyHostToDevice, 0));
+    k_reciprocal<<<grid_for(n, 256), 256>>>(n, d.p, d.p + n);
+    V2D_CUDA_TRY(cudaGetLastError());
+    count_launches(1);
+    V2D_CUDA_TRY(cudaMemcpyAsync(y, d.p + n, n * sizeof(double), cudaMemcpyDeviceToHost, 0));
+    V2D_CUDA_TRY(cudaStreamSynchronize(0));
+    return V2D_OK;
+}
+
 // Planning aid for the solve's work items (host only): info4 = {work items,
 // counters, fronts, levels}; when cap_items >= items, items gets 12 ints per
 // item (kind 0 forward / 1 backward, front, first row, end row, wait counter

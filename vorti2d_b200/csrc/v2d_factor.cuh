@@ -19,14 +19,15 @@
 // and H: 1.5 times as many on a front without contribution rows, 1.09 times
 // at f = 2 S, almost none more on wide fronts.
 //
-// Pivoting is partial over the rows of the pivot block, by implicit row
-// exchanges inside X (no permutation leaves the block); the row scaling
-// applied at assembly keeps the blocks well scaled, and the FP64 Krylov
-// iteration around the factors absorbs the restriction.  X is computed in
-// FP64 in both precisions: on a 181 x 181 Jacobian one FP32 solve then
-// reduces the residual to 5e-6, against 2e-2 with an FP32 X and 9e-2 with
-// FP32 LU factors and their explicit inverses (one and two GMRES iterations
-// more).
+// Pivoting is partial among 32 rows: a pivot block is inverted as two 32 x 32
+// diagonal blocks one after the other, each by implicit row exchanges inside X
+// (no permutation leaves the block), so a block whose leading half is singular
+// fails although the whole is regular.  The row scaling applied at assembly keeps
+// the blocks well scaled, and the FP64 Krylov iteration around the factors absorbs
+// the restriction.  X is computed in FP64 in both precisions: on a 181 x 181
+// Jacobian one FP32 solve then reduces the residual to 5e-6, against 2e-2 with an
+// FP32 X and 9e-2 with FP32 LU factors and their explicit inverses (one and two
+// GMRES iterations more).
 #pragma once
 
 #include <algorithm>
@@ -220,9 +221,9 @@ __device__ __forceinline__ void dmma_8x8x4(double &c0, double &c1, double a, dou
 // The block sits in shared memory as 2 x 2 blocks of 32 and is inverted by
 // block Gauss-Jordan: the 32 x 32 diagonal blocks one after the other in
 // registers (invert32), the products between the blocks on the FP64 tensor
-// cores.  The chain of pivot columns
-// bounds it, not its 2 kPiv^3 flops: the code is kept short and rolled, since
-// straight-line code that runs once waits for its own instructions.
+// cores.  The chain of pivot columns bounds it, not its 2 kPiv^3 flops: the code
+// is kept short and rolled, since straight-line code that runs once waits for its
+// own instructions.
 constexpr int kInvThreads = 128;
 constexpr int kHalf = kPiv / 2;
 constexpr int kLdX = kPiv + 2;   // two wavefronts per fragment read, rows 16-byte aligned

@@ -115,7 +115,8 @@ struct MfPlan {
     int leaf_entries = 0, leaf_warps = 0;
     size_t leaf_smem = 0;
     // work items of the solve (12 ints each: kind, front, rows [beg, end),
-    // two (counter, target) waits, two done counters), forward items level by
+    // two (counter, target) waits and two done counters for the order check, level,
+    // gathered), forward items level by
     // level bottom-up, then backward items top-down; the items of level L's
     // forward sweep are [lvl_fwd[L], lvl_fwd[L + 1]), of its backward sweep
     // [lvl_bwd[L], lvl_bwd[L + 1]) (lvl_bwd descends with L).  The order is
@@ -123,10 +124,10 @@ struct MfPlan {
     int nitems = 0, nctr = 0;
     std::vector<int> h_items, lvl_fwd, lvl_bwd;
     std::vector<int> item_rows_b;  // backward rows per item of the device's split (empty: item_rows)
-    std::vector<int> item_rows;    // rows per item of each level (0: whole fronts; R < 0:
-                                   // -R rows per item after one gather item per front)
+    std::vector<int> item_rows;    // rows per item of each level (0: whole fronts; R < 0: -R
+                                   // rows, with a place for one gather item per split front)
     std::vector<int> lvl_fwd_g, lvl_bwd_g;   // gather items at the start of each level's
-                                             // forward / backward range
+                                             // forward / backward range (the kernels skip them)
     SolveItemDev *d_items = nullptr;   // the same items with their fronts' scalars
     long long items_ver = 0;       // bumped whenever d_items is replaced
     // host copies, kept only between the build and the upload
@@ -176,7 +177,8 @@ struct MfFactor {
     void *cols = nullptr;       // one elimination step's pivot columns of a level's fronts
     void *wb = nullptr;         // transposed solve: per-front adjoint right-hand sides (vtotal)
     double *rs = nullptr;       // row scaling 1 / max |a_r.|
-    int *flag = nullptr;        // singular pivot block; then a tile counter per elimination step
+    int *flag = nullptr;        // a pivot column of zeros was left out; then a tile counter per
+                                // elimination step
     int steps = 0;
     MfBarrier *bar = nullptr;
     void *msg = nullptr;        // dataflow solve: the tickets, upd and z in one allocation
@@ -242,7 +244,6 @@ int mf_set_wait_limits(MfPlan *P, MfFactor *M, int gather, int pipe);
 // with A11^-T / H^T, then a top-down sweep with G^T).
 int mf_apply_transpose(const MfPlan *P, MfFactor *M, const void *g, void *lambda, cudaStream_t s,
                        long long *launches = nullptr);
-int mf_flag(const MfFactor *M, int *flag, cudaStream_t s);
 // V2D_ETIMEOUT (and a reset error state) if a wait of the dataflow solve or of
 // the factorization ran out since the last check.
 int mf_check_barrier(MfFactor *M, cudaStream_t s);
@@ -253,7 +254,7 @@ const int *mf_error_word(const MfFactor *M);
 int mf_time_apply(const MfPlan *P, const MfFactor *M, int reps, size_t flush_bytes, cudaStream_t s,
                   double *ms_avg);
 // One dataflow solve with per-item global-timer ticks (3 per item: ticket,
-// end of wait, done); *n = items.
+// vector gathered, rows done); *n = items.
 int mf_trace_apply(const MfPlan *P, const MfFactor *M, cudaStream_t s, unsigned long long *ticks,
                    int cap, int *n);
 // Per-launch device time of one solve (average of reps), with the launch

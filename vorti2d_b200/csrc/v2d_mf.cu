@@ -61,14 +61,15 @@ constexpr int kSolveRowsHost = 8;
 // the default work-item split aims at about this many items per level
 constexpr int kItemsPerLevel = 600;
 
-// Dependency counters of the plan's order check, per front q: forward items of
-// q that wrote z rows (fz), the children's forward items that wrote
-// contribution rows (fin), backward items of q (bx), gather items (fg, bg).
-__host__ __device__ inline int ctr_fz(int q, int nf) { return q; }
-__host__ __device__ inline int ctr_fin(int q, int nf) { return nf + q; }
-__host__ __device__ inline int ctr_bx(int q, int nf) { return 2 * nf + q; }
-__host__ __device__ inline int ctr_fg(int q, int nf) { return 3 * nf + q; }
-__host__ __device__ inline int ctr_bg(int q, int nf) { return 4 * nf + q; }
+// Dependency counters of the plan's order check (host only; the kernels wait for
+// the values themselves), per front q: forward items of q that wrote z rows (fz),
+// the children's forward items that wrote contribution rows (fin), backward items
+// of q (bx), gather items (fg, bg).
+inline int ctr_fz(int q, int nf) { return q; }
+inline int ctr_fin(int q, int nf) { return nf + q; }
+inline int ctr_bx(int q, int nf) { return 2 * nf + q; }
+inline int ctr_fg(int q, int nf) { return 3 * nf + q; }
+inline int ctr_bg(int q, int nf) { return 4 * nf + q; }
 constexpr int kCtrPerFront = 5;
 
 // ================================================================ symbolic
@@ -1651,12 +1652,6 @@ int mf_apply_transpose(const MfPlan *P, MfFactor *M, const void *g, void *lambda
                                             launches);
 }
 
-int mf_flag(const MfFactor *M, int *flag, cudaStream_t s)
-{
-    V2D_CUDA_TRY(cudaMemcpyAsync(flag, M->flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-    return V2D_OK;
-}
-
 int mf_set_wait_limits(MfPlan *P, MfFactor *M, int gather, int pipe)
 {
     M->limits.gather = gather < 0 ? kFlowSpins : std::min(gather, kFlowSpins);
@@ -1717,8 +1712,8 @@ int mf_time_apply(const MfPlan *P, const MfFactor *M, int reps, size_t flush_byt
 }
 
 // Measurement aid: one dataflow solve of a zero vector with a per-item
-// trace (ns of the global timer at the ticket, at the end of the item's
-// wait, after its done counters): ticks[3 i + k] for the n items (n <= cap).
+// trace (ns of the global timer at the ticket, when the item's vector is
+// gathered, after its rows): ticks[3 i + k] for the n items (n <= cap).
 int mf_trace_apply(const MfPlan *P, const MfFactor *M, cudaStream_t s, unsigned long long *ticks,
                    int cap, int *n)
 {

@@ -29,7 +29,6 @@ __device__ __forceinline__ bool stopped(const int *a, const int *b)
 }
 
 constexpr int kSolveThreads = 256;   // threads that compute a work item
-constexpr int kFlowSlots = 4;    // ticket counters (three used)
 constexpr int kGatherRegs = 4;   // gathered entries per thread whose indices load before the wait
 constexpr int kRowGroup = 4;     // rows a warp sums at once
 constexpr int kStages = 2;       // matrix chunks in flight ahead of the rows
@@ -77,9 +76,10 @@ __device__ __forceinline__ void plan_chunks(SolveItem &it, int bytes, int nw)
 // dataflow solve z, upd and x are filled with 0xff bytes (unset: a NaN that no
 // arithmetic makes), and an item reads an entry again until it is set.  FP64
 // arithmetic may hand on an operand's NaN, so a store replaces this one, which a
-// caller's matrix could hold, by the ordinary NaN (no measurable cost).  One word is one message, so neither side needs an ordering
-// between words: no counter, no release fence after an item's writes (about 0.8
-// us) and no separate poll before its gather (about 0.6 us).
+// caller's matrix could hold, by the ordinary NaN (no measurable cost).  One word
+// is one message, so neither side needs an ordering between words: no counter, no
+// release fence after an item's writes (about 0.8 us) and no separate poll before
+// its gather (about 0.6 us).
 template <class T> struct Unset;
 template <> struct Unset<float> {
     __device__ __forceinline__ static bool is(float v) { return __float_as_uint(v) == 0xffffffffu; }

@@ -2,12 +2,13 @@
 
 The solve (one dataflow launch over the front tree) runs in one of two
 kernel forms (two resident CTAs per SM, or three with less shared memory each)
-and splits each front's rows
-into work items; on tree level L an item is ``rows[L]`` rows of one front, or
-the whole front (0); ``rows[L] = -R`` is the split of R with a place for one
-gather item per split front in the plan, which the kernels skip (every item
-gathers its own right-hand side).  Small items spread a level's rows over more
-CTAs and shorten the chain of dependent steps; large ones gather each front's
+and splits each front's rows into work items; on tree level L an item is
+``rows[L]`` rows of one front, or the whole front (0); ``rows[L] = -R`` is the
+split of R with a place for one gather item per split front in the plan, which
+the kernels skip (every item gathers its own right-hand side).  A level at its
+starting count keeps the starting split's own count for the backward sweep; any
+other count holds for both.  Small items spread a level's rows over more CTAs
+and shorten the chain of dependent steps; large ones gather each front's
 right-hand side once and keep a CTA's rows together.  Which wins depends on
 the grid, the precision and the GPU, so it is measured: a coordinate search
 over the levels (each level's candidates tried with the others fixed, two
@@ -108,7 +109,7 @@ def tune_lu_solve(solver, candidates=CANDIDATES, sweeps: int = 2, reps: int | No
     t0 = time_apply(solver, reps)
     best = t0
     trials = 0
-    # kernel form first (resident CTAs per SM against row registers)
+    # kernel form first (two or three resident CTAs per SM)
     form = flow_form(solver)
     for f in (0, 1):
         if f == form or not set_flow_form(solver, f):

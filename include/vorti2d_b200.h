@@ -159,7 +159,12 @@ int v2d_compute_velocity(int imax, int jmax, double dksi, double deta, const dou
 
 #define V2D_PREC_FP64 0    /* FP64 Krylov                                     */
 #define V2D_PREC_MIXED 1   /* FP32 SpMV/PC/Krylov vectors, FP64 Gram-Schmidt
-                              sums, FP64 outer defect correction              */
+                              sums, FP64 outer defect correction.  With
+                              V2D_PC_LU a solve that stalls with fresh FP32
+                              factors (ill-conditioned Jacobians far from a
+                              solution) goes on with FP64 factors, allocated
+                              the first time, within the same max_it; where
+                              they do not fit it stays in FP32.               */
 
 typedef struct {
     int restart;          /* GMRES(m) restart length                  (30)   */

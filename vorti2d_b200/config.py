@@ -62,7 +62,9 @@ class Config:
     precision: str = "fp64"
     """``"fp64"``: FP64 GMRES.  ``"mixed"``: FP32 SpMV / preconditioner /
     Krylov vectors inside an FP64 defect correction (FP64 residual, metrics,
-    Jacobian entries, Gram-Schmidt sums and forces)."""
+    Jacobian entries, Gram-Schmidt sums and forces); with ``precond="lu"`` a
+    solve that stalls with FP32 factors goes on with FP64 ones, allocated the
+    first time it is needed."""
     precond: str = "lu"
     """Krylov preconditioner: ``"lu"`` (multifrontal LU of each Newton
     Jacobian on the device, FP32 factors in the mixed form; converges in a few

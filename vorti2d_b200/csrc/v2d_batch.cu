@@ -154,6 +154,7 @@ struct v2d_batch {
     int nblk = 0, nublk = 0;
     MfPlan *plan = nullptr;
     MfFactor *lu = nullptr;
+    MfFactor *lu64 = nullptr;   // mixed: FP64 factors, made on first need (krylov_solve_fresh)
     KrylovWork *kw = nullptr;
     bool lu_valid = false;
     int lu_last_its = 0;
@@ -166,6 +167,7 @@ extern "C" int v2d_batch_destroy(v2d_batch *B)
     if (B->s) cudaStreamSynchronize(B->s);
     krylov_destroy(B->kw);
     mf_factor_destroy(B->lu);
+    mf_factor_destroy(B->lu64);
     mf_plan_destroy(B->plan);
     void *ptrs[] = {B->rowptr, B->colind, B->row_inst, B->val, B->b, B->x, B->val32,
                     B->d_inst, B->d_blk0, B->d_ublk0, B->d_nodes, B->d_rowoff, B->d_active,
@@ -400,8 +402,7 @@ extern "C" int v2d_batch_newton(v2d_batch *B, double *res, int *flags, v2d_lin_s
     if (refactor) {
         V2D_TRY(mf_factor(B->plan, B->lu, B->rowptr, B->val, s));
         ++B->factorizations;
-        A.lu_fresh = true;
-        V2D_TRY(krylov_solve(B->kw, A, B->b, B->x, kp, &ls, s));
+        V2D_TRY(krylov_solve_fresh(B->kw, A, &B->lu64, B->b, B->x, kp, &ls, s));
     } else {
         v2d_krylov_params k2 = kp;
         k2.max_it = std::min(kp.max_it, kp.lu_reuse_its + 5);
@@ -411,13 +412,14 @@ extern "C" int v2d_batch_newton(v2d_batch *B, double *res, int *flags, v2d_lin_s
             const int its0 = ls.iterations;
             V2D_TRY(mf_factor(B->plan, B->lu, B->rowptr, B->val, s));
             ++B->factorizations;
-            refactor = A.lu_fresh = true;
-            V2D_TRY(krylov_solve(B->kw, A, B->b, B->x, kp, &ls, s));
+            refactor = true;
+            V2D_TRY(krylov_solve_fresh(B->kw, A, &B->lu64, B->b, B->x, kp, &ls, s));
             ls.iterations += its0;
         }
     }
-    V2D_TRY(mf_check_barrier(B->lu, s));
-    B->lu_valid = true;
+    V2D_TRY(mf_check_barrier(const_cast<MfFactor *>(A.lu), s));
+    B->lu_valid = A.lu == B->lu;
+    if (!B->lu_valid) ++B->factorizations;
     B->lu_last_its = refactor ? 0 : ls.iterations;
     if (st) *st = ls;
     k_batch_update<<<B->nublk, kBatchUpd, 0, s>>>(ni, B->d_ublk0, B->d_nodes, B->d_rowoff,

@@ -303,7 +303,16 @@ struct KrylovTail {
 // Solves A x = b (x is overwritten, starting from zero).  d_b, d_x device.
 int krylov_solve(KrylovWork *w, const CsrOp &A, const double *d_b, double *d_x,
                  const v2d_krylov_params &prm, v2d_lin_stats *st, cudaStream_t s,
-                 const KrylovTail *tail = nullptr);
+                 const KrylovTail *tail = nullptr, bool *stalled = nullptr);
+// The same with factors of A's own values.  FP32 ones fail on Jacobians far from a
+// solution (steady Newton at Re 600 on 65 x 49: pivot blocks so ill conditioned
+// that their explicit inverses in FP32 are no preconditioner, where FP32 LU factors
+// still were one): a mixed solve that stalls is done again with FP64 factors,
+// which are made on first need in *lu64, and in FP64 throughout (there: 6 + 2
+// steps).  A.lu then is *lu64, and the caller's FP32 factors are not worth keeping.
+int krylov_solve_fresh(KrylovWork *w, CsrOp &A, MfFactor **lu64, const double *d_b, double *d_x,
+                       const v2d_krylov_params &prm, v2d_lin_stats *st, cudaStream_t s,
+                       const KrylovTail *tail = nullptr);
 
 int time_spmv(const CsrOp &A, bool fp32, int reps, size_t flush_bytes, cudaStream_t s,
               double *ms_avg);

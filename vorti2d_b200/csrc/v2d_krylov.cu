@@ -732,10 +732,21 @@ static int capture_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, doub
     return V2D_OK;
 }
 
-// One restart cycle; *h receives the control block at its end.
+// An FP32 cycle whose preconditioner does not precondition: after kStallSteps
+// steps the residual is not below kStallFactor times the cycle's first one, or the
+// whole cycle does not take the true one below kStallCycle times it.  Fresh FP32
+// factors that serve reach 1e-4 and less in six steps (129 x 129 at Re 40 and 400:
+// 1e-11 and 6e-10; 65 x 49 at Re 300: 6e-5), ones that do not stay above 1e-2 (65 x
+// 49 at Re 600, after five Newton steps from the free stream: 8e-2, then 8e-3 after
+// 30).
+constexpr int kStallSteps = 6;
+constexpr double kStallFactor = 1e-2, kStallCycle = 0.1;
+
+// One restart cycle; *h receives the control block at its end.  stalled (may be
+// null): ends the cycle early, without a result, when it stalls.
 template <class T>
 static int run_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, double *x, const CsrOp &A,
-                     int precond, cudaStream_t s, Ctl *h, const KrylovTail *tail)
+                     int precond, cudaStream_t s, Ctl *h, const KrylovTail *tail, bool *stalled)
 {
     const bool lu = precond == V2D_PC_LU;
     if (w->seg[which].empty() || !w->fin[which] || w->graph_m[which] != w->m ||
@@ -763,6 +774,12 @@ static int run_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, double *
             return V2D_OK;
         }
         if (w->ctl_host->cyc_stop) break;
+        if (stalled && w->ctl_host->jdone >= kStallSteps &&
+            !(w->ctl_host->resid <= kStallFactor * w->ctl_host->beta)) {
+            *stalled = true;
+            *h = *w->ctl_host;
+            return V2D_OK;
+        }
     }
     V2D_CUDA_TRY(cudaGraphLaunch(w->fin[which], s));
     count_launches(3);
@@ -837,7 +854,7 @@ static int ensure_basis(KrylovWork *w, bool fp32, bool lu)
 
 int krylov_solve(KrylovWork *w, const CsrOp &A, const double *d_b, double *d_x,
                  const v2d_krylov_params &prm, v2d_lin_stats *st, cudaStream_t s,
-                 const KrylovTail *tail)
+                 const KrylovTail *tail, bool *stalled)
 {
     V2D_ARG_CHECK(A.n == w->n, "krylov_solve: operator size %d != workspace size %d", A.n, w->n);
     V2D_ARG_CHECK(prm.restart == w->m, "krylov_solve: restart changed (%d != %d)", prm.restart, w->m);
@@ -868,14 +885,19 @@ int krylov_solve(KrylovWork *w, const CsrOp &A, const double *d_b, double *d_x,
     // kernels end at once where that has met the tolerance already
     Ctl h = c;
     int guard = 0;
+    double beta = 0.0;   // at the cycle's start
     do {
         int status = fp32 ? run_cycle<float>(w, 1, w->V32, w->w32, w->z32, w->Z32, d_x, A,
-                                             hd.precond, s, &h, tail)
+                                             hd.precond, s, &h, tail, stalled)
                           : run_cycle<double>(w, 0, w->V64, w->w64, w->z64, w->Z64, d_x, A,
-                                              hd.precond, s, &h, tail);
+                                              hd.precond, s, &h, tail, nullptr);
         if (status != V2D_OK) return status;
         if (++guard > 1000000) break;
-    } while (!h.conv);
+        if (stalled && !h.conv && !(h.beta <= kStallCycle * (guard == 1 ? h.res0 : beta)))
+            *stalled = true;
+        beta = h.beta;
+    } while (!h.conv && !(stalled && *stalled));
+    if (stalled && fp32 && h.nonfinite && h.its > 0) *stalled = true;
     const bool converged = h.ok != 0;
     if (st) {
         st->iterations = h.its;
@@ -885,10 +907,36 @@ int krylov_solve(KrylovWork *w, const CsrOp &A, const double *d_b, double *d_x,
         st->res0 = h.res0;
         st->res = h.beta;
     }
-    if (h.nonfinite) {
+    if (h.nonfinite && !(stalled && *stalled)) {
         set_error("GMRES: non-finite residual (iteration %d)", h.its);
         return V2D_ENONFINITE;
     }
+    return V2D_OK;
+}
+
+int krylov_solve_fresh(KrylovWork *w, CsrOp &A, MfFactor **lu64, const double *d_b, double *d_x,
+                       const v2d_krylov_params &prm, v2d_lin_stats *st, cudaStream_t s,
+                       const KrylovTail *tail)
+{
+    A.lu_fresh = true;
+    bool stalled = false;
+    V2D_TRY(krylov_solve(w, A, d_b, d_x, prm, st, s, tail,
+                         prm.precision == V2D_PREC_MIXED ? &stalled : nullptr));
+    if (!stalled) return V2D_OK;
+    const int its = st->iterations;
+    if (ensure_basis(w, false, true) != V2D_OK ||
+        (!*lu64 && mf_factor_create(A.lu_plan, 0, 0, lu64) != V2D_OK)) {
+        cudaGetLastError();   // no room for them: FP32 has to do
+        return krylov_solve(w, A, d_b, d_x, prm, st, s, tail);
+    }
+    (*lu64)->flow = A.lu->flow;
+    A.lu = *lu64;
+    V2D_TRY(mf_factor(A.lu_plan, *lu64, A.rowptr, A.val, s));
+    v2d_krylov_params p64 = prm;
+    p64.precision = V2D_PREC_FP64;
+    p64.max_it = std::max(1, prm.max_it - its);
+    V2D_TRY(krylov_solve(w, A, d_b, d_x, p64, st, s, tail));
+    st->iterations += its;
     return V2D_OK;
 }
 

@@ -49,6 +49,7 @@ struct v2d_linsys {
     int imax = 0, jmax = 0;
     MfPlan *plan = nullptr;
     MfFactor *lu = nullptr;
+    MfFactor *lu64 = nullptr;   // mixed: FP64 factors, made on first need (krylov_solve_fresh)
     bool lu_fresh = false;      // factors of the current values
     int lu_last_its = 0;
 };
@@ -180,6 +181,7 @@ extern "C" int v2d_linsys_destroy(v2d_linsys *L)
         if (p) cudaFree(p);
     krylov_destroy(L->kw);
     mf_factor_destroy(L->lu);
+    mf_factor_destroy(L->lu64);
     mf_plan_destroy(L->plan);
     if (L->s) cudaStreamDestroy(L->s);
     delete L;
@@ -420,7 +422,7 @@ extern "C" int v2d_linsys_solve(v2d_linsys *L, double *x, v2d_lin_stats *st)
         bool fresh = L->lu_fresh;
         // a wait that ran out: the factors are not used again
         auto check = [&]() -> int {
-            const int status = mf_check_barrier(L->lu, L->s);
+            const int status = mf_check_barrier(const_cast<MfFactor *>(A.lu), L->s);
             if (status != V2D_OK) {
                 L->lu_fresh = false;
                 L->lu_last_its = -1;
@@ -446,14 +448,13 @@ extern "C" int v2d_linsys_solve(v2d_linsys *L, double *x, v2d_lin_stats *st)
             }
         }
         if (fresh) {
-            A.lu_fresh = true;
-            V2D_TRY(krylov_solve(L->kw, A, L->b, L->x, kp, &ls, L->s));
+            V2D_TRY(krylov_solve_fresh(L->kw, A, &L->lu64, L->b, L->x, kp, &ls, L->s));
             V2D_TRY(check());
             ls.iterations += its0;
         }
         const bool refactored = fresh && !L->lu_fresh;
         if (fresh) L->lu_fresh = true;
-        L->lu_last_its = refactored ? 0 : ls.iterations;
+        L->lu_last_its = A.lu != L->lu ? -1 : refactored ? 0 : ls.iterations;
     } else {
         V2D_TRY(krylov_solve(L->kw, A, L->b, L->x, L->prm, &ls, L->s));
     }

@@ -210,7 +210,7 @@ int sync_flag(v2d_solver *S, const char *what)
 // (an iteration of 25 x 17: 0.30 ms, 0.37 before).
 struct NewtonTail {
     v2d_solver *S;
-    const int *bad;
+    const CsrOp *A;   // with the factors of the solve (if any)
     NewtonReport *host;
 };
 
@@ -229,7 +229,8 @@ int newton_tail(void *self, const int *ok, cudaStream_t s)
 {
     NewtonTail *t = static_cast<NewtonTail *>(self);
     V2D_CUDA_TRY(cudaEventRecord(t->S->ev[3], s));
-    V2D_TRY(launch_update(t->S, NewtonGate{ok, t->bad, t->S->flag}, t->host));
+    const int *bad = t->A->lu ? mf_error_word(t->A->lu) : nullptr;
+    V2D_TRY(launch_update(t->S, NewtonGate{ok, bad, t->S->flag}, t->host));
     V2D_CUDA_TRY(cudaEventRecord(t->S->ev[4], s));
     return V2D_OK;
 }
@@ -445,7 +446,7 @@ extern "C" int v2d_solver_newton(v2d_solver *S, double urot, double *res, v2d_li
         if (!mixed) ++S->lu0_ver;
         ++S->lu_factorizations;
         S->lu_ready = true;
-        refactored = A.lu_fresh = true;
+        refactored = true;
         return V2D_OK;
     };
     if (lu) {
@@ -458,20 +459,26 @@ extern "C" int v2d_solver_newton(v2d_solver *S, double urot, double *res, v2d_li
     V2D_CUDA_TRY(cudaEventRecord(S->ev[2], S->s));
     NewtonReport *rep = reinterpret_cast<NewtonReport *>(S->host + 12);
     *rep = NewtonReport{};   // nothing of an earlier iteration is in flight
-    NewtonTail nt{S, lu ? mf_error_word(S->lu[mixed]) : nullptr, rep};
+    NewtonTail nt{S, &A, rep};
     const KrylovTail tail{newton_tail, &nt};
     v2d_lin_stats ls{};
     // one solve with what its tail reported: the assembly's flag first (its
     // values have been factorized by then), then the LU solve's own error
     auto solve = [&](const v2d_krylov_params &k) -> int {
-        const int status = krylov_solve(S->kw, A, g.b, S->delta, k, &ls, S->s, &tail);
+        const int status =
+            refactored ? krylov_solve_fresh(S->kw, A, &S->lu[0], g.b, S->delta, k, &ls, S->s, &tail)
+                       : krylov_solve(S->kw, A, g.b, S->delta, k, &ls, S->s, &tail);
+        if (mixed && A.lu && A.lu == S->lu[0]) {   // with FP64 factors in the end
+            ++S->lu0_ver;
+            ++S->lu_factorizations;
+        }
         if (rep->flag && lu) {
             if (refactored) S->lu_valid = false;
             return flag_error(rep->flag, "newton assembly");
         }
         // (a wait may also have run out behind the last report: GMRES stops then)
         if (status == V2D_OK && lu && (rep->bad || !ls.converged)) {
-            const int timeout = mf_check_barrier(S->lu[mixed], S->s);
+            const int timeout = mf_check_barrier(const_cast<MfFactor *>(A.lu), S->s);
             if (timeout != V2D_OK) S->lu_valid = false;
             return timeout;
         }
@@ -492,7 +499,7 @@ extern "C" int v2d_solver_newton(v2d_solver *S, double urot, double *res, v2d_li
         V2D_TRY(solve(kp));
     }
     if (lu) {
-        S->lu_valid = true;
+        S->lu_valid = A.lu == S->lu[mixed];
         S->lu_last_its = refactored ? 0 : ls.iterations;
     }
     if (st) *st = ls;

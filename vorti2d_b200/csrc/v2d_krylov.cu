@@ -56,7 +56,7 @@ struct Ctl {
     int cycles;
     int nonfinite;
     int ok;              // conv, and the true residual reached its target (or stagnated near it)
-    int hold;            // steps 0 and 1 run as one: no end between them
+    int hold;            // no cycle's end behind the first `hold` steps
     int stagnated;       // a cycle failed to halve the residual near the target
     double prev_beta;
     unsigned int cnt[4]; // last-block counters
@@ -82,6 +82,7 @@ struct KrylovWork {
     // FP64 and FP32 Arnoldi bases (allocated on first use of each precision)
     double *V64 = nullptr, *w64 = nullptr, *z64 = nullptr, *Z64 = nullptr;
     float *V32 = nullptr, *w32 = nullptr, *z32 = nullptr, *Z32 = nullptr;
+    int kept_its = 0;             // steps of the last FP64 solve with kept factors
     double *r = nullptr;          // FP64 residual
     double *H = nullptr;          // (m+1) x m column-major
     double *g = nullptr, *cs = nullptr, *sn = nullptr, *y = nullptr, *hcur = nullptr;
@@ -392,11 +393,11 @@ __global__ void __launch_bounds__(kRedThreads) k_update(const Desc *d, Ctl *ctl,
     }
 }
 
-// The kernels of a cycle's end, queued before it is known whether the cycle has
-// ended (guard 1; 2 after step 0, where it is left for step 1's under hold).
+// The kernels of a cycle's end, queued behind `guard` steps before it is known
+// whether the cycle has ended there (guard 0: it has).
 __device__ __forceinline__ bool no_end(const Ctl *ctl, int guard)
 {
-    return guard && (!ctl->cyc_stop || (guard == 2 && ctl->hold));
+    return guard && (!ctl->cyc_stop || guard <= ctl->hold);
 }
 
 // End of a cycle: back-substitution R y = g over the completed columns.
@@ -579,26 +580,29 @@ static int tile_grid(long long n)
     return (int)std::max(1LL, std::min<long long>(kTileBlocks, g));
 }
 
-// A restart cycle runs as a few captured segments of Arnoldi steps ([0,2),
-// [2,6), [6,10), [10,14), then 8 at a time; steps 0 and 1 apart in FP64), the
-// ones up to step 1 with the cycle's end behind them, then a finishing graph
+// A restart cycle runs as a few captured segments of Arnoldi steps, the ones up
+// to step 1 with the cycle's end behind them, then a finishing graph
 // (back-substitution, correction, FP64 residual).  The host reads the control
-// block after each segment and skips the remaining segments once the cycle has
-// stopped, so a cycle that converges in a few steps (the usual case with the LU
-// preconditioner: 6-12 with factors kept across Newton iterations) launches few
-// steps past its last one; each step after the stop is a chain of launches that
-// return at once.  With fresh FP64 factors one step is enough up to about 257 x
-// 257 and two beyond: there the host reads after step 0 too (25 x 17: 1.22 ms a
-// pass against 1.27 without).  FP32 cycles need two or more (181 x 181 mixed:
-// 28.1 ms against 29.3 with a read after step 0).
+// block after a segment and skips the remaining ones once the cycle has stopped,
+// so a cycle that converges in a few steps launches few steps past its last one;
+// each step after the stop is a chain of launches that return at once.  A read
+// costs about as much as one such step on a small grid, so it pays where the cycle
+// may end:
+//   FP32 ([0,2), then 4, 4, 4 and 8 at a time): after two steps (181 x 181 mixed:
+//     28.1 ms a pass against 29.3 with a read after step 0 too);
+//   FP64 (1, 1, then 2 four times, 4 three times and 8 at a time) with fresh LU
+//     factors: after one, which is enough up to about 257 x 257, and two (25 x 17:
+//     1.22 ms a pass against 1.27 without the first);
+//   with kept factors: one step before the last such solve ended, and from there
+//     on (44 x 43, reuse 12: 7.3 ms a pass with reads after 1, 4, 8, 12 steps, 7.5
+//     after 2, 6, 10, 14, 7.2 so).
 static std::vector<int> segment_bounds(int m, bool fp32)
 {
+    const std::vector<int> len = fp32 ? std::vector<int>{2, 4, 4, 4}
+                                      : std::vector<int>{1, 1, 2, 2, 2, 2, 4, 4, 4};
     std::vector<int> b{0};
-    if (!fp32) b.push_back(1);
-    for (int len : {2, 4, 4, 4}) b.push_back(b.back() == 1 ? 2 : b.back() + len);
-    while (b.back() < m) b.push_back(b.back() + 8);
-    while (b.size() > 2 && b[b.size() - 2] >= m) b.pop_back();
-    b.back() = std::min(b.back(), m);
+    for (size_t q = 0; b.back() < m; ++q)
+        b.push_back(std::min(m, b.back() + (q < len.size() ? len[q] : 8)));
     return b;
 }
 
@@ -711,7 +715,7 @@ static int capture_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, doub
             }
         }
         if (bnd[q] < 2) {   // the first steps often are the last: their end without a round trip
-            finish(bnd[q + 1] == 1 ? 2 : 1);
+            finish(bnd[q + 1]);
             nl += 3;
         }
         cudaGraphExec_t ge = nullptr;
@@ -746,7 +750,8 @@ constexpr double kStallFactor = 1e-2, kStallCycle = 0.1;
 // null): ends the cycle early, without a result, when it stalls.
 template <class T>
 static int run_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, double *x, const CsrOp &A,
-                     int precond, cudaStream_t s, Ctl *h, const KrylovTail *tail, bool *stalled)
+                     int precond, cudaStream_t s, Ctl *h, const KrylovTail *tail, int look,
+                     bool *stalled)
 {
     const bool lu = precond == V2D_PC_LU;
     if (w->seg[which].empty() || !w->fin[which] || w->graph_m[which] != w->m ||
@@ -766,9 +771,8 @@ static int run_cycle(KrylovWork *w, int which, T *V, T *wv, T *z, T *Z, double *
     for (size_t q = 0; q < w->seg[which].size(); ++q) {
         V2D_CUDA_TRY(cudaGraphLaunch(w->seg[which][q], s));
         count_launches(w->seg_launches[which][q]);
-        const bool first = w->seg_bounds[which][q] < 2;
-        if (q == 0 && which == 0 && !A.lu_fresh && w->seg[which].size() > 1) continue;
-        V2D_TRY(read(first));
+        if (w->seg_bounds[which][q + 1] < look && q + 1 < w->seg[which].size()) continue;
+        V2D_TRY(read(w->seg_bounds[which][q] < 2 && look <= 2));
         if (w->ctl_host->conv || w->ctl_host->cycles != cycles) {   // it ended in the first steps
             *h = *w->ctl_host;
             return V2D_OK;
@@ -876,7 +880,9 @@ int krylov_solve(KrylovWork *w, const CsrOp &A, const double *d_b, double *d_x,
     c.atol = prm.atol;
     c.max_it = prm.max_it;
     c.inner_rtol = fp32 ? prm.inner_rtol : 0.0;
-    c.hold = !A.lu_fresh;
+    // the step after which the host looks first (segment_bounds)
+    const int look = fp32 ? 2 : A.lu_fresh ? 1 : lu ? std::max(2, std::min(w->kept_its - 1, 14)) : 2;
+    c.hold = fp32 ? 0 : std::min(look - 1, 2);
     k_begin<<<grid_for(A.n, 256), 256, 0, s>>>(hd, c, w->desc, w->ctl);
     k_residual<<<res_grid(A.n), kSpmvThreads, 0, s>>>(w->desc, w->ctl, w->r, w->partial, w->g, 1, 0);
     V2D_CUDA_TRY(cudaGetLastError());
@@ -888,9 +894,9 @@ int krylov_solve(KrylovWork *w, const CsrOp &A, const double *d_b, double *d_x,
     double beta = 0.0;   // at the cycle's start
     do {
         int status = fp32 ? run_cycle<float>(w, 1, w->V32, w->w32, w->z32, w->Z32, d_x, A,
-                                             hd.precond, s, &h, tail, stalled)
+                                             hd.precond, s, &h, tail, look, stalled)
                           : run_cycle<double>(w, 0, w->V64, w->w64, w->z64, w->Z64, d_x, A,
-                                              hd.precond, s, &h, tail, nullptr);
+                                              hd.precond, s, &h, tail, look, nullptr);
         if (status != V2D_OK) return status;
         if (++guard > 1000000) break;
         if (stalled && !h.conv && !(h.beta <= kStallCycle * (guard == 1 ? h.res0 : beta)))
@@ -899,6 +905,7 @@ int krylov_solve(KrylovWork *w, const CsrOp &A, const double *d_b, double *d_x,
     } while (!h.conv && !(stalled && *stalled));
     if (stalled && fp32 && h.nonfinite && h.its > 0) *stalled = true;
     const bool converged = h.ok != 0;
+    if (lu && !fp32 && !A.lu_fresh) w->kept_its = converged ? h.its : 0;
     if (st) {
         st->iterations = h.its;
         st->restarts = h.cycles;

@@ -51,7 +51,7 @@ struct v2d_linsys {
     MfFactor *lu = nullptr;
     MfFactor *lu64 = nullptr;   // mixed: FP64 factors, made on first need (krylov_solve_fresh)
     bool lu_fresh = false;      // factors of the current values
-    int lu_last_its = 0;
+    int lu_last_its = -1;       // steps of the last solve with the factors (-1: none to keep)
 };
 
 namespace {
